@@ -290,7 +290,7 @@ int vebi_batch_destroy(vebi_batch* b);
 int vebi_set_solver_grid(vebi_ctx* ctx, int32_t rows_per_thread);
 /* Tile size of the multigrid V-cycle (VEBI_PRECOND_MULTIGRID; no reference counterpart): the
  * coarse levels of at most `rows` rows run in one thread block with block barriers instead of
- * across the grid with grid barriers (default 2048).  Results do not depend on it. */
+ * across the grid with grid barriers (default 512).  Results do not depend on it. */
 int vebi_set_coarse_block_rows(vebi_ctx* ctx, int32_t rows);
 
 /* Static description of the library build. */

@@ -17,7 +17,8 @@
 // one post-smoothing sweep; the particle level is pre-smoothed only (two particle-level
 // products per V-cycle cost more than the iterations they save).  The coarsest level takes
 // MG_SWEEPS Jacobi sweeps.  Levels of at most MG_BLOCK_ROWS rows run in
-// block 0 alone with block barriers.  Every sum runs in a fixed order.
+// block 0 alone with block barriers: one SM's FP64 pipe takes longer over a larger level than the
+// two grid barriers (1-3 us each) that the level costs on the whole grid.  Every sum runs in a fixed order.
 //
 // Solver.  BiCGSTAB with right preconditioning, in the persistent cooperative kernel of the
 // unpreconditioned solver: the same recurrences, residual test and, for closed domains, mean
@@ -302,11 +303,19 @@ __device__ __forceinline__ double ap_stencil(const double* __restrict__ rv9, con
 }
 
 // ---------------------------------------------------------------- V-cycle
+// the coarse levels, as the FP64 and the mixed V-cycle share them
+struct MgCoarse {
+  const MgLevel* lv;   // finest first
+  int nl;              // number of coarse levels (>= 1)
+  int tail;            // first level handled by block 0 alone
+  const double* kinv;  // the coarsest level's dense inverse, if *kinv_ok
+  const int* kinv_ok;
+  float* g32;          // mixed precision: the level-1 solution rounded to FP32, else null
+};
+
 struct MgArgs {
   BiArgs b;                  // the unpreconditioned solver's arguments
-  const MgLevel* lv;         // coarse levels, finest first
-  int nl;                    // number of coarse levels (>= 1)
-  int tail;                  // first level handled by block 0 alone
+  MgCoarse co;
   const int *agg, *cstart, *ccnt, *ip;  // fine aggregate (cell) of each row; cell lists
   double *z, *fr, *dinv0, *rsum;        // fine work vectors, 1/diag, row sums
   // A P by fine row (k_mg_rows): (cell, sum of the row's values in that cell) pairs, own cell
@@ -315,12 +324,40 @@ struct MgArgs {
   const double *rval, *rv9;
   int ncx;
   double* w;
-  const double* kinv;        // the coarsest level's dense inverse, if *kinv_ok
-  const int* kinv_ok;
-  float* g32;                // mixed precision: the level-1 solution rounded to FP32, else null
 };
 
-// (A x)_c on a coarse level; x may have been written by other blocks in this launch
+// (A x)_c on a coarse level with x_c = xc: the diagonal, then the slots in order.  load(k)
+// returns what x_k is formed from and value(load(k)) is x_k.  U slots' columns and values are
+// loaded at once and then their operands, so a row waits for two round trips to memory per U
+// slots, not two per slot (the grid-wide levels, whose operands come from other blocks; 4M FP64
+// solve 31.4 -> 30.7 ms.  Eight slots of two operands each spill, so the upward phase takes four).
+template <int U, class Load, class Value>
+__device__ __forceinline__ double lv_row(const MgLevel& L, int c, double xc, Load load, Value value) {
+  double y = __ldg(L.diag + c) * xc;
+  const int m = __ldg(L.cnt + c);
+  const int* cp = L.col + c;
+  const double* vp = L.val + c;
+  for (int t0 = 0; t0 < m; t0 += U) {
+    int k[U];
+    double v[U];
+    decltype(load(0)) x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const size_t e = (size_t)(t0 + u) * L.n;
+      k[u] = t0 + u < m ? __ldg(cp + e) : c;
+      v[u] = t0 + u < m ? __ldg(vp + e) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) x[u] = load(k[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (t0 + u < m) y = fma(v[u], value(x[u]), y);
+  }
+  return y;
+}
+
+// (A x)_c with x written by this block: its operands are in L1 mostly, and the plain loop has the
+// fewest instructions (20k-particle mixed solve 2.01 -> 1.88 ms against the batched form)
 __device__ __forceinline__ double lv_Ax(const MgLevel& L, const double* x, int c) {
   double y = __ldg(L.diag + c) * x[c];
   const int m = __ldg(L.cnt + c);
@@ -381,7 +418,7 @@ __device__ __forceinline__ void lv_residual_restrict(const MgLevel& F, const MgL
       const int fx = 2 * X + (q & 1), fy = 2 * Y + (q >> 1);
       if (fx < F.gx && fy < F.gy) {
         const int f = fx + fy * F.gx;
-        r = F.b[f] - lv_Ax(F, F.x, f);
+        r = F.b[f] - lv_row<8>(F, f, F.x[f], [&](int k) { return F.x[k]; }, [](double v) { return v; });
         ok = 1;
       }
     }
@@ -409,14 +446,13 @@ __device__ __forceinline__ void lv_residual_restrict(const MgLevel& F, const MgL
 __device__ __forceinline__ void lv_prolong_smooth(const MgLevel& F, const double* gsol, int ggx, int i0, int st,
                                                   float* x32 = nullptr) {
   for (int c = i0; c < F.n; c += st) {
-    auto xp = [&](int k) {
+    auto load = [&](int k) {
       const int X = (k % F.gx) >> 1, Y = (k / F.gx) >> 1;
-      return fma(MG_GAMMA, gsol[X + Y * ggx], F.x[k]);
+      return make_double2(gsol[X + Y * ggx], F.x[k]);
     };
-    const double xc = xp(c);
-    double y = __ldg(F.diag + c) * xc;
-    const int m = __ldg(F.cnt + c);
-    for (int t = 0; t < m; ++t) y = fma(__ldg(F.val + (size_t)t * F.n + c), xp(__ldg(F.col + (size_t)t * F.n + c)), y);
+    auto value = [](const double2& o) { return fma(MG_GAMMA, o.x, o.y); };
+    const double xc = value(load(c));
+    const double y = lv_row<4>(F, c, xc, load, value);
     const double v = fma(MG_OMEGA * __ldg(F.dinv + c), F.b[c] - y, xc);
     F.r[c] = v;
     if (x32) x32[c] = narrow(v);
@@ -424,12 +460,12 @@ __device__ __forceinline__ void lv_prolong_smooth(const MgLevel& F, const double
 }
 
 // the solution of level l after the upward pass: post-smoothed into r, or x on the coarsest
-__device__ __forceinline__ const double* lv_sol(const MgArgs& a, int l) {
+__device__ __forceinline__ const double* lv_sol(const MgCoarse& a, int l) {
   return l == a.nl - 1 ? a.lv[l].x : a.lv[l].r;
 }
 
 // levels tail..nl-1 by block 0 alone
-__device__ void mg_block_levels(const MgArgs& a) {
+__device__ __forceinline__ void mg_block_levels(const MgCoarse& a) {
   const int i0 = threadIdx.x, st = blockDim.x;
   for (int l = a.tail; l + 1 < a.nl; ++l) {
     const MgLevel F = a.lv[l], G = a.lv[l + 1];
@@ -467,12 +503,12 @@ __device__ void mg_block_levels(const MgArgs& a) {
   }
 }
 
-// out = M^-1 q by one V-cycle; the last loop also writes the block partial of sum(out) into
-// slot.  q needs only its own rows complete (the calling thread wrote them).
+// out = M^-1 q by one V-cycle; the last loop also sums this thread's rows of out into `sum`.
+// q needs only its own rows complete (the calling thread wrote them).
 // q -= qshift first (the closed domain's mean removal), stored back.  As in the solvers, the
 // vector passes load each row's operands one row ahead (rows_ahead).
-__device__ bool mg_vcycle(const MgArgs& a, double* q, double qshift, double* out, double* slot, double* sh,
-                          int tid, int stride) {
+__device__ bool mg_vcycle(const MgArgs& a, double* q, double qshift, double* out, double& sum, int tid,
+                          int stride) {
   const int n = a.b.n;
   Scal* s = a.b.sc;
   double* z = a.z;
@@ -487,7 +523,7 @@ __device__ bool mg_vcycle(const MgArgs& a, double* q, double qshift, double* out
   for (int i = tid; i < n; i += stride) a.fr[i] = q[i] - spmv_row(a.b, z, i);
   if (!grid_sync(s)) return false;
   {  // restriction to the cells (level 1)
-    const MgLevel L1 = a.lv[0];
+    const MgLevel L1 = a.co.lv[0];
     for (int cc = tid; cc < L1.n; cc += stride) {
       const int s0 = __ldg(a.cstart + cc), ne = __ldg(a.ccnt + cc);
       double b = 0.0;
@@ -501,14 +537,15 @@ __device__ bool mg_vcycle(const MgArgs& a, double* q, double qshift, double* out
     }
   }
   if (!grid_sync(s)) return false;
-  for (int l = 0; l < a.tail; ++l) {
-    lv_residual_restrict(a.lv[l], a.lv[l + 1], tid, stride);
+  const MgCoarse& co = a.co;
+  for (int l = 0; l < co.tail; ++l) {
+    lv_residual_restrict(co.lv[l], co.lv[l + 1], tid, stride);
     if (!grid_sync(s)) return false;
   }
-  if (blockIdx.x == 0) mg_block_levels(a);
+  if (blockIdx.x == 0) mg_block_levels(co);
   if (!grid_sync(s)) return false;
-  for (int l = a.tail - 1; l >= 0; --l) {
-    lv_prolong_smooth(a.lv[l], lv_sol(a, l + 1), a.lv[l + 1].gx, tid, stride);
+  for (int l = co.tail - 1; l >= 0; --l) {
+    lv_prolong_smooth(co.lv[l], lv_sol(co, l + 1), co.lv[l + 1].gx, tid, stride);
     if (!grid_sync(s)) return false;
   }
   // prolongation to the particles (the particle level is pre-smoothed only), and
@@ -516,7 +553,7 @@ __device__ bool mg_vcycle(const MgArgs& a, double* q, double qshift, double* out
   // direct form over the row's cells (ap_stencil).
   // Software-pipelined: a row's streamed operands are loaded one pass ahead, together with the
   // gathers of the row before, so each pass waits for one round trip to memory, not two.
-  const double* g1 = lv_sol(a, 0);
+  const double* g1 = lv_sol(co, 0);
   double acc = 0.0;
   struct Row {
     int c, rx;
@@ -548,33 +585,32 @@ __device__ bool mg_vcycle(const MgArgs& a, double* q, double qshift, double* out
     a.w[i] = w;
     acc += o;
   }
-  write_partials(acc, 0.0, 1, slot, sh);
+  sum = acc;
   return true;
 }
 
 // ---------------------------------------------------------------- preconditioned BiCGSTAB
 template <bool NONULL>
 __global__ void __launch_bounds__(TPB, 4) k_bicgstab_mg(MgArgs m) {
-  __shared__ double sh[64];
-  __shared__ double shv[4];
+  __shared__ SolverSh sh;
   const BiArgs& a = m.b;
   const int n = a.n;
   const int nb = gridDim.x;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int stride = gridDim.x * blockDim.x;
   Scal* s = a.sc;
-  if (*((volatile int*)&s->first_error)) return;  // this state already failed a step
+  if (state_failed(s)) return;
+  solver_begin(sh);
   const bool use_mg = *((volatile int*)&s->mg_fail) == 0;
   double* part = a.part;
   const double rinv1 = 1.0 / (1.0 + 1.0e-15);
   const double small = NONULL ? 1.0e-6 : 4.0;  // open solver: the integer expression 10-6
-  double red[4];
   double acc = 0.0;
-  // out = M^-1 (q - qshift) with q -= qshift stored back (q: own rows complete), and the
-  // block partial of sum(out) into slot
-  auto precond = [&](double* q, double qshift, double* out, double* slot) -> bool {
-    if (use_mg) return mg_vcycle(m, q, qshift, out, slot, sh, tid, stride);
-    double sum = 0.0;
+  // out = M^-1 (q - qshift) with q -= qshift stored back (q: own rows complete), and this
+  // thread's part of sum(out)
+  auto precond = [&](double* q, double qshift, double* out, double& sum) -> bool {
+    if (use_mg) return mg_vcycle(m, q, qshift, out, sum, tid, stride);
+    sum = 0.0;
     for (int i = tid; i < n; i += stride) {
       const double qi = q[i] - qshift;
       q[i] = qi;
@@ -582,7 +618,6 @@ __global__ void __launch_bounds__(TPB, 4) k_bicgstab_mg(MgArgs m) {
       out[i] = o;
       sum += o;
     }
-    write_partials(sum, 0.0, 1, slot, sh);
     return true;
   };
   for (int i = tid; i < n; i += stride) {  // 1/diag and row sums of the fine matrix
@@ -612,38 +647,34 @@ __global__ void __launch_bounds__(TPB, 4) k_bicgstab_mg(MgArgs m) {
     a.p[i] = 0.0;
     acc = fma(bi, bi, acc);
   }
-  write_partials(acc, 0.0, 1, part + 10 * (size_t)nb, sh);
-  if (!grid_sync(s)) return;
-  reduce_partials(part + 10 * (size_t)nb, nb, 1, red, shv);
-  double rho = red[0], alpha = 1.0, omega = 1.0;
-  double beta = 0.0;  // for iteration 2 on, derived with the previous iteration's last reduction
+  if (!grid_reduce<1>(s, acc, 0.0, part + 10 * (size_t)nb, sh, [&](double* v, int&) { sh.rho = v[0]; })) return;
   const double dn = (double)n;
-  double n2r0 = 1.0, n2s0 = 1.0, resid = 0.0;
+  bool at_s = false;  // the solve stopped on s, not on r
   int iter = 1, warn = 0;
   bool done = false;
   while (iter <= a.itermax) {
-    if (rho == 0.0) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
+    if (is_zero(sh.rho)) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
+    const double beta = sh.beta, omega0 = sh.omega;
     acc = 0.0;
     // the vector passes load each row's operands one row ahead (rows_ahead)
     rows_ahead(
         tid, stride, n, [&](int i) { return make_double3(a.r[i], a.v[i], a.p[i]); },
         [&](int i, const double3& o) {
-          const double ni = (iter == 1) ? o.x : fma(beta, fma(-omega, o.y, o.z), o.x);
+          const double ni = (iter == 1) ? o.x : fma(beta, fma(-omega0, o.y, o.z), o.x);
           a.p[i] = ni;
           acc += ni;
         });
     double mean = 0.0;
     if (NONULL) {
-      write_partials(acc, 0.0, 1, part, sh);
-      if (!grid_sync(s)) return;
-      reduce_partials(part, nb, 1, red, shv, [=](double* v) { v[0] = v[0] / dn; });
-      mean = red[0];
+      if (!grid_reduce<1>(s, acc, 0.0, part, sh, [=](double* v, int&) { v[0] = v[0] / dn; })) return;
+      mean = sh.v[0];
     }
     // p_hat = M^-1 (p - mean), made mean-free (closed domains) through mp
-    if (!precond(a.p, mean, a.pinv, part + 1 * (size_t)nb)) return;
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 1 * (size_t)nb, nb, 1, red, shv, [=](double* v) { v[0] = NONULL ? v[0] / dn : 0.0; });
-    const double mp = red[0];
+    if (!precond(a.p, mean, a.pinv, acc)) return;
+    if (!grid_reduce<1>(s, acc, 0.0, part + 1 * (size_t)nb, sh,
+                        [=](double* v, int&) { v[0] = NONULL ? v[0] / dn : 0.0; }))
+      return;
+    const double mp = sh.v[0];
     // v = A (p_hat - mp) ; (r_bar, v)
     acc = 0.0;
     if (use_mg) {
@@ -661,10 +692,10 @@ __global__ void __launch_bounds__(TPB, 4) k_bicgstab_mg(MgArgs m) {
         acc = fma(a.rb[i], vi, acc);
       }
     }
-    write_partials(acc, 0.0, 1, part + 2 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 2 * (size_t)nb, nb, 1, red, shv, [=](double* v) { v[0] = rho / (v[0] + 1.0e-15); });
-    alpha = red[0];
+    if (!grid_reduce<1>(s, acc, 0.0, part + 2 * (size_t)nb, sh,
+                        [&](double* v, int&) { sh.alpha = sh.rho / (v[0] + 1.0e-15); }))
+      return;
+    const double alpha = sh.alpha;
     double a2 = 0.0;
     acc = 0.0;
     rows_ahead(
@@ -675,22 +706,26 @@ __global__ void __launch_bounds__(TPB, 4) k_bicgstab_mg(MgArgs m) {
           acc = fma(si, si, acc);
           a2 += si;
         });
-    write_partials(acc, a2, 2, part + 4 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 4 * (size_t)nb, nb, 2, red, shv, [=](double* v) { v[1] = v[1] / dn; });
-    const double n2s = red[0];
-    const double mean_s = red[1];
-    if (iter == 1) n2s0 = (n2s <= small) ? 1.0 : n2s;
-    if (n2s <= a.tol * a.tol * n2s0) {
+    // |s|^2 against the first one (1 when small), and the mean of s
+    if (!grid_reduce<2>(s, acc, a2, part + 4 * (size_t)nb, sh, [&](double* v, int& flag) {
+          sh.n2 = v[0];
+          if (iter == 1) sh.n2s0 = (v[0] <= small) ? 1.0 : v[0];
+          flag = v[0] <= a.tol * a.tol * sh.n2s0;
+          v[1] = v[1] / dn;
+        }))
+      return;
+    const double mean_s = sh.v[1];
+    if (sh.flag) {
       for (int i = tid; i < n; i += stride) a.x[i] = fma(alpha, a.pinv[i] - mp, a.x[i]);
-      resid = sqrt(n2s / n2s0);
+      at_s = true;
       done = true;
       break;
     }
-    if (!precond(a.s, NONULL ? mean_s : 0.0, a.sinv, part + 3 * (size_t)nb)) return;
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 3 * (size_t)nb, nb, 1, red, shv, [=](double* v) { v[0] = NONULL ? v[0] / dn : 0.0; });
-    const double ms = red[0];
+    if (!precond(a.s, NONULL ? mean_s : 0.0, a.sinv, acc)) return;
+    if (!grid_reduce<1>(s, acc, 0.0, part + 3 * (size_t)nb, sh,
+                        [=](double* v, int&) { v[0] = NONULL ? v[0] / dn : 0.0; }))
+      return;
+    const double ms = sh.v[0];
     // t = A (s_hat - ms) ; (t, s) ; |t|^2
     acc = 0.0;
     a2 = 0.0;
@@ -711,48 +746,46 @@ __global__ void __launch_bounds__(TPB, 4) k_bicgstab_mg(MgArgs m) {
         a2 = fma(ti, ti, a2);
       }
     }
-    write_partials(acc, a2, 2, part + 6 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 6 * (size_t)nb, nb, 2, red, shv, [](double* v) { v[0] = v[0] / (v[1] + 1.0e-15); });
-    omega = red[0];
+    if (!grid_reduce<2>(s, acc, a2, part + 6 * (size_t)nb, sh, [&](double* v, int&) {
+          sh.omega = v[0] / (v[1] + 1.0e-15);
+          v[2] = fma(sh.alpha, mp, sh.omega * ms);  // the two mean shifts of x folded into one
+        }))
+      return;
+    const double alpha1 = sh.alpha, omega = sh.omega;
     acc = 0.0;
     a2 = 0.0;
-    // x += alpha (p_hat - mp) + omega (s_hat - ms), with the two mean shifts folded into one
-    const double xshift = fma(alpha, mp, omega * ms);
+    // x += alpha (p_hat - mp) + omega (s_hat - ms)
+    const double xshift = sh.v[2];
     struct XRow {
       double s, p, x, t, sv, rb;
     };
     rows_ahead(
         tid, stride, n, [&](int i) { return XRow{a.sinv[i], a.pinv[i], a.x[i], a.t[i], a.s[i], a.rb[i]}; },
         [&](int i, const XRow& o) {
-          a.x[i] = fma(omega, o.s, fma(alpha, o.p, o.x - xshift));
+          a.x[i] = fma(omega, o.s, fma(alpha1, o.p, o.x - xshift));
           const double ri = fma(-omega, o.t, o.sv);
           a.r[i] = ri;
           acc = fma(ri, ri, acc);
           a2 = fma(o.rb, ri, a2);
         });
-    write_partials(acc, a2, 2, part + 8 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    // v[2] = the relative residual, v[3] = the next iteration's beta from the new rho v[1]
-    reduce_partials(part + 8 * (size_t)nb, nb, 2, red, shv, [=](double* v) {
-      const double r0 = iter == 1 ? ((v[0] <= small) ? 1.0 : v[0]) : n2r0;
-      v[2] = sqrt(v[0] / r0);
-      v[3] = v[1] / (rho + 1.0e-15) * alpha / (omega + 1.0e-15);
-    });
-    const double n2r = red[0];
-    if (iter == 1) n2r0 = (n2r <= small) ? 1.0 : n2r;
-    resid = red[2];
-    if (n2r <= a.tol * a.tol * n2r0) { done = true; break; }
+    // |r|^2 against the first one (1 when small), the new rho and the next iteration's beta
+    if (!grid_reduce<2>(s, acc, a2, part + 8 * (size_t)nb, sh, [&](double* v, int& flag) {
+          sh.n2 = v[0];
+          if (iter == 1) sh.n2r0 = (v[0] <= small) ? 1.0 : v[0];
+          flag = v[0] <= a.tol * a.tol * sh.n2r0;
+          sh.beta = v[1] / (sh.rho + 1.0e-15) * sh.alpha / (sh.omega + 1.0e-15);
+          sh.rho = v[1];
+        }))
+      return;
+    if (sh.flag) { done = true; break; }
     iter = iter + 1;
-    rho = red[1];
-    beta = red[3];
   }
   if (!done) warn |= VEBI_WARN_MAXITER;
   for (int i = tid; i < n; i += stride) a.P[i] = a.x[i];
   if (tid == 0) {
     s->ls_iters = iter;
     s->ls_iters_total += iter;
-    s->ls_residual = resid;
+    s->ls_residual = sqrt(sh.n2 / (at_s ? sh.n2s0 : sh.n2r0));
     atomicOr(&s->warnings, warn);
   }
 }
@@ -765,8 +798,7 @@ __global__ void __launch_bounds__(TPB, 4) k_bicgstab_mg(MgArgs m) {
 // iteration count, not the residual test the solve stops on.
 struct MgMxArgs {
   MxArgs b;
-  const MgLevel* lv;
-  int nl, tail;
+  MgCoarse co;
   const int *agg, *cstart, *ccnt, *ip;
   float *z, *fr, *dinv0;
   const int *ragg, *rx;  // A P by fine row, as in MgArgs, with FP32 direction values
@@ -774,9 +806,6 @@ struct MgMxArgs {
   const float* rv9;
   int ncx;
   float* w;                // A times the V-cycle's output, FP32
-  const double* kinv;      // the coarsest level's dense inverse, if *kinv_ok
-  const int* kinv_ok;
-  float* g32;              // the level-1 solution rounded to FP32
   float* rs32;             // the row sums rounded to FP32
   float* q32;              // the V-cycle's input (after mean removal) rounded to FP32
   const double* diag;      // the PPE matrix's FP64 diagonal
@@ -836,12 +865,12 @@ __device__ __forceinline__ float ap_stencil32(const float* __restrict__ rv9, con
   return ap;
 }
 
-// out = M^-1 q in FP64 (the preconditioned direction); block partial of sum(out) into slot.
+// out = M^-1 q in FP64 (the preconditioned direction), and this thread's part of sum(out).
 // The vector passes load each row's operands one row ahead (rows_ahead), so a pass's loads are
 // in flight before the previous row's stores: the compiler cannot move a load above a store
 // to another array it may alias.
-__device__ bool mg_vcycle_mixed(const MgMxArgs& a, double* q, double qshift, double* out, double* slot,
-                                double* sh, int tid, int stride) {
+__device__ bool mg_vcycle_mixed(const MgMxArgs& a, double* q, double qshift, double* out, double& sum, int tid,
+                                int stride) {
   const int n = a.b.n;
   Scal* s = a.b.sc;
   float* z = a.z;
@@ -864,7 +893,7 @@ __device__ bool mg_vcycle_mixed(const MgMxArgs& a, double* q, double qshift, dou
   for (int i = tid; i < n; i += stride) a.fr[i] = q32[i] - spmv_diff32s(a.b, a.rs32, z, i);
   if (!grid_sync(s)) return false;
   {
-    const MgLevel L1 = a.lv[0];
+    const MgLevel L1 = a.co.lv[0];
     for (int cc = tid; cc < L1.n; cc += stride) {
       const int s0 = __ldg(a.cstart + cc), ne = __ldg(a.ccnt + cc);
       float b32 = 0.f;  // the cell's residuals summed in FP32, in cell-list order
@@ -879,21 +908,15 @@ __device__ bool mg_vcycle_mixed(const MgMxArgs& a, double* q, double qshift, dou
     }
   }
   if (!grid_sync(s)) return false;
-  MgArgs c{};  // the coarse-level view shared with the FP64 V-cycle
-  c.lv = a.lv;
-  c.nl = a.nl;
-  c.tail = a.tail;
-  c.kinv = a.kinv;
-  c.kinv_ok = a.kinv_ok;
-  c.g32 = a.g32;
-  for (int l = 0; l < a.tail; ++l) {
-    lv_residual_restrict(a.lv[l], a.lv[l + 1], tid, stride);
+  const MgCoarse& co = a.co;
+  for (int l = 0; l < co.tail; ++l) {
+    lv_residual_restrict(co.lv[l], co.lv[l + 1], tid, stride);
     if (!grid_sync(s)) return false;
   }
-  if (blockIdx.x == 0) mg_block_levels(c);
+  if (blockIdx.x == 0) mg_block_levels(co);
   if (!grid_sync(s)) return false;
-  for (int l = a.tail - 1; l >= 0; --l) {
-    lv_prolong_smooth(a.lv[l], lv_sol(c, l + 1), a.lv[l + 1].gx, tid, stride, l == 0 ? a.g32 : nullptr);
+  for (int l = co.tail - 1; l >= 0; --l) {
+    lv_prolong_smooth(co.lv[l], lv_sol(co, l + 1), co.lv[l + 1].gx, tid, stride, l == 0 ? co.g32 : nullptr);
     if (!grid_sync(s)) return false;
   }
   // prolongation to the particles (pre-smoothed only) from the FP32 level-1 solution g, and
@@ -901,7 +924,7 @@ __device__ bool mg_vcycle_mixed(const MgMxArgs& a, double* q, double qshift, dou
   // gamma (A P) g in difference form with the FP32 row sums.  The output is stored as FP64 and
   // summed in FP64 (the mean removal).  This GPU issues FP64 at 1/64 of the FP32 rate, so the
   // pass keeps to FP32 arithmetic; streamed operands are loaded one pass ahead of the gathers.
-  const float* g32 = a.g32;
+  const float* g32 = co.g32;
   const float gam = (float)MG_GAMMA;
   double acc = 0.0;
   struct Row {
@@ -935,7 +958,7 @@ __device__ bool mg_vcycle_mixed(const MgMxArgs& a, double* q, double qshift, dou
     a.w[i] = wi;
     acc += od;
   }
-  write_partials(acc, 0.0, 1, slot, sh);
+  sum = acc;
   return true;
 }
 
@@ -946,29 +969,28 @@ __device__ bool mg_vcycle_mixed(const MgMxArgs& a, double* q, double qshift, dou
 
 template <bool NONULL>
 __global__ void __launch_bounds__(TPB, VEBI_MIXED_MG_BLOCKS_PER_SM) k_bicgstab_mixed_mg(MgMxArgs m) {
-  __shared__ double sh[64];
-  __shared__ double shv[4];
+  __shared__ SolverSh sh;
   const MxArgs& a = m.b;
   const int n = a.n;
   const int nb = gridDim.x;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int stride = gridDim.x * blockDim.x;
   Scal* s = a.sc;
-  if (*((volatile int*)&s->first_error)) return;  // this state already failed a step
+  if (state_failed(s)) return;
+  solver_begin(sh);
   const bool use_mg = *((volatile int*)&s->mg_fail) == 0;
   double* part = a.part;
   const double rinv1 = 1.0 / (1.0 + 1.0e-15);
   const double small = NONULL ? 1.0e-6 : 4.0;
-  double red[4];
   double acc = 0.0;
-  // out = M^-1 (q - qshift), with q -= qshift stored back; block partial of sum(out) into slot
+  // out = M^-1 (q - qshift), with q -= qshift stored back; this thread's part of sum(out)
   // With the multigrid the preconditioned directions are FP64 (pi, si read as double: same
   // size as the (hi, lo) pairs the unpreconditioned products gather)
   double* const pd = reinterpret_cast<double*>(a.pi);
   double* const sd = reinterpret_cast<double*>(a.si);
-  auto precond = [&](double* q, double qshift, float2* out, double* slot) -> bool {
-    if (use_mg) return mg_vcycle_mixed(m, q, qshift, reinterpret_cast<double*>(out), slot, sh, tid, stride);
-    double sum = 0.0;
+  auto precond = [&](double* q, double qshift, float2* out, double& sum) -> bool {
+    if (use_mg) return mg_vcycle_mixed(m, q, qshift, reinterpret_cast<double*>(out), sum, tid, stride);
+    sum = 0.0;
     for (int i = tid; i < n; i += stride) {
       const double qi = q[i] - qshift;
       q[i] = qi;
@@ -976,7 +998,6 @@ __global__ void __launch_bounds__(TPB, VEBI_MIXED_MG_BLOCKS_PER_SM) k_bicgstab_m
       out[i] = split2(o);
       sum += o;
     }
-    write_partials(sum, 0.0, 1, slot, sh);
     return true;
   };
   for (int i = tid; i < n; i += stride) {
@@ -1003,37 +1024,33 @@ __global__ void __launch_bounds__(TPB, VEBI_MIXED_MG_BLOCKS_PER_SM) k_bicgstab_m
     a.p[i] = 0.0;
     acc = fma(bi, bi, acc);
   }
-  write_partials(acc, 0.0, 1, part + 10 * (size_t)nb, sh);
-  if (!grid_sync(s)) return;
-  reduce_partials(part + 10 * (size_t)nb, nb, 1, red, shv);
-  double rho = red[0], alpha = 1.0, omega = 1.0;
-  double beta = 0.0;  // for iteration 2 on, derived with the previous iteration's last reduction
+  if (!grid_reduce<1>(s, acc, 0.0, part + 10 * (size_t)nb, sh, [&](double* v, int&) { sh.rho = v[0]; })) return;
   const double dn = (double)n;
-  double n2r0 = 1.0, n2s0 = 1.0, resid = 0.0;
+  bool at_s = false;  // the solve stopped on s, not on r
   int iter = 1, warn = 0;
   bool done = false;
   while (iter <= a.itermax) {
-    if (rho == 0.0) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
+    if (is_zero(sh.rho)) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
+    const double beta = sh.beta, omega0 = sh.omega;
     acc = 0.0;
     // The vector passes load each row's operands one row ahead (rows_ahead)
     rows_ahead(
         tid, stride, n, [&](int i) { return make_double3(a.r[i], a.v[i], a.p[i]); },
         [&](int i, const double3& o) {
-          const double ni = (iter == 1) ? o.x : fma(beta, fma(-omega, o.y, o.z), o.x);
+          const double ni = (iter == 1) ? o.x : fma(beta, fma(-omega0, o.y, o.z), o.x);
           a.p[i] = ni;
           acc += ni;
         });
     double mean = 0.0;
     if (NONULL) {
-      write_partials(acc, 0.0, 1, part, sh);
-      if (!grid_sync(s)) return;
-      reduce_partials(part, nb, 1, red, shv, [=](double* v) { v[0] = v[0] / dn; });
-      mean = red[0];
+      if (!grid_reduce<1>(s, acc, 0.0, part, sh, [=](double* v, int&) { v[0] = v[0] / dn; })) return;
+      mean = sh.v[0];
     }
-    if (!precond(a.p, mean, a.pi, part + 1 * (size_t)nb)) return;
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 1 * (size_t)nb, nb, 1, red, shv, [=](double* v) { v[0] = NONULL ? v[0] / dn : 0.0; });
-    const double mp = red[0];
+    if (!precond(a.p, mean, a.pi, acc)) return;
+    if (!grid_reduce<1>(s, acc, 0.0, part + 1 * (size_t)nb, sh,
+                        [=](double* v, int&) { v[0] = NONULL ? v[0] / dn : 0.0; }))
+      return;
+    const double mp = sh.v[0];
     acc = 0.0;
     if (use_mg) {
       rows_ahead(
@@ -1050,10 +1067,10 @@ __global__ void __launch_bounds__(TPB, VEBI_MIXED_MG_BLOCKS_PER_SM) k_bicgstab_m
         acc = fma(a.rb[i], vi, acc);
       }
     }
-    write_partials(acc, 0.0, 1, part + 2 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 2 * (size_t)nb, nb, 1, red, shv, [=](double* v) { v[0] = rho / (v[0] + 1.0e-15); });
-    alpha = red[0];
+    if (!grid_reduce<1>(s, acc, 0.0, part + 2 * (size_t)nb, sh,
+                        [&](double* v, int&) { sh.alpha = sh.rho / (v[0] + 1.0e-15); }))
+      return;
+    const double alpha = sh.alpha;
     double a2 = 0.0;
     acc = 0.0;
     rows_ahead(
@@ -1064,23 +1081,27 @@ __global__ void __launch_bounds__(TPB, VEBI_MIXED_MG_BLOCKS_PER_SM) k_bicgstab_m
           acc = fma(si, si, acc);
           a2 += si;
         });
-    write_partials(acc, a2, 2, part + 4 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 4 * (size_t)nb, nb, 2, red, shv, [=](double* v) { v[1] = v[1] / dn; });
-    const double n2s = red[0];
-    const double mean_s = red[1];
-    if (iter == 1) n2s0 = (n2s <= small) ? 1.0 : n2s;
-    if (n2s <= a.tol * a.tol * n2s0) {
+    // |s|^2 against the first one (1 when small), and the mean of s
+    if (!grid_reduce<2>(s, acc, a2, part + 4 * (size_t)nb, sh, [&](double* v, int& flag) {
+          sh.n2 = v[0];
+          if (iter == 1) sh.n2s0 = (v[0] <= small) ? 1.0 : v[0];
+          flag = v[0] <= a.tol * a.tol * sh.n2s0;
+          v[1] = v[1] / dn;
+        }))
+      return;
+    const double mean_s = sh.v[1];
+    if (sh.flag) {
       for (int i = tid; i < n; i += stride)
         a.x[i] = fma(alpha, (use_mg ? pd[i] : join2(a.pi[i])) - mp, a.x[i]);
-      resid = sqrt(n2s / n2s0);
+      at_s = true;
       done = true;
       break;
     }
-    if (!precond(a.s, NONULL ? mean_s : 0.0, a.si, part + 3 * (size_t)nb)) return;
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 3 * (size_t)nb, nb, 1, red, shv, [=](double* v) { v[0] = NONULL ? v[0] / dn : 0.0; });
-    const double ms = red[0];
+    if (!precond(a.s, NONULL ? mean_s : 0.0, a.si, acc)) return;
+    if (!grid_reduce<1>(s, acc, 0.0, part + 3 * (size_t)nb, sh,
+                        [=](double* v, int&) { v[0] = NONULL ? v[0] / dn : 0.0; }))
+      return;
+    const double ms = sh.v[0];
     acc = 0.0;
     a2 = 0.0;
     if (use_mg) {
@@ -1100,19 +1121,21 @@ __global__ void __launch_bounds__(TPB, VEBI_MIXED_MG_BLOCKS_PER_SM) k_bicgstab_m
         a2 = fma(ti, ti, a2);
       }
     }
-    write_partials(acc, a2, 2, part + 6 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 6 * (size_t)nb, nb, 2, red, shv, [](double* v) { v[0] = v[0] / (v[1] + 1.0e-15); });
-    omega = red[0];
+    if (!grid_reduce<2>(s, acc, a2, part + 6 * (size_t)nb, sh, [&](double* v, int&) {
+          sh.omega = v[0] / (v[1] + 1.0e-15);
+          v[2] = fma(sh.alpha, mp, sh.omega * ms);  // the two mean shifts of x folded into one
+        }))
+      return;
+    const double alpha1 = sh.alpha, omega = sh.omega;
     acc = 0.0;
     a2 = 0.0;
-    // x += alpha (p_hat - mp) + omega (s_hat - ms), with the two mean shifts folded into one
-    const double xshift = fma(alpha, mp, omega * ms);
+    // x += alpha (p_hat - mp) + omega (s_hat - ms)
+    const double xshift = sh.v[2];
     struct XRow {
       double p, s, x, t, sv, rb;
     };
     auto xr_update = [&](int i, const XRow& o) {
-      a.x[i] = fma(omega, o.s, fma(alpha, o.p, o.x - xshift));
+      a.x[i] = fma(omega, o.s, fma(alpha1, o.p, o.x - xshift));
       const double ri = fma(-omega, o.t, o.sv);
       a.r[i] = ri;
       acc = fma(ri, ri, acc);
@@ -1127,28 +1150,24 @@ __global__ void __launch_bounds__(TPB, VEBI_MIXED_MG_BLOCKS_PER_SM) k_bicgstab_m
           tid, stride, n,
           [&](int i) { return XRow{join2(a.pi[i]), join2(a.si[i]), a.x[i], a.t[i], a.s[i], a.rb[i]}; }, xr_update);
     }
-    write_partials(acc, a2, 2, part + 8 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    // v[2] = the relative residual, v[3] = the next iteration's beta from the new rho v[1]
-    reduce_partials(part + 8 * (size_t)nb, nb, 2, red, shv, [=](double* v) {
-      const double r0 = iter == 1 ? ((v[0] <= small) ? 1.0 : v[0]) : n2r0;
-      v[2] = sqrt(v[0] / r0);
-      v[3] = v[1] / (rho + 1.0e-15) * alpha / (omega + 1.0e-15);
-    });
-    const double n2r = red[0];
-    if (iter == 1) n2r0 = (n2r <= small) ? 1.0 : n2r;
-    resid = red[2];
-    if (n2r <= a.tol * a.tol * n2r0) { done = true; break; }
+    // |r|^2 against the first one (1 when small), the new rho and the next iteration's beta
+    if (!grid_reduce<2>(s, acc, a2, part + 8 * (size_t)nb, sh, [&](double* v, int& flag) {
+          sh.n2 = v[0];
+          if (iter == 1) sh.n2r0 = (v[0] <= small) ? 1.0 : v[0];
+          flag = v[0] <= a.tol * a.tol * sh.n2r0;
+          sh.beta = v[1] / (sh.rho + 1.0e-15) * sh.alpha / (sh.omega + 1.0e-15);
+          sh.rho = v[1];
+        }))
+      return;
+    if (sh.flag) { done = true; break; }
     iter = iter + 1;
-    rho = red[1];
-    beta = red[3];
   }
   if (!done) warn |= VEBI_WARN_MAXITER;
   for (int i = tid; i < n; i += stride) a.P[i] = a.x[i];
   if (tid == 0) {
     s->ls_iters = iter;
     s->ls_iters_total += iter;
-    s->ls_residual = resid;
+    s->ls_residual = sqrt(sh.n2 / (at_s ? sh.n2s0 : sh.n2r0));
     atomicOr(&s->warnings, warn);
   }
 }
@@ -1221,9 +1240,9 @@ void launch_ppe_mg_mixed(Ctx& x) {
   MgMxArgs m{MxArgs{d.bx, d.br, d.brb, d.bv, d.bp, d.bs, d.bt, d.bM, d.partials, d.p, d.pi2, d.si2, d.ppe_B,
                     d.rowsum, d.ppe_val32, d.ppe_col, d.ij_count, d.s, (long long)c.npfb, c.npfb, c.itermax, c.tol,
                     c.warm_start},
-             x.d_mg, (int)x.mg.size(), tail, d.cellpart, d.cell_start, d.cell_cnt, d.ip, (float*)x.mg_z,
+             MgCoarse{x.d_mg, (int)x.mg.size(), tail, x.mg_kinv, x.mg_kinv_ok, x.mg_g32}, d.cellpart, d.cell_start, d.cell_cnt, d.ip, (float*)x.mg_z,
              (float*)x.mg_fr, (float*)x.mg_dinv0, x.mg_ragg, x.mg_rx, x.mg_rval, (const float*)x.mg_rv9, c.ncx,
-             (float*)x.mg_w, x.mg_kinv, x.mg_kinv_ok, x.mg_g32, (float*)x.mg_rsum, x.mg_q32, d.ppe_diag};
+             (float*)x.mg_w, (float*)x.mg_rsum, x.mg_q32, d.ppe_diag};
   if (c.open_domain == 0) cudaLaunchKernelEx(&cfg, k_bicgstab_mixed_mg<true>, m);
   else cudaLaunchKernelEx(&cfg, k_bicgstab_mixed_mg<false>, m);
   x.launches++;
@@ -1250,8 +1269,8 @@ void launch_ppe_mg(Ctx& x) {
   MgArgs m{BiArgs{d.bx, d.br, d.brb, d.bv, d.bp, d.bpi, d.bs, d.bsi, d.bt, d.bM, d.partials, d.p, d.ppe_B,
                   d.ppe_diag, d.ppe_val, d.ppe_col, d.ij_count, d.s, (long long)c.npfb, c.npfb, c.itermax, c.tol,
                   c.warm_start},
-           x.d_mg, nl, tail, d.cellpart, d.cell_start, d.cell_cnt, d.ip, x.mg_z, x.mg_fr, x.mg_dinv0, x.mg_rsum,
-           x.mg_ragg, x.mg_rx, x.mg_rval, x.mg_rv9, c.ncx, x.mg_w, x.mg_kinv, x.mg_kinv_ok};
+           MgCoarse{x.d_mg, nl, tail, x.mg_kinv, x.mg_kinv_ok, nullptr}, d.cellpart, d.cell_start, d.cell_cnt, d.ip, x.mg_z, x.mg_fr, x.mg_dinv0, x.mg_rsum,
+           x.mg_ragg, x.mg_rx, x.mg_rval, x.mg_rv9, c.ncx, x.mg_w};
   if (c.open_domain == 0) cudaLaunchKernelEx(&cfg, k_bicgstab_mg<true>, m);
   else cudaLaunchKernelEx(&cfg, k_bicgstab_mg<false>, m);
   x.launches++;

@@ -70,11 +70,6 @@ __global__ void k_ppe_mean(Consts c, Dev d, int nblk) {
 // sum_k A_ik, which is exactly 0 for such a row.  This GPU issues FP64 at 1/64 of the FP32 rate,
 // and the FP64 form of this pass was bound by it.  keep64 (the adjoint's recompute of a
 // recorded step, which tapes the FP64 matrix) takes the FP64 form.
-__device__ __forceinline__ double plus_zero(double x) {  // 0.0 + x without the FP64 pipe
-  const long long b = __double_as_longlong(x);
-  return __longlong_as_double(b == (long long)0x8000000000000000ull ? 0ll : b);
-}
-
 __global__ void k_ppe_assemble(Consts c, Dev d, const float* __restrict__ wL32, int keep64) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c.npfb) return;
@@ -192,18 +187,17 @@ __global__ void k_ppe_assemble(Consts c, Dev d, const float* __restrict__ wL32, 
 // of dividing by it (inverseM), which changes results by rounding only.
 template <bool NONULL>
 __global__ void __launch_bounds__(TPB, 5) k_bicgstab(BiArgs a) {
-  __shared__ double sh[64];
-  __shared__ double shv[4];
+  __shared__ SolverSh sh;
   const int n = a.n;
   const int nb = gridDim.x;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int stride = gridDim.x * blockDim.x;
   Scal* s = a.sc;
-  if (*((volatile int*)&s->first_error)) return;  // this state already failed a step
+  if (state_failed(s)) return;
+  solver_begin(sh);
   double* part = a.part;
   const double rinv1 = 1.0 / (1.0 + 1.0e-15);
   const double small = NONULL ? 1.0e-6 : 4.0;  // open solver: the integer expression 10-6
-  double red[4];
   double acc = 0.0;
   if (a.warm) {  // x0 = P of the previous step: r0 = B - A x0 (the SpMV reads x through pinv)
     for (int i = tid; i < n; i += stride) {
@@ -225,17 +219,14 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab(BiArgs a) {
     acc = fma(bi, bi, acc);
   }
   // slot 10 for the initial reduction: slot 0 is rewritten before every block has read it
-  write_partials(acc, 0.0, 1, part + 10 * (size_t)nb, sh);
-  if (!grid_sync(s)) return;
-  reduce_partials(part + 10 * (size_t)nb, nb, 1, red, shv);
-  double rho = red[0], alpha = 1.0, omega = 1.0;
-  double n2r0 = 1.0, n2s0 = 1.0, resid = 0.0;
-  double beta = 0.0;  // for iteration 2 on, derived with the previous iteration's last reduction
+  if (!grid_reduce<1>(s, acc, 0.0, part + 10 * (size_t)nb, sh, [&](double* v, int&) { sh.rho = v[0]; })) return;
+  bool at_s = false;  // the solve stopped on s, not on r
   int iter = 1, warn = 0;
   bool done = false;
   const double dn = (double)n;
   while (iter <= a.itermax) {
-    if (rho == 0.0) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
+    if (is_zero(sh.rho)) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
+    const double beta = sh.beta, omega0 = sh.omega;
     // p = r + beta (p - omega v).  The vector passes load each row's operands one row ahead
     // (rows_ahead), so a row's loads are in flight before the previous row's stores: the
     // compiler cannot move a load of one array above a store to another that may alias it.
@@ -243,16 +234,13 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab(BiArgs a) {
     rows_ahead(
         tid, stride, n, [&](int i) { return make_double3(a.r[i], a.v[i], a.p[i]); },
         [&](int i, const double3& o) {
-          const double pi = (iter == 1) ? o.x : fma(beta, fma(-omega, o.y, o.z), o.x);
+          const double pi = (iter == 1) ? o.x : fma(beta, fma(-omega0, o.y, o.z), o.x);
           a.p[i] = pi;
           acc += pi;
         });
-    double* slot = part;
     if (NONULL) {
-      write_partials(acc, 0.0, 1, slot, sh);
-      if (!grid_sync(s)) return;
-      reduce_partials(slot, nb, 1, red, shv, [=](double* v) { v[0] = v[0] / dn; });
-      const double mean = red[0];
+      if (!grid_reduce<1>(s, acc, 0.0, part, sh, [=](double* v, int&) { v[0] = v[0] / dn; })) return;
+      const double mean = sh.v[0];
       rows_ahead(
           tid, stride, n, [&](int i) { return a.p[i]; },
           [&](int i, double p) {
@@ -273,11 +261,10 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab(BiArgs a) {
       a.v[i] = vi;
       acc = fma(a.rb[i], vi, acc);
     }
-    slot = part + 2 * (size_t)nb;
-    write_partials(acc, 0.0, 1, slot, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(slot, nb, 1, red, shv, [=](double* v) { v[0] = rho / (v[0] + 1.0e-15); });
-    alpha = red[0];
+    if (!grid_reduce<1>(s, acc, 0.0, part + 2 * (size_t)nb, sh,
+                        [&](double* v, int&) { sh.alpha = sh.rho / (v[0] + 1.0e-15); }))
+      return;
+    const double alpha = sh.alpha;
     // s = r - alpha v ; |s|^2 ; sum(s)
     double a2 = 0.0;
     acc = 0.0;
@@ -289,16 +276,18 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab(BiArgs a) {
           acc = fma(si, si, acc);
           a2 += si;
         });
-    slot = part + 4 * (size_t)nb;
-    write_partials(acc, a2, 2, slot, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(slot, nb, 2, red, shv, [=](double* v) { v[1] = v[1] / dn; });
-    const double n2s = red[0];
-    const double mean_s = red[1];
-    if (iter == 1) n2s0 = (n2s <= small) ? 1.0 : n2s;
-    if (n2s <= a.tol * a.tol * n2s0) {
+    // |s|^2 against the first one (1 when small), and the mean of s
+    if (!grid_reduce<2>(s, acc, a2, part + 4 * (size_t)nb, sh, [&](double* v, int& flag) {
+          sh.n2 = v[0];
+          if (iter == 1) sh.n2s0 = (v[0] <= small) ? 1.0 : v[0];
+          flag = v[0] <= a.tol * a.tol * sh.n2s0;
+          v[1] = v[1] / dn;
+        }))
+      return;
+    const double mean_s = sh.v[1];
+    if (sh.flag) {
       for (int i = tid; i < n; i += stride) a.x[i] = fma(alpha, a.pinv[i], a.x[i]);
-      resid = sqrt(n2s / n2s0);
+      at_s = true;
       done = true;
       break;
     }
@@ -320,11 +309,10 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab(BiArgs a) {
       acc = fma(ti, a.s[i], acc);
       a2 = fma(ti, ti, a2);
     }
-    slot = part + 6 * (size_t)nb;
-    write_partials(acc, a2, 2, slot, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(slot, nb, 2, red, shv, [](double* v) { v[0] = v[0] / (v[1] + 1.0e-15); });
-    omega = red[0];
+    if (!grid_reduce<2>(s, acc, a2, part + 6 * (size_t)nb, sh,
+                        [&](double* v, int&) { sh.omega = v[0] / (v[1] + 1.0e-15); }))
+      return;
+    const double alpha1 = sh.alpha, omega = sh.omega;
     // x, r update ; |r|^2 ; (r_bar, r) for the next rho
     acc = 0.0;
     a2 = 0.0;
@@ -334,35 +322,30 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab(BiArgs a) {
     rows_ahead(
         tid, stride, n, [&](int i) { return XRow{a.sinv[i], a.pinv[i], a.x[i], a.t[i], a.s[i], a.rb[i]}; },
         [&](int i, const XRow& o) {
-          a.x[i] = fma(omega, o.s, fma(alpha, o.p, o.x));
+          a.x[i] = fma(omega, o.s, fma(alpha1, o.p, o.x));
           const double ri = fma(-omega, o.t, o.sv);
           a.r[i] = ri;
           acc = fma(ri, ri, acc);
           a2 = fma(o.rb, ri, a2);
         });
-    slot = part + 8 * (size_t)nb;
-    write_partials(acc, a2, 2, slot, sh);
-    if (!grid_sync(s)) return;
-    // v[2] = the relative residual, v[3] = the next iteration's beta from the new rho v[1]
-    reduce_partials(slot, nb, 2, red, shv, [=](double* v) {
-      const double r0 = iter == 1 ? ((v[0] <= small) ? 1.0 : v[0]) : n2r0;
-      v[2] = sqrt(v[0] / r0);
-      v[3] = v[1] / (rho + 1.0e-15) * alpha / (omega + 1.0e-15);
-    });
-    const double n2r = red[0];
-    if (iter == 1) n2r0 = (n2r <= small) ? 1.0 : n2r;
-    resid = red[2];
-    if (n2r <= a.tol * a.tol * n2r0) { done = true; break; }
+    // |r|^2 against the first one (1 when small), the new rho and the next iteration's beta
+    if (!grid_reduce<2>(s, acc, a2, part + 8 * (size_t)nb, sh, [&](double* v, int& flag) {
+          sh.n2 = v[0];
+          if (iter == 1) sh.n2r0 = (v[0] <= small) ? 1.0 : v[0];
+          flag = v[0] <= a.tol * a.tol * sh.n2r0;
+          sh.beta = v[1] / (sh.rho + 1.0e-15) * sh.alpha / (sh.omega + 1.0e-15);
+          sh.rho = v[1];
+        }))
+      return;
+    if (sh.flag) { done = true; break; }
     iter = iter + 1;
-    rho = red[1];
-    beta = red[3];
   }
   if (!done) warn |= VEBI_WARN_MAXITER;
   for (int i = tid; i < n; i += stride) a.P[i] = a.x[i];
   if (tid == 0) {
     s->ls_iters = iter;
     s->ls_iters_total += iter;
-    s->ls_residual = resid;
+    s->ls_residual = sqrt(sh.n2 / (at_s ? sh.n2s0 : sh.n2r0));
     atomicOr(&s->warnings, warn);
   }
 }
@@ -470,18 +453,17 @@ namespace vebi {
 
 template <bool NONULL>
 __global__ void __launch_bounds__(TPB, 5) k_bicgstab_mixed(MxArgs a) {
-  __shared__ double sh[64];
-  __shared__ double shv[4];
+  __shared__ SolverSh sh;
   const int n = a.n;
   const int nb = gridDim.x;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int stride = gridDim.x * blockDim.x;
   Scal* s = a.sc;
-  if (*((volatile int*)&s->first_error)) return;  // this state already failed a step
+  if (state_failed(s)) return;
+  solver_begin(sh);
   double* part = a.part;
   const double rinv1 = 1.0 / (1.0 + 1.0e-15);
   const double small = NONULL ? 1.0e-6 : 4.0;
-  double red[4];
   double acc = 0.0;
   if (a.warm) {  // x0 = P of the previous step
     for (int i = tid; i < n; i += stride) {
@@ -501,32 +483,27 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab_mixed(MxArgs a) {
     a.p[i] = 0.0;
     acc = fma(bi, bi, acc);
   }
-  write_partials(acc, 0.0, 1, part + 10 * (size_t)nb, sh);
-  if (!grid_sync(s)) return;
-  reduce_partials(part + 10 * (size_t)nb, nb, 1, red, shv);
-  double rho = red[0], alpha = 1.0, omega = 1.0;
-  double n2r0 = 1.0, n2s0 = 1.0, resid = 0.0;
-  double beta = 0.0;  // for iteration 2 on, derived with the previous iteration's last reduction
+  if (!grid_reduce<1>(s, acc, 0.0, part + 10 * (size_t)nb, sh, [&](double* v, int&) { sh.rho = v[0]; })) return;
+  bool at_s = false;  // the solve stopped on s, not on r
   int iter = 1, warn = 0;
   bool done = false;
   const double dn = (double)n;
   while (iter <= a.itermax) {
-    if (rho == 0.0) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
+    if (is_zero(sh.rho)) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
+    const double beta = sh.beta, omega0 = sh.omega;
     acc = 0.0;
     // vector passes: each row's operands loaded one row ahead (rows_ahead)
     rows_ahead(
         tid, stride, n, [&](int i) { return make_double3(a.r[i], a.v[i], a.p[i]); },
         [&](int i, const double3& o) {
-          const double pi = (iter == 1) ? o.x : fma(beta, fma(-omega, o.y, o.z), o.x);
+          const double pi = (iter == 1) ? o.x : fma(beta, fma(-omega0, o.y, o.z), o.x);
           a.p[i] = pi;
           acc += pi;
         });
     double mean = 0.0;
     if (NONULL) {
-      write_partials(acc, 0.0, 1, part, sh);
-      if (!grid_sync(s)) return;
-      reduce_partials(part, nb, 1, red, shv, [=](double* v) { v[0] = v[0] / dn; });
-      mean = red[0];
+      if (!grid_reduce<1>(s, acc, 0.0, part, sh, [=](double* v, int&) { v[0] = v[0] / dn; })) return;
+      mean = sh.v[0];
     }
     rows_ahead(
         tid, stride, n, [&](int i) { return make_double2(a.p[i], NONULL ? rinv1 : a.rinvM[i]); },
@@ -542,10 +519,10 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab_mixed(MxArgs a) {
       a.v[i] = vi;
       acc = fma(a.rb[i], vi, acc);
     }
-    write_partials(acc, 0.0, 1, part + 2 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 2 * (size_t)nb, nb, 1, red, shv, [=](double* v) { v[0] = rho / (v[0] + 1.0e-15); });
-    alpha = red[0];
+    if (!grid_reduce<1>(s, acc, 0.0, part + 2 * (size_t)nb, sh,
+                        [&](double* v, int&) { sh.alpha = sh.rho / (v[0] + 1.0e-15); }))
+      return;
+    const double alpha = sh.alpha;
     double a2 = 0.0;
     acc = 0.0;
     rows_ahead(
@@ -556,15 +533,18 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab_mixed(MxArgs a) {
           acc = fma(si, si, acc);
           a2 += si;
         });
-    write_partials(acc, a2, 2, part + 4 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 4 * (size_t)nb, nb, 2, red, shv, [=](double* v) { v[1] = v[1] / dn; });
-    const double n2s = red[0];
-    const double mean_s = red[1];
-    if (iter == 1) n2s0 = (n2s <= small) ? 1.0 : n2s;
-    if (n2s <= a.tol * a.tol * n2s0) {
+    // |s|^2 against the first one (1 when small), and the mean of s
+    if (!grid_reduce<2>(s, acc, a2, part + 4 * (size_t)nb, sh, [&](double* v, int& flag) {
+          sh.n2 = v[0];
+          if (iter == 1) sh.n2s0 = (v[0] <= small) ? 1.0 : v[0];
+          flag = v[0] <= a.tol * a.tol * sh.n2s0;
+          v[1] = v[1] / dn;
+        }))
+      return;
+    const double mean_s = sh.v[1];
+    if (sh.flag) {
       for (int i = tid; i < n; i += stride) a.x[i] = fma(alpha, join2(a.pi[i]), a.x[i]);
-      resid = sqrt(n2s / n2s0);
+      at_s = true;
       done = true;
       break;
     }
@@ -584,10 +564,10 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab_mixed(MxArgs a) {
       acc = fma(ti, a.s[i], acc);
       a2 = fma(ti, ti, a2);
     }
-    write_partials(acc, a2, 2, part + 6 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    reduce_partials(part + 6 * (size_t)nb, nb, 2, red, shv, [](double* v) { v[0] = v[0] / (v[1] + 1.0e-15); });
-    omega = red[0];
+    if (!grid_reduce<2>(s, acc, a2, part + 6 * (size_t)nb, sh,
+                        [&](double* v, int&) { sh.omega = v[0] / (v[1] + 1.0e-15); }))
+      return;
+    const double alpha1 = sh.alpha, omega = sh.omega;
     acc = 0.0;
     a2 = 0.0;
     struct XRow {
@@ -597,34 +577,30 @@ __global__ void __launch_bounds__(TPB, 5) k_bicgstab_mixed(MxArgs a) {
     rows_ahead(
         tid, stride, n, [&](int i) { return XRow{a.si[i], a.pi[i], a.x[i], a.t[i], a.s[i], a.rb[i]}; },
         [&](int i, const XRow& o) {
-          a.x[i] = fma(omega, join2(o.s), fma(alpha, join2(o.p), o.x));
+          a.x[i] = fma(omega, join2(o.s), fma(alpha1, join2(o.p), o.x));
           const double ri = fma(-omega, o.t, o.sv);
           a.r[i] = ri;
           acc = fma(ri, ri, acc);
           a2 = fma(o.rb, ri, a2);
         });
-    write_partials(acc, a2, 2, part + 8 * (size_t)nb, sh);
-    if (!grid_sync(s)) return;
-    // v[2] = the relative residual, v[3] = the next iteration's beta from the new rho v[1]
-    reduce_partials(part + 8 * (size_t)nb, nb, 2, red, shv, [=](double* v) {
-      const double r0 = iter == 1 ? ((v[0] <= small) ? 1.0 : v[0]) : n2r0;
-      v[2] = sqrt(v[0] / r0);
-      v[3] = v[1] / (rho + 1.0e-15) * alpha / (omega + 1.0e-15);
-    });
-    const double n2r = red[0];
-    if (iter == 1) n2r0 = (n2r <= small) ? 1.0 : n2r;
-    resid = red[2];
-    if (n2r <= a.tol * a.tol * n2r0) { done = true; break; }
+    // |r|^2 against the first one (1 when small), the new rho and the next iteration's beta
+    if (!grid_reduce<2>(s, acc, a2, part + 8 * (size_t)nb, sh, [&](double* v, int& flag) {
+          sh.n2 = v[0];
+          if (iter == 1) sh.n2r0 = (v[0] <= small) ? 1.0 : v[0];
+          flag = v[0] <= a.tol * a.tol * sh.n2r0;
+          sh.beta = v[1] / (sh.rho + 1.0e-15) * sh.alpha / (sh.omega + 1.0e-15);
+          sh.rho = v[1];
+        }))
+      return;
+    if (sh.flag) { done = true; break; }
     iter = iter + 1;
-    rho = red[1];
-    beta = red[3];
   }
   if (!done) warn |= VEBI_WARN_MAXITER;
   for (int i = tid; i < n; i += stride) a.P[i] = a.x[i];
   if (tid == 0) {
     s->ls_iters = iter;
     s->ls_iters_total += iter;
-    s->ls_residual = resid;
+    s->ls_residual = sqrt(sh.n2 / (at_s ? sh.n2s0 : sh.n2r0));
     atomicOr(&s->warnings, warn);
   }
 }

@@ -29,39 +29,8 @@ __device__ __forceinline__ unsigned long long bar_clock() {
 }
 #endif
 
-// bounded grid-wide barrier for a co-resident (cooperative) grid; false on error/timeout.
-// A block that polls more than `limit` times records VEBI_ERR_TIMEOUT and returns false, and so
-// does every block that arrives or polls after the error is recorded.
-__device__ __forceinline__ bool grid_sync_bounded(Scal* s, unsigned long long limit) {
 #ifdef VEBI_BARRIER_TIMESTAMPS
-  const unsigned long long ts_arrive = bar_clock();
-#endif
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned int* vgen = &s->bar_gen;
-    volatile int* verr = &s->error;
-    unsigned int g = *vgen;
-    __threadfence();
-    unsigned int arrived = atomicAdd((unsigned int*)&s->bar_count, 1u) + 1u;
-    if (arrived == gridDim.x) {
-      atomicExch((unsigned int*)&s->bar_count, 0u);
-      __threadfence();
-      atomicAdd((unsigned int*)&s->bar_gen, 1u);
-    } else {
-      unsigned long long spins = 0;
-      while (*vgen == g) {
-        if (*verr != 0) break;
-        if (++spins > limit) {
-          atomicCAS((int*)&s->error, 0, VEBI_ERR_TIMEOUT);
-          break;
-        }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-#ifdef VEBI_BARRIER_TIMESTAMPS
+__device__ __forceinline__ void bar_mark(unsigned long long ts_arrive) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     const unsigned int q = g_bar_n++;
     if (q < BAR_TS_MAX) {
@@ -78,34 +47,204 @@ __device__ __forceinline__ bool grid_sync_bounded(Scal* s, unsigned long long li
       g_bar_smid[blockIdx.x] = sm;
     }
   }
+}
+#define BAR_ARRIVE const unsigned long long ts_arrive_ = bar_clock()
+#define BAR_LEAVE bar_mark(ts_arrive_)
+#else
+#define BAR_ARRIVE (void)0
+#define BAR_LEAVE (void)0
 #endif
-  return *((volatile int*)&s->error) == 0;
+
+// ---- words that blocks of the grid signal each other through (gpu scope)
+__device__ __forceinline__ unsigned int atom_add_release(unsigned int* a, unsigned int v) {
+  unsigned int old;
+  asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(a), "r"(v) : "memory");
+  return old;
+}
+__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* a) {
+  unsigned int v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
+  return v;
+}
+
+// Poll *word until done(value); false when more than `limit` polls go by (VEBI_ERR_TIMEOUT is
+// recorded) or another block has recorded an error, looked at every 64th poll.  A poll is one
+// round trip to L2 (~0.5 us on GB300), so sleeping between polls only adds to the wait.
+template <class Done>
+__device__ __forceinline__ bool poll_bounded(const unsigned int* word, int* error, unsigned long long limit, Done done) {
+  for (unsigned long long spins = 0;; ++spins) {
+    if (done(ld_acquire(word))) return true;
+    if ((spins & 63) == 63 && *((volatile int*)error) != 0) return false;
+    if (spins >= limit) {
+      atomicCAS(error, 0, VEBI_ERR_TIMEOUT);
+      return false;
+    }
+  }
+}
+
+// Arrival and wait of one thread per block at the grid barrier.  Block 0 adds 2^31 less the
+// other blocks' number and every other block adds one, so the counter's top bit flips when all
+// have arrived and its low bits return to zero: one atomic per block and no reset, which a
+// waiter would otherwise see one round trip later.
+__device__ __forceinline__ bool barrier_arrive_wait(unsigned int* count, int* error, unsigned long long limit) {
+  const unsigned int old = atom_add_release(count, blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1u) : 1u);
+  return poll_bounded(count, error, limit, [=](unsigned int cur) { return ((cur ^ old) & 0x80000000u) != 0u; });
+}
+
+// bounded grid-wide barrier for a co-resident (cooperative) grid; false on error/timeout.
+// A block that polls more than `limit` times records VEBI_ERR_TIMEOUT and returns false, and so
+// does every block that is waiting, or comes to wait, after an error is recorded.  The writes of
+// every thread before it are visible to every thread after it: the block barriers order them
+// with thread 0's release and acquire.
+// Measured with 7 / 152 / 760 blocks of 256 threads: 0.68 / 1.17 / 2.6 us; with a reset counter,
+// a generation word and fences around volatile polls it was 1.6 / 2.9 / 7.4 us.
+__device__ __forceinline__ bool grid_sync_bounded(Scal* s, unsigned long long limit) {
+  BAR_ARRIVE;
+  __syncthreads();
+  int bad = 0;
+  if (threadIdx.x == 0) bad = barrier_arrive_wait(&s->bar_count, &s->error, limit) ? 0 : 1;
+  bad = __syncthreads_or(bad);
+  BAR_LEAVE;
+  return bad == 0;
 }
 
 __device__ __forceinline__ bool grid_sync(Scal* s) { return grid_sync_bounded(s, SPIN_LIMIT); }
 
-// Sum of the block partials of `slot` in a fixed order; identical in every block.  `post`,
-// run by thread 0 alone on the nval sums in v[0..3] before they are shared, derives the
-// iteration's scalars (its divisions and square roots) in place: this GPU issues FP64 at 1/64
-// of the FP32 rate, so uniform FP64 work is done once per block rather than once per warp.
-struct NoPost {
-  __device__ void operator()(double*) const {}
+// a solve starts only on a state without a recorded failure (of this step or an earlier one)
+__device__ __forceinline__ bool state_failed(const Scal* s) {
+  return *((const volatile int*)&s->first_error) != 0 || *((const volatile int*)&s->error) != 0;
+}
+
+__device__ __forceinline__ bool is_zero(double v) {  // v == 0.0 without the FP64 pipe
+  return ((unsigned long long)__double_as_longlong(v) << 1) == 0ull;
+}
+
+// ---- grid-wide sums
+// Shared memory of a solver block: the reductions' work space, the last reduction's results (up
+// to four values derived from the sums and a flag, the same in every block) and the iteration's
+// scalars, which thread 0 updates and every thread reads where a pass needs one.
+struct SolverSh {
+  double x[2][TPB];       // one value per thread
+  double y[TPB];          // after the first tree level of two values
+  double w[2][TPB / 32];  // warp sums
+  double v[4];
+  double rho, alpha, omega, beta, n2r0, n2s0, n2;
+  int flag;
 };
-template <class Post = NoPost>
-__device__ __forceinline__ void reduce_partials(const double* part, int nb, int nval, double* out, double* shv,
-                                                Post post = Post()) {
-  if (threadIdx.x < 32) {
-    for (int q = 0; q < nval; ++q) {
-      double v = 0.0;
-      for (int b = threadIdx.x; b < nb; b += 32) v += __ldcg(part + (size_t)q * nb + b);
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (threadIdx.x == 0) shv[q] = v;
+
+__device__ __forceinline__ double plus_zero(double x) {  // 0.0 + x without the FP64 pipe
+  const long long b = __double_as_longlong(x);
+  return __longlong_as_double(b == (long long)0x8000000000000000ull ? 0ll : b);
+}
+
+// Block partial of one or two values into part[q*nb + blockIdx.x], by thread q.  The sums are
+// those of a shuffle tree over each warp (lane l + lane l+16, then 8, 4, 2, 1) and of the warps
+// in order.  An FP64 instruction holds a warp scheduler for 64-76 cycles on this GPU however few
+// of its lanes are active, so the tree is packed: the 16 sums of a warp's first level take half a
+// warp, and only as many warps run it as it fills (20 instructions a value in place of 40).
+template <int NV>
+__device__ __forceinline__ void block_partial(double a, double b, double* part, SolverSh& sh) {
+  constexpr int W = TPB / 32;
+  const int t = threadIdx.x;
+  sh.x[0][t] = a;
+  if (NV > 1) sh.x[1][t] = b;
+  __syncthreads();
+  if (NV == 1) {
+    if (t < TPB / 2) {
+      const double* q = sh.x[0] + (t >> 4) * 32 + (t & 15);
+      double y = q[0] + q[16];
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o, 16);
+      if ((t & 15) == 0) sh.w[0][t >> 4] = y;
     }
-    if (threadIdx.x == 0) post(shv);
+  } else {
+    const double* q = sh.x[t / (TPB / 2)] + ((t % (TPB / 2)) >> 4) * 32 + (t & 15);
+    sh.y[t] = q[0] + q[16];
+    __syncthreads();
+    if (t < TPB / 2) {
+      const double* r = sh.y + (t >> 3) * 16 + (t & 7);
+      double y = r[0] + r[8];
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o, 8);
+      if ((t & 7) == 0) sh.w[(t >> 3) / W][(t >> 3) % W] = y;
+    }
   }
   __syncthreads();
-  for (int q = 0; q < 4; ++q) out[q] = shv[q];
+  if (t < NV) {
+    double v = plus_zero(sh.w[t][0]);
+#pragma unroll
+    for (int q = 1; q < W; ++q) v += sh.w[t][q];
+    part[(size_t)t * gridDim.x + blockIdx.x] = v;
+  }
+  if (t < 32) __syncwarp();
+}
+
+// Sum of the block partials of each value in a fixed order, by warp q for value q: lane l takes
+// blocks l, l+32, ... in order, then the lanes by a shuffle tree (levels that would only add the
+// zeros of lanes without a block are skipped).  One value: returned to thread 0; two: in sh.v.
+template <int NV>
+__device__ __forceinline__ double sum_partials(const double* part, int nb, SolverSh& sh) {
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double v = 0.0;
+  if (q < NV) {
+    const double* p = part + (size_t)q * nb;
+    if (lane < nb) v = plus_zero(__ldcg(p + lane));
+    int b = lane + 32;
+    for (; b + 32 * 7 < nb; b += 32 * 8) {
+      double u[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) u[e] = __ldcg(p + b + 32 * e);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v += u[e];
+    }
+    for (; b < nb; b += 32) v += __ldcg(p + b);
+    for (int o = 16; o > 0; o >>= 1)
+      if (o < nb) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (NV > 1 && lane == 0) sh.v[q] = v;
+  }
+  if (NV > 1) __syncthreads();
+  return v;
+}
+
+// every solver's first statement; the caller's first barrier orders it before any use
+__device__ __forceinline__ void solver_begin(SolverSh& sh) {
+  if (threadIdx.x == 0) {
+    sh.alpha = sh.omega = sh.n2r0 = sh.n2s0 = 1.0;
+    sh.beta = sh.n2 = 0.0;
+  }
+}
+
+// The part of grid_reduce that does not depend on the caller's post, one copy per kernel: the
+// sums in sh.v[0..NV-1] for thread 0.
+template <int NV>
+static __device__ __noinline__ bool grid_sums(Scal* s, double a, double b, double* part, SolverSh& sh) {
+  block_partial<NV>(a, b, part, sh);
+  int bad = 0;
+  if (threadIdx.x == 0) bad = barrier_arrive_wait(&s->bar_count, &s->error, SPIN_LIMIT) ? 0 : 1;
+  if (__syncthreads_or(bad)) return false;
+  const double v = sum_partials<NV>(part, gridDim.x, sh);
+  if (NV == 1 && threadIdx.x == 0) sh.v[0] = v;
+  return true;
+}
+
+// Grid-wide sums of one or two values, which are also a grid barrier; false on error/timeout.
+// post(v, flag), run by thread 0 on the sums v[0..NV-1], derives the iteration's scalars in
+// v[0..3], in sh and in a flag (its divisions, square roots and comparisons), so uniform FP64
+// work is done once per block and not by every warp.  Every block sums the partials itself: a
+// form in which the last block to arrive did it for all, at one more round trip, was slower from
+// 7 to 760 blocks (the 100k-particle FP64 solve 55.5 ms against 51.7).
+// `part` takes NV * gridDim.x block partials.
+template <int NV, class Post>
+__device__ __forceinline__ bool grid_reduce(Scal* s, double a, double b, double* part, SolverSh& sh, Post post) {
+  BAR_ARRIVE;
+  if (!grid_sums<NV>(s, a, b, part, sh)) return false;
+  if (threadIdx.x == 0) {
+    sh.flag = 0;
+    post(sh.v, sh.flag);
+  }
   __syncthreads();
+  BAR_LEAVE;
+  return true;
 }
 
 // A vector pass over the rows tid, tid + stride, ... with each row's operands loaded one row
@@ -123,27 +262,6 @@ __device__ __forceinline__ void rows_ahead(int tid, int stride, int n, Load load
     body(i, cur);
     cur = nxt;
   }
-}
-
-// block partial of one or two values into part[q*nb + blockIdx.x]
-__device__ __forceinline__ void write_partials(double a, double b, int nval, double* part, double* sh) {
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_down_sync(0xffffffffu, a, o);
-    if (nval > 1) b += __shfl_down_sync(0xffffffffu, b, o);
-  }
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) { sh[w] = a; sh[32 + w] = b; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double sa = 0.0, sb = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
-      sa += sh[q];
-      if (nval > 1) sb += sh[32 + q];
-    }
-    part[blockIdx.x] = sa;
-    if (nval > 1) part[gridDim.x + blockIdx.x] = sb;
-  }
-  __syncthreads();
 }
 
 // Solver arguments: only what the loop touches (keeps the kernel's register footprint small).
