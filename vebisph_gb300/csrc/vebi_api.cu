@@ -251,7 +251,9 @@ static int allocate_all(Ctx& x) {
   if (x.mg_blocks > part_blocks) part_blocks = x.mg_blocks;
   if (x.mg_blocks_mixed > part_blocks) part_blocks = x.mg_blocks_mixed;
   size_t coop_part = (size_t)part_blocks * 12;
-  A_(d.partials, (2 * np_part > coop_part ? 2 * np_part : coop_part) + 64);
+  size_t part = 2 * np_part > coop_part ? 2 * np_part : coop_part;
+  if (resident_partials(c.npfb) > part) part = resident_partials(c.npfb);
+  A_(d.partials, part + 64);
   A_(d.gpx, n); A_(d.gpy, n);
   if (x.precision == VEBI_PREC_MIXED) {
     A_(d.ppe_val32, E); A_(d.rowsum, n); A_(d.pi2, n); A_(d.si2, n);
@@ -803,6 +805,7 @@ int vebi_batch_create(const vebi_params* params, int32_t n, vebi_batch** out) {
       vebi_batch_destroy(b);
       return fail(st, "batch instance " + std::to_string(i) + ": " + m);
     }
+    c->x.in_batch = true;
     b->ctx.push_back(c);
   }
   *out = b;

@@ -31,6 +31,7 @@ struct Ctx {
   bool graph_used[2][VEBI_NSTAGES] = {};
   int coop_blocks = 0;       // persistent PPE grid (co-resident blocks)
   int coop_blocks_mixed = 0; // same for the mixed-precision solver
+  bool in_batch = false;     // one of a batch's instances: its solver leaves room on the SMs for the others'
   int solver_rows_per_thread = 1;  // batch tuning: rows per solver thread
   int mg_block_rows = MG_BLOCK_ROWS;  // batch tuning: coarse levels of at most this many rows run in one block
   int grid_gen = 0;                // bumped when a launch shape changes (captured graphs are stale)
@@ -71,6 +72,11 @@ struct Ctx {
 int run_one_step(Ctx& x, vebi_step_stats* stats);
 // the context behind a handle (nullptr for a null handle)
 Ctx* ctx_of(vebi_ctx* h);
+
+// the PPE solve spread over all SMs (vebi_resident.cu)
+struct BiArgs;
+size_t resident_partials(int n);
+bool launch_bicgstab_resident(Ctx& x, const BiArgs& a, bool nonull);
 
 // kernel launch with launch accounting and an immediate launch-error check
 #define VEBI_LAUNCH(x, kern, grid, block, ...)                         \

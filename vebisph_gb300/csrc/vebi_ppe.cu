@@ -365,6 +365,29 @@ void launch_ppe_mixed_solve(Ctx& x);
 void launch_ppe_mg(Ctx& x);
 void launch_ppe_rhs32(Ctx& x);
 
+// The FP64 solve on its grid: the resident kernel where it fits (one row per thread, outside a
+// batch, whose instances' solves share the SMs), else the persistent kernel, as a cooperative
+// launch (all blocks co-resident, so the grid barrier is safe).
+static void launch_bicgstab(Ctx& x, const BiArgs& a, bool nonull, int rows_per_thread) {
+  if (rows_per_thread == 1 && !x.in_batch && launch_bicgstab_resident(x, a, nonull)) return;
+  int nblk = x.coop_blocks;
+  const long long rows_per_block = (long long)TPB * rows_per_thread;
+  const long long need = (a.n + rows_per_block - 1) / rows_per_block;
+  if (need < nblk) nblk = (int)(need < 1 ? 1 : need);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nblk);
+  cfg.blockDim = dim3(TPB);
+  cfg.stream = x.st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (nonull) cudaLaunchKernelEx(&cfg, k_bicgstab<true>, a);
+  else cudaLaunchKernelEx(&cfg, k_bicgstab<false>, a);
+  x.launches++;
+}
+
 void launch_ppe(Ctx& x) {
   const Consts& c = x.c;
   int g = grid_for(c.npfb);
@@ -388,49 +411,17 @@ void launch_ppe(Ctx& x) {
     launch_ppe_mg(x);
     return;
   }
-  // persistent cooperative launch: all blocks co-resident, so the grid barrier is safe
-  int nblk = x.coop_blocks;
-  const long long rows_per_block = (long long)TPB * (x.solver_rows_per_thread > 0 ? x.solver_rows_per_thread : 1);
-  long long need = (c.npfb + rows_per_block - 1) / rows_per_block;
-  if (need < nblk) nblk = (int)(need < 1 ? 1 : need);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nblk);
-  cfg.blockDim = dim3(TPB);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = x.st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   const Dev& d = x.d;
   BiArgs a{d.bx, d.br, d.brb, d.bv, d.bp, d.bpi, d.bs, d.bsi, d.bt, d.bM, d.partials, d.p,
            d.ppe_B, d.ppe_diag, d.ppe_val, d.ppe_col, d.ij_count, d.s, (long long)c.npfb, c.npfb, c.itermax, c.tol,
            c.warm_start};
-  if (c.open_domain == 0) cudaLaunchKernelEx(&cfg, k_bicgstab<true>, a);
-  else cudaLaunchKernelEx(&cfg, k_bicgstab<false>, a);
-  x.launches++;
+  launch_bicgstab(x, a, c.open_domain == 0, x.solver_rows_per_thread > 0 ? x.solver_rows_per_thread : 1);
 }
 
 // The persistent FP64 BiCGSTAB on a caller's system (the adjoint's transposed PPE): the same
 // grid and kernels as the step's solve, other arrays.
-void launch_bicgstab_on(Ctx& x, const BiArgs& a, bool nonull) {
-  int nblk = x.coop_blocks;
-  const long long need = (a.n + TPB - 1) / TPB;
-  if (need < nblk) nblk = (int)(need < 1 ? 1 : need);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nblk);
-  cfg.blockDim = dim3(TPB);
-  cfg.stream = x.st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (nonull) cudaLaunchKernelEx(&cfg, k_bicgstab<true>, a);
-  else cudaLaunchKernelEx(&cfg, k_bicgstab<false>, a);
-  x.launches++;
-}
+void launch_bicgstab_on(Ctx& x, const BiArgs& a, bool nonull) { launch_bicgstab(x, a, nonull, 1); }
+
 
 }  // namespace vebi
 

@@ -1,0 +1,317 @@
+// vebi_resident.cu -- the FP64 BiCGSTAB of a small or medium PPE, spread over the whole GPU with
+// its vectors in registers.
+//
+//  SPARSE_PBICGSTAB_nonull (closed)       linear_solver.F90:275-425
+//  SPARSE_PBICGSTAB (open, Jacobi)        linear_solver.F90:82-227
+//
+// k_bicgstab (vebi_ppe.cu) gives each block 256 rows and each row one thread.  On a small system
+// that leaves SMs idle -- a 10k-row solve occupies 40 of 152 -- and each row walks its 44 slots
+// through two dependent trips to L2 per four slots, after every barrier.  Here the rows are dealt
+// in groups of 32 to one block per SM, up to 256 rows a block:
+//  * a product takes four lanes a row, one for each of the four interleaved accumulators of
+//    spmv_row, so a row waits for its slots' operands once; up to 56 slots of a row stay in its
+//    lanes' registers for the whole solve when a block has at most 128 rows;
+//  * each row's r, r_bar, v, p, s, t, x stay in its thread's registers: only the gathered vectors
+//    p_inv and s_inv and the reductions' partial sums pass through L2.
+// Every sum runs in k_bicgstab's order -- a shuffle tree over 32 rows, the eight groups of a
+// virtual block of 256 rows in sequence, the virtual blocks in lane order -- so the solution is
+// the same bit for bit, whatever the number of SMs.
+//
+// What bounds it.  FP64 issues one warp instruction per 64-76 cycles and scheduler on this GPU:
+// ~107 operations a row and iteration are 64 cycles per row of an SM (2 us at 66 rows).  The
+// dependent chain of an iteration is the rest: seven barriers of ~1.1 us, five sums of some 20
+// dependent adds (0.6-1 us with their load), six divisions of 0.27 us, two products' gathers.
+// Measured, ms per solve, k_bicgstab / this kernel: 1.7k rows x 60 iterations 2.39 / 1.21, 2.9k x
+// 75 2.48 / 1.36, 10k x 139 5.37 / 3.40, 20k x 363 14.9 / 12.1, 29k x 247 10.2 /
+// 9.8.
+#include "vebi_solver.cuh"
+
+namespace vebi {
+
+namespace {
+
+constexpr int RES_GROUP = 32;       // rows of a group (a warp's rows in the vector passes)
+constexpr int RES_VB = 8;           // groups of a virtual block (256 rows)
+constexpr int RES_MAX_ROWS = 256;   // rows of a block: four lanes a row fill it
+constexpr int RES_MAX_VB = 256;     // virtual blocks the shared table holds
+
+struct ResSh {
+  double vec[RES_MAX_ROWS];  // a product's results, by row of the block
+  double vb[2 * RES_MAX_VB]; // virtual-block sums
+  double v[2];
+  double rho, alpha, omega, beta, n2r0, n2s0, n2, mean;
+  int flag;
+};
+
+// the grid-wide sums of a and (NV = 2) b over all rows, a barrier among them: for thread 0 the
+// totals are in sh.v when this returns true
+template <int NV>
+__device__ __noinline__ bool res_sums(Scal* s, double a, double b, double* part, int gpb, int nvb, ResSh& sh) {
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  const int G = nvb * RES_VB, g0 = blockIdx.x * gpb;
+  if (w < gpb) {
+    double z;
+    if (NV == 1) {
+      z = a;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) z += __shfl_down_sync(0xffffffffu, z, o);
+    } else {  // both trees at once: lanes 0..15 carry a's, lanes 16..31 b's
+      const bool lo = lane < 16;
+      z = (lo ? a : b) + __shfl_xor_sync(0xffffffffu, lo ? b : a, 16);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) z += __shfl_down_sync(0xffffffffu, z, o, 16);
+    }
+    if ((lane == 0 || (NV > 1 && lane == 16)) && g0 + w < G) part[(size_t)(lane >> 4) * G + g0 + w] = z;
+  }
+  __syncthreads();
+  int bad = 0;
+  if (t == 0) bad = barrier_arrive_wait(&s->bar_count, &s->error, SPIN_LIMIT) ? 0 : 1;
+  if (__syncthreads_or(bad)) return false;
+  auto vb_sum = [&](int q, int vb) {  // a virtual block's eight group sums in sequence
+    const double2* p = reinterpret_cast<const double2*>(part + (size_t)q * G + (size_t)vb * RES_VB);
+    double2 u[RES_VB / 2];
+#pragma unroll
+    for (int k = 0; k < RES_VB / 2; ++k) u[k] = __ldcg(p + k);
+    double z = plus_zero(u[0].x) + u[0].y;
+#pragma unroll
+    for (int k = 1; k < RES_VB / 2; ++k) {
+      z += u[k].x;
+      z += u[k].y;
+    }
+    return z;
+  };
+  const bool spread = nvb > 32;  // over all threads, else each summing lane does its own
+  if (spread) {
+    for (int e = t; e < NV * nvb; e += blockDim.x) sh.vb[e] = vb_sum(e / nvb, e % nvb);
+    __syncthreads();
+  }
+  if (w < NV) {  // warp q: lane l adds virtual blocks l, l+32, ... in order, then the lanes' tree
+    double z = 0.0;
+    if (lane < nvb) z = plus_zero(spread ? sh.vb[w * nvb + lane] : vb_sum(w, lane));
+#pragma unroll 1
+    for (int e = lane + 32; e < nvb; e += 32) z += sh.vb[w * nvb + e];
+    for (int o = 16; o > 0; o >>= 1)
+      if (o < nvb) z += __shfl_down_sync(0xffffffffu, z, o);
+    if (lane == 0) sh.v[w] = z;
+  }
+  if (NV > 1) __syncthreads();
+  return true;
+}
+
+// grid_reduce over the resident layout: post() runs on thread 0 with the sums in sh.v
+template <int NV, class Post>
+__device__ __forceinline__ bool res_reduce(Scal* s, double a, double b, double* part, int gpb, int nvb, ResSh& sh,
+                                           Post post) {
+  if (!res_sums<NV>(s, a, b, part, gpb, nvb, sh)) return false;
+  if (threadIdx.x == 0) post();
+  __syncthreads();
+  return true;
+}
+
+// One of a row's four lanes: lane q has spmv_row's accumulator q, which takes slots q, q+4, ... of
+// the whole quads of slots; lane 0 also takes the diagonal before them and the up to three slots
+// after them.
+struct LaneRow {
+  int row, q, nq, cnt;  // row (or -1), lane, whole quads, slots
+  __device__ __forceinline__ LaneRow(const BiArgs& a, int row_, bool in)
+      : row(in ? row_ : -1), q((int)threadIdx.x & 3), nq(0), cnt(0) {
+    if (in) {
+      cnt = __ldg(a.cnt + row);
+      nq = cnt >> 2;
+    }
+  }
+  // N slots k(u), u = 0.. N-1, of which those with in(u): columns and values, then operands, then FMAs
+  template <int N, class Slot, class In>
+  __device__ __forceinline__ void slots(const BiArgs& a, const double* xv, double& b, Slot k, In in) const {
+    int c[N];
+    double v[N], x[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const long long o = (long long)k(u) * a.stride + row;
+      c[u] = in(u) ? __ldg(a.col + o) : 0;
+      v[u] = in(u) ? __ldg(a.val + o) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u) x[u] = in(u) ? __ldca(xv + c[u]) : 0.0;
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+      if (in(u)) b = fma(v[u], x[u], b);
+  }
+};
+
+// KEEP: this many quads of a row stay in registers for the whole solve (0: all come from L2)
+template <bool NONULL, int T_MAX, int KEEP>
+__global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gpb, int nvb) {
+  __shared__ ResSh sh;
+  const int n = a.n, t = threadIdx.x;
+  const int R = gpb * RES_GROUP, row0 = blockIdx.x * R;
+  Scal* s = a.sc;
+  if (state_failed(s)) return;
+  const double rinv1 = 1.0 / (1.0 + 1.0e-15);
+  const double small = NONULL ? 1.0e-6 : 4.0;  // open solver: the integer expression 10-6
+  const double dn = (double)n;
+  double* const part0 = a.part;
+  double* const part1 = a.part + 2 * (size_t)nvb * RES_VB;  // used in turn: a slow block may still read one
+  if (t == 0) {
+    sh.alpha = sh.omega = sh.n2r0 = sh.n2s0 = 1.0;
+    sh.beta = sh.n2 = 0.0;
+  }
+  // this thread's row in the vector passes
+  const int i = row0 + t;
+  const bool mine = t < R && i < n;
+  const int l = t >> 2;  // this lane's row of the block in the products
+  const LaneRow L(a, row0 + l, l < R && row0 + l < n);
+  int ck[KEEP ? KEEP : 1];
+  double vk[KEEP ? KEEP : 1];
+  double dk = 0.0;
+  if (L.row >= 0 && L.q == 0) dk = __ldg(a.diag + L.row);
+  if (KEEP && L.row >= 0) {
+#pragma unroll
+    for (int e = 0; e < KEEP; ++e) {
+      const long long o = (4ll * e + L.q) * a.stride + L.row;
+      ck[e] = e < L.nq ? __ldg(a.col + o) : 0;
+      vk[e] = e < L.nq ? __ldg(a.val + o) : 0.0;
+    }
+  }
+  // y = A x for the block's rows, to their threads (x complete and visible in every block)
+  auto product = [&](const double* xv) {
+    double b = 0.0;
+    if (L.row >= 0) {
+      if (KEEP) {
+        double x[KEEP ? KEEP : 1];
+#pragma unroll
+        for (int e = 0; e < KEEP; ++e) x[e] = e < L.nq ? __ldca(xv + ck[e]) : 0.0;
+        if (L.q == 0) b = dk * __ldca(xv + L.row);
+#pragma unroll
+        for (int e = 0; e < KEEP; ++e)
+          if (e < L.nq) b = fma(vk[e], x[e], b);
+      } else if (L.q == 0) {
+        b = dk * __ldca(xv + L.row);
+      }
+      constexpr int Q = KEEP ? 4 : 6;
+#pragma unroll 1
+      for (int m = KEEP; m < L.nq; m += Q)
+        L.slots<Q>(a, xv, b, [&](int u) { return 4 * (m + u) + L.q; }, [&](int u) { return m + u < L.nq; });
+      if (L.q == 0)
+        L.slots<3>(a, xv, b, [&](int u) { return 4 * L.nq + u; }, [&](int u) { return 4 * L.nq + u < L.cnt; });
+    }
+    b += __shfl_xor_sync(0xffffffffu, b, 1);  // (b0 + b1) + (b2 + b3)
+    b += __shfl_xor_sync(0xffffffffu, b, 2);
+    if (L.q == 0 && L.row >= 0) sh.vec[l] = b;
+    __syncthreads();
+    return mine ? sh.vec[t] : 0.0;
+  };
+  double r = 0.0, rb = 0.0, v = 0.0, p = 0.0, x = 0.0, rinvM = rinv1;
+  if (a.warm) {  // x0 = P of the previous step: r0 = B - A x0
+    if (mine) {
+      x = a.P[i];
+      a.pinv[i] = x;
+    }
+    if (!grid_sync(s)) return;
+    const double y = product(a.pinv);
+    if (mine) r = a.B[i] - y;
+    if (!grid_sync(s)) return;  // every product has read x0 before p_inv is written
+  } else if (mine) {
+    r = a.B[i];
+  }
+  rb = r;
+  if (!NONULL && mine) rinvM = 1.0 / (__ldg(a.diag + i) + 1.0e-15);
+  if (!res_reduce<1>(s, mine ? fma(r, r, 0.0) : 0.0, 0.0, part1, gpb, nvb, sh, [&]() { sh.rho = sh.v[0]; })) return;
+  int iter = 1, warn = 0;
+  bool done = false, at_s = false;
+  while (iter <= a.itermax) {
+    if (is_zero(sh.rho)) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
+    if (mine) p = iter == 1 ? r : fma(sh.beta, fma(-sh.omega, v, p), r);
+    if (NONULL) {
+      if (!res_reduce<1>(s, mine ? plus_zero(p) : 0.0, 0.0, part0, gpb, nvb, sh, [&]() { sh.mean = sh.v[0] / dn; }))
+        return;
+      p = p - sh.mean;
+    }
+    const double pinv = p * rinvM;
+    if (mine) a.pinv[i] = pinv;
+    if (!grid_sync(s)) return;
+    v = product(a.pinv);
+    if (!res_reduce<1>(s, mine ? fma(rb, v, 0.0) : 0.0, 0.0, part1, gpb, nvb, sh,
+                       [&]() { sh.alpha = sh.rho / (sh.v[0] + 1.0e-15); }))
+      return;
+    const double alpha = sh.alpha;
+    double sv = mine ? fma(-alpha, v, r) : 0.0;
+    if (!res_reduce<2>(s, mine ? fma(sv, sv, 0.0) : 0.0, mine ? plus_zero(sv) : 0.0, part0, gpb, nvb, sh, [&]() {
+          sh.n2 = sh.v[0];
+          if (iter == 1) sh.n2s0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
+          sh.flag = sh.v[0] <= a.tol * a.tol * sh.n2s0;
+          if (NONULL) sh.mean = sh.v[1] / dn;
+        }))
+      return;
+    if (sh.flag) {
+      x = fma(alpha, pinv, x);
+      done = at_s = true;
+      break;
+    }
+    if (NONULL) sv = sv - sh.mean;
+    const double sinv = sv * rinvM;
+    if (mine) a.sinv[i] = sinv;
+    if (!grid_sync(s)) return;
+    const double tv = product(a.sinv);
+    if (!res_reduce<2>(s, mine ? fma(tv, sv, 0.0) : 0.0, mine ? fma(tv, tv, 0.0) : 0.0, part1, gpb, nvb, sh,
+                       [&]() { sh.omega = sh.v[0] / (sh.v[1] + 1.0e-15); }))
+      return;
+    const double omega = sh.omega;
+    x = fma(omega, sinv, fma(alpha, pinv, x));
+    r = fma(-omega, tv, sv);
+    if (!res_reduce<2>(s, mine ? fma(r, r, 0.0) : 0.0, mine ? fma(rb, r, 0.0) : 0.0, part0, gpb, nvb, sh, [&]() {
+          sh.n2 = sh.v[0];
+          if (iter == 1) sh.n2r0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
+          sh.flag = sh.v[0] <= a.tol * a.tol * sh.n2r0;
+          sh.beta = sh.v[1] / (sh.rho + 1.0e-15) * alpha / (omega + 1.0e-15);
+          sh.rho = sh.v[1];
+        }))
+      return;
+    if (sh.flag) { done = true; break; }
+    iter = iter + 1;
+  }
+  if (!done) warn |= VEBI_WARN_MAXITER;
+  if (mine) a.P[i] = x;
+  if (blockIdx.x == 0 && t == 0) {
+    s->ls_iters = iter;
+    s->ls_iters_total += iter;
+    s->ls_residual = sqrt(sh.n2 / (at_s ? sh.n2s0 : sh.n2r0));
+    atomicOr(&s->warnings, warn);
+  }
+}
+
+}  // namespace
+
+// doubles of partial sums the resident solver needs for n rows
+size_t resident_partials(int n) { return 4 * (size_t)RES_VB * ((n + 255) / 256); }
+
+// Runs the solve when it fits: at most 256 rows (eight groups, four lanes a row) per SM, and a
+// caller whose k_bicgstab grid has one row per thread (ceil(n / 256) blocks, whose summation order
+// this kernel keeps).  false: not launched.  Above 256 rows an SM the FP64 pipe is busy either way:
+// 60k / 100k rows with two rows or one lane a row took 33 / 47 ms against k_bicgstab's 32 / 48.
+bool launch_bicgstab_resident(Ctx& x, const BiArgs& a, bool nonull) {
+  const int nvb = (a.n + TPB - 1) / TPB;
+  if (nvb > x.coop_blocks || nvb > RES_MAX_VB) return false;
+  const int gpb = (nvb * RES_VB + x.nsm - 1) / x.nsm;
+  if (gpb * RES_GROUP > RES_MAX_ROWS) return false;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((nvb * RES_VB + gpb - 1) / gpb);
+  cfg.blockDim = dim3(4 * gpb * RES_GROUP);
+  cfg.stream = x.st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  auto go = [&](auto closed, auto open) { return cudaLaunchKernelEx(&cfg, nonull ? closed : open, a, gpb, nvb); };
+  const cudaError_t e = cfg.blockDim.x <= 512 ? go(k_bicgstab_resident<true, 512, 14>, k_bicgstab_resident<false, 512, 14>)
+                                              : go(k_bicgstab_resident<true, 1024, 0>, k_bicgstab_resident<false, 1024, 0>);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  x.launches++;
+  return true;
+}
+
+}  // namespace vebi
