@@ -100,6 +100,7 @@ static int build_consts(Ctx& x) {
   c.coeff_polymeric = (1.0 - P.beta) * P.Pr / (P.Ra * P.El);
   c.coeff_theta = 1.0 / std::sqrt(P.Ra * P.Pr);
   c.wab1 = host_wab(c.ad_7, c.dx / c.h);
+  c.inv_wab1 = 1.0 / c.wab1;
   c.cell_size = 1.0 / c.uno_sup_size;
   c.tol = P.tol > 0 ? P.tol : 1.0e-8;
   c.itermax = P.itermax > 0 ? P.itermax : 1000;

@@ -209,6 +209,9 @@ __global__ void __launch_bounds__(TPB) k_neighbours(Consts c, Dev d) {
     const int icy = ic / c.ncx + 1;
     const int cxi = key % c.ncx, cyi = key / c.ncx;
     const bool e_ok = icx + 1 <= c.ncx, w_ok = icx - 1 >= 1, n_ok = icy + 1 <= c.ncy, s_ok = icy - 1 >= 1;
+    // The reference's column rule gives a particle of the last column no western cells, whose
+    // particles do see it: with a cut row the only pairs that one particle alone lists.
+    if (icx == 0) d.s->one_sided = 1;
     bool over = false;
     int* const out = d.ij_link + i;
     // the nine cells C, E, NE, SE, W, NW, SW, N, S as (dx + 1, dy + 1) in two bits each; the
@@ -256,6 +259,7 @@ __global__ void __launch_bounds__(TPB) k_neighbours(Consts c, Dev d) {
     }
     if (over) {
       set_error(d.s, VEBI_ERR_NEIGH_CAPACITY);
+      d.s->one_sided = 1;
       cnt = c.nplink;
     }
   }

@@ -9,8 +9,11 @@
 #include <stdint.h>
 
 #include "../../include/vebi.h"
+#include "vebi_fp64.cuh"
 
 namespace vebi {
+
+using fp::is_zero;
 
 constexpr double PI = 3.14159265358979323846;  // common_parameter.F90:12
 constexpr int TPB = 256;                         // threads per block of per-particle kernels
@@ -25,7 +28,7 @@ struct Consts {
   double bf[2];
   double dt_coef_cfl, dt_coef_visc, dt_visc;
   double coeff_solvent, coeff_polymeric, coeff_theta;
-  double wab1;                                      // Wab(dx/h) of shifting_forces
+  double wab1, inv_wab1;                            // Wab(dx/h) of shifting_forces, and 1/wab1
   double cell_size;                                 // 1/uno_sup_size: edge of a cell
   double tol;
   // boundary framework (IBOUND)
@@ -77,6 +80,7 @@ struct Scal {
   int refine_iters;
   int ls_iters_total;                // summed over the steps of one vebi_run_steps call
   int first_error;                   // first failing status since the last upload (sticky)
+  int one_sided;                     // some pairs are listed by one of their particles only (k_neighbours)
   int mg_fail;                       // multigrid set-up overflowed a coarse row: solve without it
   int n_near_pole;                   // particles whose conformation eigenvalues are < 1e-7 apart
   int n_near_pole_total;             // the same summed over the steps of one vebi_run_steps call

@@ -41,6 +41,7 @@ __global__ void k_step_reset(Scal* s, int npfb, int nbS) {
   s->rms_u = 0.0;
   s->bar_count = 0u;
   s->refine_iters = 0;
+  s->one_sided = 0;
   s->mg_fail = 0;
   s->n_near_pole = 0;
 }

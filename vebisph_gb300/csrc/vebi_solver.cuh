@@ -115,10 +115,6 @@ __device__ __forceinline__ bool state_failed(const Scal* s) {
   return *((const volatile int*)&s->first_error) != 0 || *((const volatile int*)&s->error) != 0;
 }
 
-__device__ __forceinline__ bool is_zero(double v) {  // v == 0.0 without the FP64 pipe
-  return ((unsigned long long)__double_as_longlong(v) << 1) == 0ull;
-}
-
 // ---- grid-wide sums
 // Shared memory of a solver block: the reductions' work space, the last reduction's results (up
 // to four values derived from the sums and a flag, the same in every block) and the iteration's

@@ -20,36 +20,245 @@ namespace vebi {
 
 #define ELL(k, i) ((size_t)(k) * c.npfb + (i))
 
-// ---------------------------------------------------------------------- kernel_calculation
-__global__ void k_weights(Consts c, Dev d) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.npfb) return;
-  const double xi = d.rx[i], yi = d.ry[i], dv = c.dv;
-  double k11 = 0.0, k12 = 0.0, k21 = 0.0, k22 = 0.0;
-  const int cnt = d.ij_count[i];
-  for (int k = 0; k < cnt; ++k) {
-    int j = d.ij_link[ELL(k, i)];
-    double r1 = xi - d.rx[j], r2 = yi - d.ry[j];
-    double rr2 = r1 * r1 + r2 * r2;
-    double rad = sqrt(rr2);
-    double qq = rad * c.oneoverh;
-    double f = fac(c, qq);
-    double m = fmax(rad, c.eta2);
-    double g1 = r1 * f / m, g2 = r2 * f / m;
-    double w1 = g1 * dv, w2 = g2 * dv;
-    d.wGx[ELL(k, i)] = w1;
-    d.wGy[ELL(k, i)] = w2;
-    d.wL[ELL(k, i)] = 2.0 * (r1 * w1 + r2 * w2) / (rr2 + c.eta_small);
-    k11 = k11 - dv * g1 * r1;
-    k12 = k12 - dv * g2 * r1;
-    k21 = k21 - dv * g1 * r2;
-    k22 = k22 - dv * g2 * r2;
+// ------------------------------------------------- kernel_calculation and new_fick_shift's sums
+// The weights of a pair and the factor 0.25 (Wab(r/h) / Wab1)^4 of its shifting force
+// (kernel_calculation.F90:22-71, new_fick_shift.F90:135-148, where the reference calls pow with
+// the exponent 4.0), each operation as the reference writes it and rounds it.  Its products, quotients
+// and root run beside the FP64 pipe (vebi_fp64.cuh): 25 FP64 instructions are left of 170.
+struct PairTerms {
+  double w1, w2, wl, fab;
+};
+__device__ __forceinline__ double power4(double x) {
+  const double x2 = fp::mul_int(x, x);
+  return fp::mul_int(x2, x2);
+}
+__device__ __forceinline__ double power5(double x) {
+  const double x2 = fp::mul_int(x, x);
+  return fp::mul_int(x2, fp::mul_int(x, x2));
+}
+// the spline's classes, compared as integers (qq >= 0)
+__device__ __forceinline__ bool below(double qq, int k) { return fp::hi(qq) < fp::hi((double)k); }
+
+__device__ __forceinline__ PairTerms pair_terms(const Consts& c, double r1, double r2) {
+  using namespace fp;
+  PairTerms o;
+  const double rr2 = mul_int(r1, r1) + mul_int(r2, r2);
+  double y;
+  const double rad = root(rr2, y);
+  const double qq = mul_int(rad, c.oneoverh);
+  double f = 0.0;
+  if (below(qq, 3)) {  // fac (sphtools.F90:11-44)
+    f = mul_int(-5.0, power4(3.0 - qq));
+    if (below(qq, 2)) f = f + mul_int(30.0, power4(2.0 - qq));
+    if (below(qq, 1)) f = f - mul_int(75.0, power4(1.0 - qq));
+    f = mul_int(c.ad_7h, f);
   }
+  double m = rad;
+  if (!(__double_as_longlong(rad) > __double_as_longlong(c.eta2))) {  // particles (almost) on one another
+    m = fmax(rad, c.eta2);
+    y = divided(1.0, m);
+  }
+  const double a1 = mul_int(r1, f), a2 = mul_int(r2, f);
+  // aligned particles: 0 / m is the zero itself
+  const double g1 = is_zero(a1) ? a1 : quotient_near(a1, m, y, a1 * y);
+  const double g2 = is_zero(a2) ? a2 : quotient_near(a2, m, y, a2 * y);
+  o.w1 = mul_int(g1, c.dv);
+  o.w2 = mul_int(g2, c.dv);
+  const double den = rr2 + c.eta_small;
+  const double num = mul_int(2.0, mul_int(r1, o.w1) + mul_int(r2, o.w2));
+  const double yd = reciprocal(den);
+  o.wl = quotient_near(num, den, yd, num * yd);
+  const double q2 = quotient_near(rad, c.h, c.oneoverh, qq);  // rad / h
+  double w = 0.0;
+  if (below(q2, 3)) {  // Wab (sphtools.F90:46-76)
+    w = power5(3.0 - q2);
+    if (below(q2, 2)) w = w - mul_int(6.0, power5(2.0 - q2));
+    if (below(q2, 1)) w = w + mul_int(15.0, power5(1.0 - q2));
+    w = mul_int(c.ad_7, w);
+  }
+  const double wn = is_zero(w) ? w : quotient_near(w, c.wab1, c.inv_wab1, mul_int(w, c.inv_wab1));
+  o.fab = mul_int(0.25, power4(wn));
+  return o;
+}
+
+// the slot of particle i in row j, or -1
+__device__ __forceinline__ int slot_of(const Consts& c, const Dev& d, int j, int i) {
+  const int cnt = d.ij_count[j];
+  for (int k0 = 0; k0 < cnt; k0 += 8) {
+    int l[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) l[u] = k0 + u < cnt ? d.ij_link[ELL(k0 + u, j)] : -1;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (l[u] == i) return k0 + u;
+  }
+  return -1;
+}
+
+// -x, a zero as it is (a pair's x - x is +0 from both sides); on the integer pipe
+__device__ __forceinline__ double negated(double x) {
+  int h;
+  asm("xor.b32 %0, %1, 0x80000000;" : "=r"(h) : "r"(fp::hi(x)));
+  return is_zero(x) ? x : fp::pack(h, fp::lo(x));
+}
+
+// The pairs' terms.  A pair's terms serve both its particles -- r_ij and w_ij change sign, wL and
+// the shifting factor do not, bit for bit -- so each pair is computed once, by the particle of
+// lower index (or the one that has a mirror for a neighbour), and stored in both rows; the search
+// of the partner's row for the slot waits in the shadow of the arithmetic.  A pair that one
+// particle alone lists (d.s->one_sided) is computed by that one.  Each lane first lists the slots
+// it computes, so that all lanes of a warp compute in every round.  P lanes share a row when the
+// // rows alone would not fill the GPU.
+// What bounds it: the issue of ~1000 integer and FP32 instructions a pair, with the FP64 pipe at 40%.
+// Measured with k_weight_sums at 4M / 250k / 20k / 1.7k particles: 12.6 / 1.08 / 0.15 / 0.08 ms, where
+// a kernel each for the weights and the shifting, all pairs from both sides in FP64 instructions,
+// took 43.9 / 3.21 / 0.64 / 0.58.
+constexpr int PAIR_SLOTS = 96;  // nplink's limit
+constexpr int PAIR_TPB = 64;    // small blocks: a 20k-particle step has few of them per SM to balance
+
+template <int P>
+__global__ void __launch_bounds__(PAIR_TPB) k_pair_terms(Consts c, Dev d, double* __restrict__ fab) {
+  __shared__ unsigned char list[PAIR_SLOTS / P][PAIR_TPB];
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = tid / P;
+  if (i >= c.npfb) return;
+  const int cnt = d.ij_count[i];
+  const bool one_sided = d.s->one_sided != 0;
+  int m = 0;
+#pragma unroll 4
+  for (int k = tid % P; k < cnt; k += P) {
+    const int j = d.ij_link[ELL(k, i)];
+    if (j > i || (one_sided && slot_of(c, d, j, i) < 0)) list[m++][threadIdx.x] = (unsigned char)k;
+  }
+  const double xi = d.rx[i], yi = d.ry[i];
+#pragma unroll 1
+  for (int e = 0; e < m; ++e) {
+    const size_t o = ELL(list[e][threadIdx.x], i);
+    const int j = d.ij_link[o];
+    const int kj = j < c.npfb ? slot_of(c, d, j, i) : -1;
+    const PairTerms t = pair_terms(c, xi - d.rx[j], yi - d.ry[j]);
+    d.wGx[o] = t.w1;
+    d.wGy[o] = t.w2;
+    d.wL[o] = t.wl;
+    fab[o] = t.fab;
+    if (kj >= 0) {
+      const size_t q = ELL(kj, j);
+      d.wGx[q] = negated(t.w1);
+      d.wGy[q] = negated(t.w2);
+      d.wL[q] = t.wl;
+      fab[q] = t.fab;
+    }
+  }
+}
+
+// Shifting displacement from the concentration gradient (new_fick_shift.F90:47-92) and the shifting
+// velocity; solid boundary particles get -u (div_free.F90:65-78).  The uncommon cases are calls:
+// inlined, the compiler computes their divisions, roots and exponential for every particle.
+static __device__ __noinline__ double speed_coefficient(const Consts& c, const Dev& d, int i, double dt) {
+  double maxU = bits_to_double(d.s->maxU_bits);
+  double absU = sqrt(d.ux[i] * d.ux[i] + d.uy[i] * d.uy[i]);
+  double temp = (double)0.2f * exp(-absU / ((double)0.2f * maxU));
+  return 4.0 * c.h * dt * (absU + temp * maxU);
+}
+static __device__ __noinline__ double2 along_surface(const Dev& d, int i, double D, double gx, double gy) {
+  double temp = sqrt(d.surf_nx[i] * d.surf_nx[i] + d.surf_ny[i] * d.surf_ny[i]);
+  double sn1 = d.surf_nx[i] / fmax(temp, (double)1e-8f);
+  double sn2 = d.surf_ny[i] / fmax(temp, (double)1e-8f);
+  double st1 = -sn2, st2 = sn1;
+  double dCds = st1 * gx + st2 * gy;
+  return make_double2(-D * dCds * st1, -D * dCds * st2);
+}
+__device__ __forceinline__ void shift_velocity(const Consts& c, const Dev& d, int i, double gx, double gy) {
+  if (i < c.nbS) {
+    d.ushx[i] = -d.ux[i];
+    d.ushy[i] = -d.uy[i];
+    return;
+  }
+  const double dt = d.s->dt;
+  const double D = c.shift_coeff == 1 ? speed_coefficient(c, d, i, dt) : 0.25 * c.h * c.h;
+  double2 s;
+  if (c.open_domain == 1 && d.n_surf[i] == 1) s = along_surface(d, i, D, gx, gy);
+  else s = make_double2(-D * gx, -D * gy);
+  const double s2 = s.x * s.x + s.y * s.y;
+  double y;
+  const double temp = is_zero(s2) ? s2 : fp::root(s2, y);
+  if (temp > 0.1 * c.h) {
+    s.x = fp::divided(0.1 * c.h * s.x, temp);
+    s.y = fp::divided(0.1 * c.h * s.y, temp);
+  }
+  y = fp::reciprocal(dt);
+  d.ushx[i] = is_zero(s.x) ? s.x : fp::quotient_near(s.x, dt, y, s.x * y);
+  d.ushy[i] = is_zero(s.y) ? s.y : fp::quotient_near(s.y, dt, y, s.y * y);
+}
+
+// The sums over each row in slot order: the Bonet-Lok matrix and the concentration gradient of the
+// shifting; in a closed domain the shifting velocity too.  What bounds it is the FP64 pipe, ten
+// instructions a pair (16 with its products, 5.8 ms at 4M; 3.7 without).  P = 4 splits a row's eight
+// sums over four lanes, two each.
+template <int P>
+__global__ void __launch_bounds__(TPB) k_weight_sums(const __grid_constant__ Consts c, const __grid_constant__ Dev d,
+                                                     const double* __restrict__ fab) {
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = tid / P, p = tid % P;
+  const bool in = i < c.npfb;
+  const int cnt = in ? d.ij_count[i] : 0;
+  double k11 = 0.0, k12 = 0.0, k21 = 0.0, k22 = 0.0, f1 = 0.0, f2 = 0.0, t1 = 0.0, t2 = 0.0;
+  if (P == 1) {
+    const double xi = in ? d.rx[i] : 0.0, yi = in ? d.ry[i] : 0.0;
+#pragma unroll 2
+    for (int k = 0; k < cnt; ++k) {
+      const size_t o = ELL(k, i);
+      const int j = d.ij_link[o];
+      const double w1 = d.wGx[o], w2 = d.wGy[o], fb = fab[o];
+      const double r1 = xi - d.rx[j], r2 = yi - d.ry[j];
+      k11 = k11 - fp::mul_int(w1, r1);  // dv * g1 * r1
+      k12 = k12 - fp::mul_int(w2, r1);
+      k21 = k21 - fp::mul_int(w1, r2);
+      k22 = k22 - fp::mul_int(w2, r2);
+      f1 = f1 + w1;
+      f2 = f2 + w2;
+      t1 = t1 + fp::mul_int(w1, fb);
+      t2 = t2 + fp::mul_int(w2, fb);
+    }
+  } else {
+    // lane 0: k11, f1; 1: k12, f2; 2: k21, t1; 3: k22, t2
+    const double* wp = (p & 1) ? d.wGy : d.wGx;
+    const double* xp = p < 2 ? d.rx : d.ry;
+    const double x0 = in ? xp[i] : 0.0;
+    double ks = 0.0, fs = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < cnt; ++k) {
+      const size_t o = ELL(k, i);
+      const double w = wp[o], r = x0 - xp[d.ij_link[o]];
+      ks = ks - w * r;
+      fs = fs + w * (p < 2 ? 1.0 : fab[o]);
+    }
+    const unsigned full = 0xffffffffu;
+    k11 = ks;
+    k12 = __shfl_down_sync(full, ks, 1);
+    k21 = __shfl_down_sync(full, ks, 2);
+    k22 = __shfl_down_sync(full, ks, 3);
+    f1 = fs;
+    f2 = __shfl_down_sync(full, fs, 1);
+    t1 = __shfl_down_sync(full, fs, 2);
+    t2 = __shfl_down_sync(full, fs, 3);
+  }
+  if (!in || p) return;
   double temp = 1.0 / ((k11 * k22 - k12 * k21) + 1.0e-15);
   d.kgcm[0][i] = temp * k22;
   d.kgcm[2][i] = -temp * k12;
   d.kgcm[1][i] = -temp * k21;
   d.kgcm[3][i] = temp * k11;
+  const double gx = f1 + t1, gy = f2 + t2;
+  d.gradCx[i] = gx;
+  d.gradCy[i] = gy;
+  if (c.open_domain == 0) shift_velocity(c, d, i, gx, gy);
+}
+
+// open domain: after the free-surface particles and their normals are known
+__global__ void k_shift_open(const __grid_constant__ Consts c, const __grid_constant__ Dev d) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < c.npfb) shift_velocity(c, d, i, d.gradCx[i], d.gradCy[i]);
 }
 
 // ---------------------------------------------------------------------- free surface (open)
@@ -89,8 +298,8 @@ __global__ void k_nsurf_mirrors(Consts c, Dev d) {
   }
 }
 
-// smooth_normals (Shepard filter) + ppe_smooth; the filtered normals go to gradCx/gradCy
-// scratch first and are copied back after (the reference uses a temporary array too)
+// smooth_normals (Shepard filter) + ppe_smooth; the filtered normals go to the shifting velocity's
+// arrays first and are copied back after (the reference uses a temporary array too)
 __global__ void k_smooth_normals(Consts c, Dev d) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c.npfb) return;
@@ -107,8 +316,8 @@ __global__ void k_smooth_normals(Consts c, Dev d) {
     b = b + w * d.surf_ny[j];
   }
   double w0 = wab(c, 0.0);
-  d.gradCx[i] = a * c.dv + d.surf_nx[i] * w0 * c.dv;
-  d.gradCy[i] = b * c.dv + d.surf_ny[i] * w0 * c.dv;
+  d.ushx[i] = a * c.dv + d.surf_nx[i] * w0 * c.dv;
+  d.ushy[i] = b * c.dv + d.surf_ny[i] * w0 * c.dv;
   double ps = 1.0;
   double dr = d.div_r[i], bdr = d.beta_div_r[i];
   if (!(dr > 1.2 * bdr)) {
@@ -121,71 +330,8 @@ __global__ void k_smooth_normals(Consts c, Dev d) {
 __global__ void k_copy_normals(Consts c, Dev d) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c.npfb) return;
-  d.surf_nx[i] = d.gradCx[i];
-  d.surf_ny[i] = d.gradCy[i];
-}
-
-// ---------------------------------------------------------------------- shifting
-__global__ void k_shift(Consts c, Dev d) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.npfb) return;
-  const double xi = d.rx[i], yi = d.ry[i];
-  double f1 = 0, f2 = 0, t1 = 0, t2 = 0;
-  const int cnt = d.ij_count[i];
-  for (int k = 0; k < cnt; ++k) {
-    int j = d.ij_link[ELL(k, i)];
-    double r1 = xi - d.rx[j], r2 = yi - d.ry[j];
-    double rad = sqrt(r1 * r1 + r2 * r2);
-    double qq = rad / c.h;
-    // Rt*(Wab/Wab1)**nt with nt = 4.0 (new_fick_shift.F90:135-148); the reference calls pow
-    double fab = 0.25 * pw4(wab(c, qq) / c.wab1);
-    double w1 = d.wGx[ELL(k, i)], w2 = d.wGy[ELL(k, i)];
-    f1 = f1 + w1;
-    f2 = f2 + w2;
-    t1 = t1 + w1 * fab;
-    t2 = t2 + w2 * fab;
-  }
-  double gx = f1 + t1, gy = f2 + t2;
-  d.gradCx[i] = gx;
-  d.gradCy[i] = gy;
-  const double dt = d.s->dt;
-  double d1 = 0.0, d2 = 0.0;
-  if (i >= c.nbS) {
-    double D;
-    if (c.shift_coeff == 1) {
-      double maxU = bits_to_double(d.s->maxU_bits);
-      double absU = sqrt(d.ux[i] * d.ux[i] + d.uy[i] * d.uy[i]);
-      double temp = (double)0.2f * exp(-absU / ((double)0.2f * maxU));
-      D = 4.0 * c.h * dt * (absU + temp * maxU);
-    } else {
-      D = 0.25 * c.h * c.h;
-    }
-    if (d.n_surf[i] == 1 && c.open_domain == 1) {
-      double temp = sqrt(d.surf_nx[i] * d.surf_nx[i] + d.surf_ny[i] * d.surf_ny[i]);
-      double sn1 = d.surf_nx[i] / fmax(temp, (double)1e-8f);
-      double sn2 = d.surf_ny[i] / fmax(temp, (double)1e-8f);
-      double st1 = -sn2, st2 = sn1;
-      double dCds = st1 * gx + st2 * gy;
-      d1 = -D * dCds * st1;
-      d2 = -D * dCds * st2;
-    } else {
-      d1 = -D * gx;
-      d2 = -D * gy;
-    }
-    double temp = sqrt(d1 * d1 + d2 * d2);
-    if (temp > 0.1 * c.h) {
-      d1 = 0.1 * c.h * d1 / temp;
-      d2 = 0.1 * c.h * d2 / temp;
-    }
-  }
-  // ushift = dr_fs/dt; solid boundary particles get -u (div_free.F90:65-78)
-  if (i < c.nbS) {
-    d.ushx[i] = -d.ux[i];
-    d.ushy[i] = -d.uy[i];
-  } else {
-    d.ushx[i] = d1 / dt;
-    d.ushy[i] = d2 / dt;
-  }
+  d.surf_nx[i] = d.ushx[i];
+  d.surf_ny[i] = d.ushy[i];
 }
 
 // ---------------------------------------------------------------------- gradients
@@ -557,13 +703,27 @@ void launch_gradients32(Ctx& x);
 void launch_predictor32(Ctx& x);
 void launch_pgrad_final32(Ctx& x);
 
+static void launch_weights(Ctx& x) {
+  const Consts& c = x.c;
+  double* fab = x.d.ppe_val;  // free until the PPE is assembled
+  const long long n = c.npfb;
+  // Lanes per row, measured with 8 / 4 / 1: 20k particles 0.15 / 0.17 / 0.44 ms, 60k 0.37 / 0.35 /
+  // 0.52, 100k 0.58 / 0.53 / 0.60, 250k 1.19 / 1.23 / 1.08.
+  if (n <= 40000) VEBI_LAUNCH(x, k_pair_terms<8>, grid_for(n * 8, PAIR_TPB), PAIR_TPB, c, x.d, fab);
+  else if (n <= 150000) VEBI_LAUNCH(x, k_pair_terms<4>, grid_for(n * 4, PAIR_TPB), PAIR_TPB, c, x.d, fab);
+  else VEBI_LAUNCH(x, k_pair_terms<1>, grid_for(n, PAIR_TPB), PAIR_TPB, c, x.d, fab);
+  if (n <= 150000) VEBI_LAUNCH(x, k_weight_sums<4>, grid_for(n * 4, PAIR_TPB), PAIR_TPB, c, x.d, fab);
+  else VEBI_LAUNCH(x, k_weight_sums<1>, grid_for(n), TPB, c, x.d, fab);
+}
+
 void launch_weights_surface_shift(Ctx& x) {
   const Consts& c = x.c;
   int g = grid_for(c.npfb);
   const bool mixed = x.precision == VEBI_PREC_MIXED;
   if (mixed) launch_prep_weights32(x);
-  // FP64 weights: the FP64 step, and the free-surface operators of an open domain
-  if (!mixed || c.open_domain == 1) VEBI_LAUNCH(x, k_weights, g, TPB, c, x.d);
+  // FP64 weights: the FP64 step, and the free-surface operators and shifting of an open domain
+  const bool f64 = !mixed || c.open_domain == 1;
+  if (f64) launch_weights(x);
   if (c.open_domain == 1) {
     VEBI_LAUNCH(x, k_part_dist_vars, g, TPB, c, x.d);
     VEBI_LAUNCH(x, k_nsurf_mirrors, x.gs_blocks, TPB, c, x.d);
@@ -573,8 +733,8 @@ void launch_weights_surface_shift(Ctx& x) {
     cudaMemsetAsync(x.d.n_surf, 0, sizeof(int) * (size_t)c.cap, x.st);
   }
   stage_mark(x, 5);
-  if (mixed && c.open_domain == 0) launch_shift32(x);
-  else VEBI_LAUNCH(x, k_shift, g, TPB, c, x.d);
+  if (!f64) launch_shift32(x);
+  else if (c.open_domain == 1) VEBI_LAUNCH(x, k_shift_open, g, TPB, c, x.d);
 }
 
 void launch_grad_mirrors(Ctx& x);
