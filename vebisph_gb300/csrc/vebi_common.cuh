@@ -57,6 +57,7 @@ struct Consts {
 // Scalars that change during a step; they live in device memory so no step needs a host sync.
 struct Scal {
   double dt;
+  double relax;                      // exp(-dt / Wi): the relaxation factor of an Oldroyd-B step
   unsigned long long umax_bits;      // max |u| over fluid (set_time_step), as ordered bits
   unsigned long long maxU_bits;      // max |u| over 1..npfb after binning (new_fick_shift)
   unsigned long long absu_bits, absv_bits, absp_bits;  // TIME-file maxima

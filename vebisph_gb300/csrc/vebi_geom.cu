@@ -631,7 +631,10 @@ __global__ void k_solid_fixup(Consts c, Dev d) {
   }
 }
 
-__global__ void k_set_np(Consts c, Scal* s) { s->np = c.npfb + s->nmirror; }
+__global__ void k_set_np(Consts c, Scal* s) {
+  s->np = c.npfb + s->nmirror;
+  s->relax = exp(-(1.0 * 1.0 * s->dt / c.Wi));  // as k_logconf's with alpha_R = 1; dt may be a replayed step's
+}
 
 static void run_stage(Ctx& x, int kind, int ib, int n0, int n1_static, int n_items_bound) {
   // stages over particles (their items end at npfb) walk the candidate list instead

@@ -27,6 +27,7 @@ namespace vebi {
 
 // ---------------------------------------------------------------------- right-hand side
 __global__ void k_ppe_rhs(Consts c, Dev d) {
+  using fp::mul_int;  // the products beside the FP64 pipe, as in k_gradients
   __shared__ double sh[TPB / 32 + 1];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double b = 0.0;
@@ -39,8 +40,8 @@ __global__ void k_ppe_rhs(Consts c, Dev d) {
       int j = d.ij_link[ELL(k, i)];
       double u1 = ui - d.ux2[j], u2 = vi - d.uy2[j];
       double w1 = d.wGx[ELL(k, i)], w2 = d.wGy[ELL(k, i)];
-      double kw1 = K11 * w1 + K12 * w2, kw2 = K21 * w1 + K22 * w2;
-      fb = fb - (u1 * kw1 + u2 * kw2);
+      double kw1 = mul_int(K11, w1) + mul_int(K12, w2), kw2 = mul_int(K21, w1) + mul_int(K22, w2);
+      fb = fb - (mul_int(u1, kw1) + mul_int(u2, kw2));
     }
     b = fb / d.s->dt;
     d.ppe_B[i] = b;

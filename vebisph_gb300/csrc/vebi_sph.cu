@@ -196,7 +196,7 @@ __device__ __forceinline__ void shift_velocity(const Consts& c, const Dev& d, in
 // instructions a pair (16 with its products, 5.8 ms at 4M; 3.7 without).  P = 4 splits a row's eight
 // sums over four lanes, two each.
 template <int P>
-__global__ void __launch_bounds__(TPB) k_weight_sums(const __grid_constant__ Consts c, const __grid_constant__ Dev d,
+__global__ void __launch_bounds__(TPB, 4) k_weight_sums(const __grid_constant__ Consts c, const __grid_constant__ Dev d,
                                                      const double* __restrict__ fab) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = tid / P, p = tid % P;
@@ -335,7 +335,12 @@ __global__ void k_copy_normals(Consts c, Dev d) {
 }
 
 // ---------------------------------------------------------------------- gradients
-__global__ void k_gradients(Consts c, Dev d) {
+// The products of a pair run on the integer pipe (vebi_fp64.cuh), beside the FP64 pipe that bounds
+// these kernels on large domains; on small ones they cost nothing either.  4M particles, without /
+// with: gradients 5.28 / 3.24 ms, predictor 10.97 / 5.81 ms (7.31 with two blocks per SM: 82
+// registers leave too few warps to cover the gathers), right-hand side 3.9 / 1.9 ms.
+__global__ void __launch_bounds__(TPB, 4) k_gradients(Consts c, Dev d) {
+  using fp::mul_int;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c.npfb) return;
   const double ui = d.ux[i], vi = d.uy[i], ti = d.th[i];
@@ -345,12 +350,12 @@ __global__ void k_gradients(Consts c, Dev d) {
     int j = d.ij_link[ELL(k, i)];
     double w1 = d.wGx[ELL(k, i)], w2 = d.wGy[ELL(k, i)];
     double du = d.ux[j] - ui, dvv = d.uy[j] - vi, dth = d.th[j] - ti;
-    a0 = a0 + du * w1;
-    a1 = a1 + du * w2;
-    a2 = a2 + dvv * w1;
-    a3 = a3 + dvv * w2;
-    a4 = a4 + dth * w1;
-    a5 = a5 + dth * w2;
+    a0 = a0 + mul_int(du, w1);
+    a1 = a1 + mul_int(du, w2);
+    a2 = a2 + mul_int(dvv, w1);
+    a3 = a3 + mul_int(dvv, w2);
+    a4 = a4 + mul_int(dth, w1);
+    a5 = a5 + mul_int(dth, w2);
   }
   const double K11 = d.kgcm[0][i], K21 = d.kgcm[1][i], K12 = d.kgcm[2][i], K22 = d.kgcm[3][i];
   d.grad[0][i] = K11 * a0 + K12 * a1;
@@ -362,26 +367,36 @@ __global__ void k_gradients(Consts c, Dev d) {
 }
 
 // ---------------------------------------------------------------------- log-conformation
+// What bounds it: the FP64 pipe, ~190 instructions a particle, of which two logarithms and two
+// exponentials are 98.  Its ~110 products, five quotients and four roots run beside the pipe
+// (vebi_fp64.cuh; all on it, it was 398 instructions and 2.98 ms at 4M, 1.59 now).
 struct M2 { double a11, a12, a21, a22; };
-__device__ __forceinline__ M2 mm(const M2& A, const M2& B) {
-  return M2{A.a11 * B.a11 + A.a12 * B.a21, A.a11 * B.a12 + A.a12 * B.a22,
-            A.a21 * B.a11 + A.a22 * B.a21, A.a21 * B.a12 + A.a22 * B.a22};
+// a call: twelve products inlined are 140 KB of code, more than the instruction cache
+static __device__ __noinline__ M2 mm(M2 A, M2 B) {
+  using fp::mul_int;
+  return M2{mul_int(A.a11, B.a11) + mul_int(A.a12, B.a21), mul_int(A.a11, B.a12) + mul_int(A.a12, B.a22),
+            mul_int(A.a21, B.a11) + mul_int(A.a22, B.a21), mul_int(A.a21, B.a12) + mul_int(A.a22, B.a22)};
 }
 __device__ __forceinline__ M2 tr(const M2& A) { return M2{A.a11, A.a21, A.a12, A.a22}; }
 
 // calc_eigens (predictor_mod.F90:253-290): closed-form symmetric 2x2 eigen-decomposition
 __device__ __forceinline__ void calc_eigens(const M2& A, double& L1, double& L2, M2& R) {
+  using namespace fp;
   double trc = A.a11 + A.a22;
-  double det = A.a11 * A.a22 - A.a21 * A.a12;
-  double tmp = 0.25 * trc * trc - det;
-  if (tmp <= 2.220446049250313e-16) tmp = 0.0;  // epsilon(1d0)
-  L1 = 0.5 * trc + sqrt(tmp);
-  L2 = 0.5 * trc - sqrt(tmp);
-  if (A.a21 != 0.0) {
+  double det = mul_int(A.a11, A.a22) - mul_int(A.a21, A.a12);
+  double tmp = mul_int(mul_int(0.25, trc), trc) - det;
+  // tmp <= epsilon(1d0), compared as integers (a NaN stays)
+  const long long bits = __double_as_longlong(tmp);
+  if (bits <= 0x3cb0000000000000ll && (bits & 0x7fffffffffffffffll) <= 0x7ff0000000000000ll) tmp = 0.0;
+  double y;
+  const double rt = is_zero(tmp) ? 0.0 : root(tmp, y), half = mul_int(0.5, trc);
+  L1 = half + rt;
+  L2 = half - rt;
+  if (!is_zero(A.a21)) {
     double r11 = L1 - A.a22, r21 = A.a21;
-    double nrm = sqrt(r11 * r11 + r21 * r21);
-    r11 = r11 / nrm;
-    r21 = r21 / nrm;
+    double nrm = root(mul_int(r11, r11) + mul_int(r21, r21), y);
+    r11 = quotient(r11, nrm, y);
+    r21 = quotient(r21, nrm, y);
     R = M2{r11, -r21, r21, r11};
   } else {
     L1 = A.a11;
@@ -389,8 +404,13 @@ __device__ __forceinline__ void calc_eigens(const M2& A, double& L1, double& L2,
     R = M2{1.0, 0.0, 0.0, 1.0};
   }
 }
+// the relaxation factor exp(-(alpha_R dt / Wi)); alpha_R = 1 is the step's own (k_set_np)
+static __device__ __noinline__ double relaxation(double alpha_R, double dt, double Wi) {
+  return exp(-(alpha_R * 1.0 * dt / Wi));
+}
 
 __global__ void k_logconf(Consts c, Dev d) {
+  using fp::mul_int;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c.npfb) return;
   const double dt = d.s->dt;
@@ -400,9 +420,10 @@ __global__ void k_logconf(Consts c, Dev d) {
   double L1, L2;
   M2 R;
   calc_eigens(A, L1, L2, R);
+  const double gap = L2 - L1;
   {  // diagnostic: particles within reach of the 1/(L2 - L1 + 1e-10) pole of step 5
     const unsigned am = __activemask();
-    const unsigned near = __ballot_sync(am, fabs(L2 - L1) < 1.0e-7);
+    const unsigned near = __ballot_sync(am, __double_as_longlong(fp::magnitude(gap)) < __double_as_longlong(1.0e-7));
     if ((threadIdx.x & 31) == __ffs(am) - 1 && near) {
       atomicAdd(&d.s->n_near_pole, __popc(near));
       atomicAdd(&d.s->n_near_pole_total, __popc(near));
@@ -414,7 +435,8 @@ __global__ void k_logconf(Consts c, Dev d) {
   // step 5: B and Omega from R^T grad(u) R
   M2 G{d.grad[0][i], d.grad[1][i], d.grad[2][i], d.grad[3][i]};
   M2 tm = mm(tr(R), mm(G, R));
-  double tmp1 = (L2 * tm.a12 + L1 * tm.a21) / (L2 - L1 + 1e-10);
+  const double den = gap + 1e-10;
+  double tmp1 = fp::quotient(mul_int(L2, tm.a12) + mul_int(L1, tm.a21), den, fp::reciprocal(fp::magnitude(den)));
   tm.a12 = 0.0;
   tm.a21 = 0.0;
   M2 B = mm(R, mm(tm, tr(R)));
@@ -422,9 +444,10 @@ __global__ void k_logconf(Consts c, Dev d) {
   M2 Om = mm(R, mm(W, tr(R)));
   // step 6: Psi += dt (2B + Omega Psi - Psi Omega)
   M2 OP = mm(Om, Psi0), PO = mm(Psi0, Om);
-  M2 t6{2.0 * B.a11 + OP.a11 - PO.a11, 2.0 * B.a12 + OP.a12 - PO.a12, 2.0 * B.a21 + OP.a21 - PO.a21,
-        2.0 * B.a22 + OP.a22 - PO.a22};
-  M2 Psi{Psi0.a11 + dt * t6.a11, Psi0.a12 + dt * t6.a12, Psi0.a21 + dt * t6.a21, Psi0.a22 + dt * t6.a22};
+  M2 t6{mul_int(2.0, B.a11) + OP.a11 - PO.a11, mul_int(2.0, B.a12) + OP.a12 - PO.a12,
+        mul_int(2.0, B.a21) + OP.a21 - PO.a21, mul_int(2.0, B.a22) + OP.a22 - PO.a22};
+  M2 Psi{Psi0.a11 + mul_int(dt, t6.a11), Psi0.a12 + mul_int(dt, t6.a12), Psi0.a21 + mul_int(dt, t6.a21),
+         Psi0.a22 + mul_int(dt, t6.a22)};
   // step 7: A = R exp(Lambda) R^T
   calc_eigens(Psi, L1, L2, R);
   L1 = exp(L1);
@@ -432,10 +455,11 @@ __global__ void k_logconf(Consts c, Dev d) {
   M2 E2{L1, 0.0, 0.0, L2};
   A = mm(R, mm(E2, tr(R)));
   // step 8: analytic PTT relaxation with the previous trace
-  double alpha_R = 1.0 + c.eps_ptt * (d.trace_conf[i] - 2.0);
-  double e1 = exp(-(alpha_R * 1.0 * dt / c.Wi));
+  double alpha_R = 1.0 + mul_int(c.eps_ptt, d.trace_conf[i] - 2.0);
+  double e1 = __double_as_longlong(alpha_R) == __double_as_longlong(1.0) ? d.s->relax : relaxation(alpha_R, dt, c.Wi);
   double e2 = (1.0 - e1) / 1.0;
-  A = M2{A.a11 * e1 + e2 * 1.0, A.a12 * e1 + e2 * 0.0, A.a21 * e1 + e2 * 0.0, A.a22 * e1 + e2 * 1.0};
+  const double z = mul_int(e2, 0.0);
+  A = M2{mul_int(A.a11, e1) + e2 * 1.0, mul_int(A.a12, e1) + z, mul_int(A.a21, e1) + z, mul_int(A.a22, e1) + e2 * 1.0};
   // step 9
   double trc = A.a11 + A.a22;
   d.trace_conf[i] = trc;
@@ -448,7 +472,8 @@ __global__ void k_logconf(Consts c, Dev d) {
 
 // ---------------------------------------------------------------------- predictor
 // rhs pair loop + buoyancy; u*, theta* written to the second buffers (walls copied)
-__global__ void k_predictor(Consts c, Dev d) {
+__global__ void __launch_bounds__(TPB, 4) k_predictor(Consts c, Dev d) {
+  using fp::mul_int;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c.npfb) return;
   const double ui = d.ux[i], vi = d.uy[i], ti = d.th[i];
@@ -467,16 +492,16 @@ __global__ void k_predictor(Consts c, Dev d) {
       double w1 = d.wGx[ELL(k, i)], w2 = d.wGy[ELL(k, i)];
       double T11 = d.tau[0][j] - Ti11, T21 = d.tau[1][j] - Ti21;
       double T12 = d.tau[2][j] - Ti12, T22 = d.tau[3][j] - Ti22;
-      double kw1 = K11 * w1 + K12 * w2, kw2 = K21 * w1 + K22 * w2;
-      double tw1 = T11 * kw1 + T12 * kw2, tw2 = T21 * kw1 + T22 * kw2;
-      s1 = s1 + cp * tw1 + cs * u1 * wl;
-      s2 = s2 + cp * tw2 + cs * u2 * wl;
+      double kw1 = mul_int(K11, w1) + mul_int(K12, w2), kw2 = mul_int(K21, w1) + mul_int(K22, w2);
+      double tw1 = mul_int(T11, kw1) + mul_int(T12, kw2), tw2 = mul_int(T21, kw1) + mul_int(T22, kw2);
+      s1 = s1 + mul_int(cp, tw1) + mul_int(mul_int(cs, u1), wl);
+      s2 = s2 + mul_int(cp, tw2) + mul_int(mul_int(cs, u2), wl);
     } else {
-      s1 = s1 + cs * u1 * wl;
-      s2 = s2 + cs * u2 * wl;
+      s1 = s1 + mul_int(mul_int(cs, u1), wl);
+      s2 = s2 + mul_int(mul_int(cs, u2), wl);
     }
     double thij = ti - d.th[j];
-    st = st + ct * thij * wl;
+    st = st + mul_int(mul_int(ct, thij), wl);
   }
   s2 = s2 + ti;  // buoyancy (predictor_mod.F90:111-119)
   const double dt = d.s->dt;
