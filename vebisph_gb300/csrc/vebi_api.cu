@@ -229,9 +229,10 @@ static int allocate_all(Ctx& x) {
   A_(d.cellpart, cap); A_(d.cell_fill, cap); A_(d.ip, cap);
   A_(d.cell_cnt, (size_t)c.nct); A_(d.cell_start, (size_t)c.nct + 1);
   A_(d.scan_part, (size_t)c.nct / 1024 + 2);
-  size_t sel_items = (size_t)(c.npfb > c.mcap ? c.npfb : c.mcap);
-  A_(d.sel_blk, sel_items / SEL_CH + 2);
-  A_(d.cand, n); A_(d.cand_blk, n / SEL_CH + 2);
+  const size_t stages = (size_t)c.nb + 2;  // mirror stages: circles, patches, candidates
+  A_(d.sel_blk, stages * (n > 200000 ? n / 1024 + 1 : n / 256 + 1) + 1);
+  A_(d.sel_bits, (stages + c.ncirc) * ((n + 31) / 32)); A_(d.mir_list, 2 * MIR_LIST);
+  A_(d.cand, n);
   A_(d.pk, cap); A_(d.pko, cap);
   A_(d.ij_count, n); A_(d.ij_link, E);
   A_(d.wGx, E); A_(d.wGy, E); A_(d.wL, E);

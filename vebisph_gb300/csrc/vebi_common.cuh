@@ -73,10 +73,8 @@ struct Scal {
   int ls_iters;
   int warnings;
   int error;
-  int sel_base;                      // mirror offset of the current ordered-select stage
-  int n_cand;                        // particles in cand (candidates of the mirror stages)
-  int sel_total;
-  int imp_temp;                      // mirror count snapshot for wall-periodic corners
+  int n_cand;                        // particles in cand
+  int n_end, n_node;                 // mirrors and particles listed for the corners (mir_list)
   unsigned int bar_count;            // grid barrier of the PPE solvers (vebi_solver.cuh)
   int refine_iters;
   int ls_iters_total;                // summed over the steps of one vebi_run_steps call
@@ -91,6 +89,9 @@ struct Scal {
 // by one block, coarsest sweeps, Jacobi damping, coarse-correction scaling.  MG_BLOCK_ROWS is
 // measured: the 20k / 250k / 4M mixed solves take 1.99 / 4.11 / 26.7 ms at 512 (within 1% from
 // 256 to 1024) and 2.36 / 4.50 / 27.5 ms at 2048.
+// items of each of the corners' two lists
+constexpr int MIR_LIST = 4096;
+
 constexpr int MG_SLOTS = 24;
 constexpr int MG_ROW_SLOTS = 16;
 constexpr int MG_COARSEST = 32;
@@ -130,7 +131,9 @@ struct Dev {
   int *scan_part;
   // ordered select scratch
   int* sel_blk;
-  int *cand, *cand_blk;                      // particles near a boundary or circle, ascending
+  unsigned* sel_bits;                        // [plane][particle / 32]
+  int* mir_list;                             // corners: mirrors past a wall's end, particles by a node
+  int* cand;                                 // with circles: particles near a boundary or circle, ascending
   // pairs
   int *ij_count, *ij_link;
   double *wGx, *wGy, *wL;

@@ -36,7 +36,6 @@ struct Ctx {
   int mg_block_rows = MG_BLOCK_ROWS;  // batch tuning: coarse levels of at most this many rows run in one block
   int grid_gen = 0;                // bumped when a launch shape changes (captured graphs are stale)
   int gs_blocks = 0;         // grid of grid-stride kernels over dynamic counts
-  int sel_max_blocks = 0;    // blocks of the ordered-select kernels
   int precision = VEBI_PREC_FP64;
   bool have_state = false;
   // multigrid-preconditioned PPE (opt-in)
@@ -99,9 +98,5 @@ inline void stage_mark(Ctx& x, int s) {
   else cudaEventRecord(x.ev[s], x.st);
   x.ev_used[s] = true;
 }
-
-// ordered-select items per block
-constexpr int SEL_IPT = 8;
-constexpr int SEL_CH = TPB * SEL_IPT;
 
 }  // namespace vebi

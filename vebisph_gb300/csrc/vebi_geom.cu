@@ -11,8 +11,8 @@
 //
 // The reference builds mirrors serially with one global counter `imp`, patch after patch,
 // then corner after corner; wall-periodic corners scan the mirrors made so far.  Here every
-// such stage is an order-preserving stream compaction (count / scan / emit) over the
-// candidate particles, so mirror k here is mirror k of the reference.
+// stage is an order-preserving stream compaction (count / scan / emit), so mirror k here is mirror k
+// of the reference.
 #include "vebi_ctx.cuh"
 
 namespace vebi {
@@ -42,6 +42,7 @@ __global__ void k_step_reset(Scal* s, int npfb, int nbS) {
   s->bar_count = 0u;
   s->refine_iters = 0;
   s->one_sided = 0;
+  s->n_end = s->n_node = 0;
   s->mg_fail = 0;
   s->n_near_pole = 0;
 }
@@ -182,14 +183,11 @@ __device__ __forceinline__ double advect_bin_one(const Consts& c, const Dev& d, 
 }
 
 // ------------------------------------------------------------------------------- mirrors
-enum SelKind { SEL_CIRCLES = 0, SEL_WALL, SEL_PERIODIC, SEL_CORNER_WW, SEL_CORNER_PP, SEL_CORNER_WP };
+enum SelKind { SEL_CIRCLES = 0, SEL_WALL, SEL_PERIODIC, SEL_CORNER_WW, SEL_CORNER_PP, SEL_CORNER_WP, SEL_CANDIDATES };
 
 struct SelArgs {
   int kind;
   int ib;      // patch (0-based)
-  int n0;      // first item
-  int n1;      // end item (static kinds)
-  int cand;    // 1: the items are the candidate list (particles 0..npfb near a boundary), from n0
 };
 
 // near-patch test of create_boundary_boxes: |perp| <= sup+1e-10 and 0<=tmp<=1
@@ -209,12 +207,9 @@ __device__ __forceinline__ bool near_corner(const Consts& c, double x, double y,
   return !(dd > c.sup_size + 1.0e-10);
 }
 
-__device__ __forceinline__ int sel_end(const Consts& c, const Dev& d, const SelArgs& a) {
-  return a.kind == SEL_CORNER_WP ? c.npfb + d.s->imp_temp : a.n1;
-}
-
-// number of mirrors item `it` creates in this stage
-__device__ int sel_count(const Consts& c, const Dev& d, const SelArgs& a, int it) {
+// number of mirrors item `it` creates in this stage.  A call, for the few items that pass an FP32
+// test: inlined, the compiler computes its quotients for every particle.
+static __device__ __noinline__ int sel_count(const Consts& c, const Dev& d, const SelArgs& a, int it) {
   const double x = d.rx[it], y = d.ry[it];
   switch (a.kind) {
     case SEL_CIRCLES: {
@@ -274,7 +269,7 @@ __device__ __forceinline__ double dPf(const Consts& c, double xk, double yk, dou
 }
 
 // write the mirrors of item `it` starting at mirror slot `slot` (0-based mirror number)
-__device__ void sel_emit(const Consts& c, const Dev& d, const SelArgs& a, int it, int slot) {
+static __device__ __noinline__ void sel_emit(const Consts& c, const Dev& d, const SelArgs& a, int it, int slot) {
   const double x = d.rx[it], y = d.ry[it];
   auto put = [&](int parent, int vrel, double mx, double my, double mu, double mv, double mth,
                  double dp) -> void {
@@ -389,114 +384,30 @@ __device__ void sel_emit(const Consts& c, const Dev& d, const SelArgs& a, int it
   }
 }
 
-// per-block item counts
-// item q of a stage: a particle or mirror index, or -1 past the end.  In candidate mode the
-// items are the ascending candidate list, and those below n0 count nothing, so every stage
-// still visits its items in ascending index order.
-__device__ __forceinline__ int sel_item(const Consts& c, const Dev& d, const SelArgs& a, int q, int n1) {
-  if (a.cand) {
-    if (q >= d.s->n_cand) return -1;
-    const int it = d.cand[q];
-    return it >= a.n0 ? it : -1;
-  }
-  const int it = a.n0 + q;
-  return it < n1 ? it : -1;
-}
+// ---- the stages.  The reference makes circle images, then patch after patch wall and periodic
+// images, then corner after corner; the order of the mirrors is that of the stages and, in a
+// stage, of its items.  The stages over particles up to the corners depend on the particles alone,
+// so one kernel selects for all of them (a bit per particle and stage, and a count per block of
+// particles), one scan places the blocks and one kernel emits, a thread per mirror.  What a corner
+// needs -- the mirrors made so far past a wall's end, the particles about a node -- is a few dozen
+// items however large the domain: the emitting kernel lists them and one block runs the corners.
+// Measured, all of it: 0.06 to 0.08 ms a step from 1,700 to 20,000 particles, 0.26 ms at 4M; a
+// count, a scan and an emission per stage (33 to 43 launches) took 0.36 to 0.72 and 0.82 ms, these
+// kernels emitting from a thread per particle, its images in turn, 0.11 to 0.18 and 0.44 ms.
+//
+// Every FP64 test is preceded by an FP32 one with a margin of dx/10 plus 4e-6 of the box's extent,
+// far above its rounding error: a wall or periodic image needs |perp| <= sup + 1e-10 to that patch's
+// line, a corner image a node distance within the same bound, a circle image rad within R + sup (or
+// |R| - sup).
+constexpr int MIR_STAGES = VEBI_MAX_PATCHES + 2;  // circles, patches, candidates
+struct MirrorPlan {
+  int ns, nc;                                  // stages over particles (the candidates last), corners
+  int first_plane[MIR_STAGES + 1];             // of each stage's selections (a bit per particle)
+  signed char kind[MIR_STAGES], ib[MIR_STAGES];
+  signed char ckind[VEBI_MAX_PATCHES], cib[VEBI_MAX_PATCHES];
+};
 
-__global__ void k_sel_count(Consts c, Dev d, SelArgs a) {
-  __shared__ int sh[TPB / 32];
-  const int n1 = sel_end(c, d, a);
-  int base = blockIdx.x * SEL_CH + threadIdx.x * SEL_IPT;
-  int cnt = 0;
-  for (int q = 0; q < SEL_IPT; ++q) {
-    int it = sel_item(c, d, a, base + q, n1);
-    if (it >= 0) cnt += sel_count(c, d, a, it);
-  }
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = cnt;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < TPB / 32; ++w) t += sh[w];
-    d.sel_blk[blockIdx.x] = t;
-  }
-}
-
-// exclusive scan of the block counts (one block), and the stage's base mirror number
-__global__ void k_sel_scan(Dev d, int nblk, int mcap) {
-  __shared__ int sh[1024];
-  const int T = blockDim.x;
-  int per = (nblk + T - 1) / T;
-  int b0 = threadIdx.x * per, b1 = min(nblk, b0 + per);
-  int loc = 0;
-  for (int b = b0; b < b1; ++b) loc += d.sel_blk[b];
-  sh[threadIdx.x] = loc;
-  __syncthreads();
-  for (int o = 1; o < T; o <<= 1) {
-    int v = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-    __syncthreads();
-    sh[threadIdx.x] += v;
-    __syncthreads();
-  }
-  int run = sh[threadIdx.x] - loc;  // exclusive prefix of this thread's range
-  for (int b = b0; b < b1; ++b) {
-    int v = d.sel_blk[b];
-    d.sel_blk[b] = run;
-    run += v;
-  }
-  if (threadIdx.x == T - 1) {
-    int total = sh[T - 1];
-    Scal* s = d.s;
-    s->sel_base = s->nmirror;
-    s->sel_total = total;
-    long long nm = (long long)s->nmirror + total;
-    if (nm > mcap) { set_error(s, VEBI_ERR_MIRROR_CAPACITY); nm = mcap; }
-    s->nmirror = (int)nm;
-  }
-}
-
-// emit in item order: block offset + ordered prefix inside the block
-__global__ void k_sel_emit(Consts c, Dev d, SelArgs a) {
-  __shared__ int sh[TPB / 32 + 1];
-  const int n1 = sel_end(c, d, a);
-  int base = blockIdx.x * SEL_CH + threadIdx.x * SEL_IPT;
-  int cnts[SEL_IPT], items[SEL_IPT];
-  int tot = 0;
-  for (int q = 0; q < SEL_IPT; ++q) {
-    items[q] = sel_item(c, d, a, base + q, n1);
-    cnts[q] = items[q] >= 0 ? sel_count(c, d, a, items[q]) : 0;
-    tot += cnts[q];
-  }
-  // block exclusive scan of tot in thread order
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int inc = tot;
-  for (int o = 1; o < 32; o <<= 1) {
-    int v = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += v;
-  }
-  if (lane == 31) sh[w] = inc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int q = 0; q < TPB / 32; ++q) { int v = sh[q]; sh[q] = run; run += v; }
-  }
-  __syncthreads();
-  int slot = d.s->sel_base + d.sel_blk[blockIdx.x] + sh[w] + inc - tot;
-  for (int q = 0; q < SEL_IPT; ++q) {
-    if (cnts[q]) {
-      sel_emit(c, d, a, items[q], slot);
-      slot += cnts[q];
-    }
-  }
-}
-
-// The candidates of the mirror stages: particles 0..npfb within the support of a boundary line
-// or a circle.  Every item any stage over particles can select is one: a wall or periodic
-// image needs |perp| <= sup + 1e-10 to that patch's line, a corner image a node distance within
-// the same bound (the node is on both lines), a circle image rad within R + sup (or |R| - sup).
-// The test runs in FP32 with a margin of dx/10 plus 4e-6 of the box's extent, far above its
-// rounding error, so the list is a superset of every stage's selection; the stages then apply
-// their own FP64 tests.
+// the candidates: every particle that any stage may select, in ascending order (k_circle_force)
 struct NearTab {
   float a[VEBI_MAX_PATCHES], b[VEBI_MAX_PATCHES], c0[VEBI_MAX_PATCHES];  // perp = a x + b y + c0
   float cx[VEBI_MAX_CIRCLES], cy[VEBI_MAX_CIRCLES], lo2[VEBI_MAX_CIRCLES], hi2[VEBI_MAX_CIRCLES];
@@ -529,8 +440,7 @@ __device__ void near_table(const Consts& c, NearTab& t) {
   __syncthreads();
 }
 
-__device__ __forceinline__ bool near_boundary(const NearTab& t, double xd, double yd) {
-  const float x = (float)xd, y = (float)yd;
+__device__ __forceinline__ bool near_boundary(const NearTab& t, float x, float y) {
   for (int k = 0; k < t.np; ++k)
     if (fabsf(fmaf(t.a[k], x, fmaf(t.b[k], y, t.c0[k]))) <= t.band) return true;
   for (int ic = 0; ic < t.nc; ++ic) {
@@ -541,111 +451,287 @@ __device__ __forceinline__ bool near_boundary(const NearTab& t, double xd, doubl
   return false;
 }
 
-__global__ void k_cand_count(Consts c, Dev d) {
-  __shared__ int sh[TPB / 32];
-  __shared__ NearTab t;
-  near_table(c, t);
-  const int base = blockIdx.x * SEL_CH + threadIdx.x * SEL_IPT;
-  int cnt = 0;
-  for (int q = 0; q < SEL_IPT; ++q) {
-    const int it = base + q;
-    if (it < c.npfb && near_boundary(t, d.rx[it], d.ry[it])) ++cnt;
+// FP32 test of the stages over particles, one bit per stage
+struct StageTab {
+  float a[MIR_STAGES], b[MIR_STAGES], c0[MIR_STAGES];
+  float band;
+};
+__device__ void stage_table(const Consts& c, const MirrorPlan& pl, StageTab& t) {
+  const int s = threadIdx.x;
+  if (s < pl.ns && (pl.kind[s] == SEL_WALL || pl.kind[s] == SEL_PERIODIC)) {
+    const int ib = pl.kind[s] == SEL_PERIODIC ? c.b_pp[pl.ib[s]] : pl.ib[s];
+    t.a[s] = c.bl_a[ib];
+    t.b[s] = c.bl_b[ib];
+    t.c0[s] = c.bl_c[ib];
   }
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = cnt;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int tt = 0;
-    for (int w = 0; w < TPB / 32; ++w) tt += sh[w];
-    d.cand_blk[blockIdx.x] = tt;
+  t.band = c.near_band;
+}
+__device__ __forceinline__ unsigned stages_near(const Consts& c, const MirrorPlan& pl, const StageTab& t, int it, float x,
+                                                float y) {
+  unsigned m = 0;
+  for (int s = 0; s < pl.ns; ++s) {
+    if (pl.kind[s] == SEL_CIRCLES) {
+      if (it < c.nbS) continue;
+      bool near = false;
+      for (int ic = 0; ic < c.ncirc; ++ic) {
+        const float R = (float)c.c_radius[ic], r1 = x - (float)c.c_centre[ic][0], r2 = y - (float)c.c_centre[ic][1];
+        const float q = fmaf(r1, r1, r2 * r2), e = fabsf(R) - t.band;
+        near |= R > 0.0f ? q <= (R + t.band) * (R + t.band) : (e <= 0.0f || q >= e * e);
+      }
+      if (near) m |= 1u << s;
+    } else if (pl.kind[s] != SEL_CANDIDATES && fabsf(fmaf(t.a[s], x, fmaf(t.b[s], y, t.c0[s]))) <= t.band) {
+      m |= 1u << s;
+    }
   }
+  return m;
 }
 
-__global__ void k_cand_scan(Dev d, int nblk) {
-  __shared__ int sh[1024];
-  const int T = blockDim.x;
-  const int per = (nblk + T - 1) / T;
-  const int b0 = threadIdx.x * per, b1 = min(nblk, b0 + per);
+// what the corners may select, in FP32: mirrors by the line of a wall, past the end of it that is
+// the corner; particles about a corner's node
+__device__ __forceinline__ int corner_wall(const Consts& c, int ib) {
+  const int ibm1 = (ib + c.nb - 1) % c.nb;
+  return c.b_type[ibm1] == 1 ? ibm1 : ib;
+}
+__device__ __forceinline__ bool past_wall_end(const Consts& c, const MirrorPlan& pl, float x, float y) {
+  const float slack = c.near_band - (float)c.sup_size;
+  for (int q = 0; q < pl.nc; ++q) {
+    if (pl.ckind[q] != SEL_CORNER_WP) continue;
+    const int ib = pl.cib[q], wl = corner_wall(c, ib);
+    const float perp = fmaf(c.bl_a[wl], x, fmaf(c.bl_b[wl], y, c.bl_c[wl]));
+    if (!(perp >= -slack && perp <= c.near_band)) continue;
+    const float len = (float)c.b_elen[wl];
+    const float along = ((x - (float)c.b_node[wl][0]) * (float)c.b_edge[wl][0] +
+                         (y - (float)c.b_node[wl][1]) * (float)c.b_edge[wl][1]) / len;
+    if (wl == ib ? along < slack : along > len - slack) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ bool by_a_node(const Consts& c, const MirrorPlan& pl, float x, float y) {
+  for (int q = 0; q < pl.nc; ++q) {
+    if (pl.ckind[q] == SEL_CORNER_WP) continue;
+    const int k = pl.ckind[q] == SEL_CORNER_PP ? c.b_pp[pl.cib[q]] : pl.cib[q];
+    const float r1 = x - (float)c.b_node[k][0], r2 = y - (float)c.b_node[k][1];
+    if (fmaf(r1, r1, r2 * r2) <= c.near_band * c.near_band) return true;
+  }
+  return false;
+}
+
+// particles of a block: small domains take small blocks, to fill the GPU; large ones fewer of them,
+// for the scan by one block (4M particles: 3,907 counts a stage)
+inline int mirror_block(int n) { return n > 200000 ? 4 * TPB : TPB; }
+
+template <int IPT>
+__global__ void __launch_bounds__(TPB) k_mirror_select(const __grid_constant__ Consts c, const __grid_constant__ Dev d,
+                                                       const __grid_constant__ MirrorPlan pl) {
+  __shared__ int cnt[MIR_STAGES];
+  __shared__ StageTab st;
+  __shared__ NearTab t;
+  if (threadIdx.x < MIR_STAGES) cnt[threadIdx.x] = 0;
+  stage_table(c, pl, st);
+  near_table(c, t);
+  const int words = (c.npfb + 31) / 32;
+  for (int q = 0; q < IPT; ++q) {
+    const int it = (blockIdx.x * IPT + q) * TPB + threadIdx.x;
+    const int word = it >> 5;
+    const bool in = it < c.npfb;
+    float x = 0.f, y = 0.f;
+    if (in) {
+      x = narrow(d.rx[it]);
+      y = narrow(d.ry[it]);
+    }
+    const unsigned near = in ? stages_near(c, pl, st, it, x, y) : 0u;
+    for (int s = 0; s < pl.ns; ++s) {
+      int n = 0;
+      if (pl.kind[s] == SEL_CANDIDATES) n = in && near_boundary(t, x, y) ? 1 : 0;
+      else if ((near >> s) & 1u) n = sel_count(c, d, SelArgs{pl.kind[s], pl.ib[s]}, it);
+      // plane e of a stage: particles with more than e images in it
+      for (int e = 0; e < pl.first_plane[s + 1] - pl.first_plane[s]; ++e) {
+        const unsigned b = __ballot_sync(0xffffffffu, n > e);
+        if ((threadIdx.x & 31) == 0 && word < words) {
+          d.sel_bits[(size_t)(pl.first_plane[s] + e) * words + word] = b;
+          if (b) atomicAdd(&cnt[s], __popc(b));
+        }
+      }
+    }
+    if (in && it >= c.nbS && by_a_node(c, pl, x, y)) {
+      const int k = atomicAdd(&d.s->n_node, 1);
+      if (k < MIR_LIST) d.mir_list[MIR_LIST + k] = it;
+    }
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < pl.ns) d.sel_blk[threadIdx.x * gridDim.x + blockIdx.x] = cnt[threadIdx.x];
+}
+
+// exclusive scan in place of the stages' block counts, stage after stage; the total after the last
+// one; nmir: entries of the stages that make mirrors
+__global__ void __launch_bounds__(1024) k_mirror_scan(Dev d, int n, int nmir, int mcap) {
+  __shared__ int sh[32];
+  int* const v = d.sel_blk;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int per = (n + 1023) / 1024, b0 = threadIdx.x * per, b1 = min(n, b0 + per);
   int loc = 0;
-  for (int b = b0; b < b1; ++b) loc += d.cand_blk[b];
-  sh[threadIdx.x] = loc;
-  __syncthreads();
-  for (int o = 1; o < T; o <<= 1) {
-    int v = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-    __syncthreads();
-    sh[threadIdx.x] += v;
-    __syncthreads();
-  }
-  int run = sh[threadIdx.x] - loc;
-  for (int b = b0; b < b1; ++b) {
-    int v = d.cand_blk[b];
-    d.cand_blk[b] = run;
-    run += v;
-  }
-  if (threadIdx.x == T - 1) d.s->n_cand = sh[T - 1];
-}
-
-__global__ void k_cand_emit(Consts c, Dev d) {
-  __shared__ int sh[TPB / 32 + 1];
-  __shared__ NearTab t;
-  near_table(c, t);
-  const int base = blockIdx.x * SEL_CH + threadIdx.x * SEL_IPT;
-  bool f[SEL_IPT];
-  int tot = 0;
-  for (int q = 0; q < SEL_IPT; ++q) {
-    const int it = base + q;
-    f[q] = it < c.npfb && near_boundary(t, d.rx[it], d.ry[it]);
-    tot += f[q] ? 1 : 0;
-  }
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int inc = tot;
+  for (int b = b0; b < b1; ++b) loc += v[b];
+  int inc = loc;
   for (int o = 1; o < 32; o <<= 1) {
-    int v = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += v;
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
   }
   if (lane == 31) sh[w] = inc;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int q = 0; q < TPB / 32; ++q) { int v = sh[q]; sh[q] = run; run += v; }
+  if (w == 0) {
+    int u = sh[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int z = __shfl_up_sync(0xffffffffu, u, o);
+      if (lane >= o) u += z;
+    }
+    sh[lane] = u;
   }
   __syncthreads();
-  int slot = d.cand_blk[blockIdx.x] + sh[w] + inc - tot;
-  for (int q = 0; q < SEL_IPT; ++q)
-    if (f[q]) d.cand[slot++] = base + q;
+  int run = (w ? sh[w - 1] : 0) + inc - loc;
+  for (int b = b0; b < b1; ++b) {
+    const int u = v[b];
+    v[b] = run;
+    run += u;
+  }
+  if (threadIdx.x == 0) v[n] = sh[31];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int total = nmir < n ? v[nmir] : sh[31];
+    if (total > mcap) set_error(d.s, VEBI_ERR_MIRROR_CAPACITY);
+    d.s->nmirror = min(total, mcap);
+    d.s->n_cand = sh[31] - total;
+  }
 }
 
-__global__ void k_snapshot_imp(Scal* s) { s->imp_temp = s->nmirror; }
-
-// mirrors of moving solid particles copy their parent's u and theta (mirror_..:191-206)
-__global__ void k_solid_fixup(Consts c, Dev d) {
-  const int nm = d.s->nmirror;
-  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < nm; m += gridDim.x * blockDim.x) {
-    int j = c.npfb + m, i = d.irel[j];
-    if (i < c.nbS) {
-      double tmp = d.ux[i] * d.ux[i] + d.uy[i] * d.uy[i];
-      if (tmp != 0.0) { d.ux[j] = d.ux[i]; d.uy[j] = d.uy[i]; }
-      double tt = d.th[i] * d.th[i];
-      if (tt != 0.0) d.th[j] = d.th[i];
+// Mirrors of the stages over particles, a thread per mirror (and per candidate): its stage and block
+// from the scan, its particle from the block's selection bits.  So the FP64 work runs on full
+// warps; a warp of 32 consecutive particles has a few that are selected, if any.  A mirror of a
+// moving solid particle copies its parent's u and theta (mirror_..:191-206).
+template <int IPT>
+__global__ void __launch_bounds__(TPB) k_mirror_emit(const __grid_constant__ Consts c, const __grid_constant__ Dev d,
+                                                     const __grid_constant__ MirrorPlan pl, int nblk) {
+  constexpr int W = IPT * TPB / 32;  // words of a block's bits
+  const int n = pl.ns * nblk, words = (c.npfb + 31) / 32;
+  const int total = d.sel_blk[n], nmir = total - d.s->n_cand;
+  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < total; m += gridDim.x * blockDim.x) {
+    int lo = 0, hi = n;  // the last entry that starts at or before m
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (d.sel_blk[mid] <= m) lo = mid;
+      else hi = mid;
+    }
+    const int s = lo / nblk, b = lo % nblk;
+    int r = m - d.sel_blk[lo];
+    const int p0 = pl.first_plane[s], np = pl.first_plane[s + 1] - p0;
+    const unsigned* bits = d.sel_bits + (size_t)p0 * words + b * W;
+    int word = 0;
+    for (; word < W; ++word) {
+      int k = 0;
+      for (int e = 0; e < np; ++e) k += __popc(bits[(size_t)e * words + word]);
+      if (r < k) break;
+      r -= k;
+    }
+    int bit = 0;
+    for (;; ++bit) {
+      int k = 0;
+      for (int e = 0; e < np; ++e) k += (bits[(size_t)e * words + word] >> bit) & 1u;
+      if (r < k) break;
+      r -= k;
+    }
+    const int it = (b * W + word) * 32 + bit;
+    if (pl.kind[s] == SEL_CANDIDATES) {
+      d.cand[m - nmir] = it;
+      continue;
+    }
+    if (r) continue;  // a particle's images in one stage are emitted together
+    int made = 0;
+    for (int e = 0; e < np; ++e) made += (bits[(size_t)e * words + word] >> bit) & 1u;
+    sel_emit(c, d, SelArgs{pl.kind[s], pl.ib[s]}, it, m);
+    for (int e = m; e < m + made && e < c.mcap; ++e) {
+      const int j = c.npfb + e;
+      if (it < c.nbS) {
+        const double u = d.ux[it], v = d.uy[it], th = d.th[it];
+        if (u * u + v * v != 0.0) { d.ux[j] = u; d.uy[j] = v; }
+        if (th * th != 0.0) d.th[j] = th;
+      }
+      if (past_wall_end(c, pl, narrow(d.rx[j]), narrow(d.ry[j]))) {
+        const int k = atomicAdd(&d.s->n_end, 1);
+        if (k < MIR_LIST) d.mir_list[k] = j;
+      }
     }
   }
 }
 
-__global__ void k_set_np(Consts c, Scal* s) {
-  s->np = c.npfb + s->nmirror;
-  s->relax = exp(-(1.0 * 1.0 * s->dt / c.Wi));  // as k_logconf's with alpha_R = 1; dt may be a replayed step's
+// ascending copy of n distinct items (each to its rank), or false when they do not fit
+__device__ bool sorted_list(const int* src, int n, int* dst) {
+  if (n > MIR_LIST) return false;
+  for (int e = threadIdx.x; e < n; e += blockDim.x) {
+    const int v = src[e];
+    int r = 0;
+    for (int k = 0; k < n; ++k) r += src[k] < v ? 1 : 0;
+    dst[r] = v;
+  }
+  return true;
 }
 
-static void run_stage(Ctx& x, int kind, int ib, int n0, int n1_static, int n_items_bound) {
-  // stages over particles (their items end at npfb) walk the candidate list instead
-  const int cand = n1_static == x.c.npfb ? 1 : 0;
-  SelArgs a{kind, ib, n0, n1_static, cand};
-  if (cand) n_items_bound = x.c.npfb;  // the list can hold every particle, walls included
-  int nblk = (n_items_bound + SEL_CH - 1) / SEL_CH;
-  if (nblk < 1) nblk = 1;
-  VEBI_LAUNCH(x, k_sel_count, nblk, TPB, x.c, x.d, a);
-  VEBI_LAUNCH(x, k_sel_scan, 1, 1024, x.d, nblk, x.c.mcap);
-  VEBI_LAUNCH(x, k_sel_emit, nblk, TPB, x.c, x.d, a);
+// The corners, one after the other, by one block: each takes its items in ascending order -- from
+// the lists, or all mirrors or particles if a list overflowed -- and appends its mirrors.  Then np
+// and the step's relaxation factor.
+__global__ void __launch_bounds__(1024) k_mirror_corners(const __grid_constant__ Consts c, const __grid_constant__ Dev d,
+                                                         const __grid_constant__ MirrorPlan pl) {
+  __shared__ int ends[MIR_LIST], nodes[MIR_LIST], wsum[32];
+  Scal* const s = d.s;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int imp = s->nmirror;
+  int n_ends = 0, n_nodes = 0;
+  bool all_ends = false, all_nodes = false;
+  if (pl.nc) {
+    n_ends = s->n_end;
+    n_nodes = s->n_node;
+    all_ends = !sorted_list(d.mir_list, n_ends, ends);
+    all_nodes = !sorted_list(d.mir_list + MIR_LIST, n_nodes, nodes);
+    __syncthreads();
+  }
+  for (int q = 0; q < pl.nc; ++q) {
+    const SelArgs a{pl.ckind[q], pl.cib[q]};
+    const bool wp = a.kind == SEL_CORNER_WP, all = wp ? all_ends : all_nodes;
+    const int total = all ? (wp ? imp : c.npfb - c.nbS) : (wp ? n_ends : n_nodes);
+    const int imp0 = imp;  // the mirrors a corner makes are not its own items
+    for (int e0 = 0; e0 < total; e0 += 1024) {
+      const int e = e0 + threadIdx.x;
+      const int it = e >= total ? -1 : all ? (wp ? c.npfb : c.nbS) + e : wp ? ends[e] : nodes[e];
+      const bool mine = it >= 0 && sel_count(c, d, a, it) != 0;
+      const unsigned b = __ballot_sync(0xffffffffu, mine);
+      if (lane == 0) wsum[w] = __popc(b);
+      __syncthreads();
+      int before = 0, made = 0;
+      for (int k = 0; k < 32; ++k) {
+        before += k < w ? wsum[k] : 0;
+        made += wsum[k];
+      }
+      if (mine) sel_emit(c, d, a, it, imp + before + __popc(b & ((1u << lane) - 1u)));
+      imp += made;
+      __syncthreads();
+    }
+    if (imp > c.mcap) {
+      if (threadIdx.x == 0) set_error(s, VEBI_ERR_MIRROR_CAPACITY);
+      imp = c.mcap;
+    }
+    if (!all_ends) {  // the new mirrors are items of the corners that follow
+      if (n_ends + imp - imp0 <= MIR_LIST) {
+        for (int e = imp0 + threadIdx.x; e < imp; e += 1024) ends[n_ends + e - imp0] = c.npfb + e;
+        n_ends += imp - imp0;
+      } else {
+        all_ends = true;
+      }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    s->nmirror = imp;
+    s->np = c.npfb + imp;
+    s->relax = exp(-(1.0 * 1.0 * s->dt / c.Wi));  // as k_logconf's with alpha_R = 1; dt may be a replayed step's
+  }
 }
 
 void launch_advect_bin(Ctx& x) {
@@ -658,33 +744,42 @@ void launch_advect_bin(Ctx& x) {
 // create_mirror_particles (mirror_boundaries_mod.F90:18-334)
 void launch_mirrors(Ctx& x) {
   const Consts& c = x.c;
-  {  // the candidate list of the stages over particles, in ascending index
-    const int nblk = (c.npfb + SEL_CH - 1) / SEL_CH;
-    VEBI_LAUNCH(x, k_cand_count, nblk, TPB, c, x.d);
-    VEBI_LAUNCH(x, k_cand_scan, 1, 1024, x.d, nblk);
-    VEBI_LAUNCH(x, k_cand_emit, nblk, TPB, c, x.d);
-  }
-  if (c.ncirc > 0) run_stage(x, SEL_CIRCLES, 0, c.nbS, c.npfb, c.npfb - c.nbS);
+  MirrorPlan pl{};
+  auto stage = [&](int kind, int ib, int planes) {
+    pl.kind[pl.ns] = (signed char)kind;
+    pl.ib[pl.ns] = (signed char)ib;
+    pl.first_plane[pl.ns + 1] = pl.first_plane[pl.ns] + planes;
+    ++pl.ns;
+  };
+  auto corner = [&](int kind, int ib) {
+    pl.ckind[pl.nc] = (signed char)kind;
+    pl.cib[pl.nc++] = (signed char)ib;
+  };
+  if (c.ncirc > 0) stage(SEL_CIRCLES, 0, c.ncirc);
   for (int ib = 0; ib < c.nb; ++ib) {
-    if (c.b_type[ib] == 1) run_stage(x, SEL_WALL, ib, 0, c.npfb, c.npfb);
-    if (c.b_type[ib] == 2) run_stage(x, SEL_PERIODIC, ib, 0, c.npfb, c.npfb);
+    if (c.b_type[ib] == 1) stage(SEL_WALL, ib, 1);
+    if (c.b_type[ib] == 2) stage(SEL_PERIODIC, ib, 1);
   }
-  VEBI_LAUNCH(x, k_solid_fixup, x.gs_blocks, TPB, c, x.d);
+  const int made = pl.ns;
+  if (c.ncirc > 0) stage(SEL_CANDIDATES, 0, 1);
   for (int ib = 0; ib < c.nb; ++ib) {
     int ibm1 = (ib + c.nb - 1) % c.nb;
     if (c.b_type[ib] == 0 || c.b_type[ibm1] == 0) continue;
     double tmp = c.b_edge[ibm1][0] * c.b_edge[ib][1] - c.b_edge[ibm1][1] * c.b_edge[ib][0];
     if (fabs(tmp) < 1e-10) continue;
-    if (c.b_type[ib] == 1 && c.b_type[ibm1] == 1) {
-      if (!(c.b_corner_angle[ib] <= 0.0)) run_stage(x, SEL_CORNER_WW, ib, c.nbS, c.npfb, c.npfb - c.nbS);
-    }
-    if (c.b_type[ib] == 2 && c.b_type[ibm1] == 2) run_stage(x, SEL_CORNER_PP, ib, c.nbS, c.npfb, c.npfb - c.nbS);
-    if (c.b_type[ib] != c.b_type[ibm1] && (c.b_type[ib] == 1 || c.b_type[ibm1] == 1)) {
-      VEBI_LAUNCH(x, k_snapshot_imp, 1, 1, x.d.s);
-      run_stage(x, SEL_CORNER_WP, ib, c.npfb, 0, c.mcap);
-    }
+    if (c.b_type[ib] == 1 && c.b_type[ibm1] == 1 && !(c.b_corner_angle[ib] <= 0.0)) corner(SEL_CORNER_WW, ib);
+    if (c.b_type[ib] == 2 && c.b_type[ibm1] == 2) corner(SEL_CORNER_PP, ib);
+    if (c.b_type[ib] != c.b_type[ibm1] && (c.b_type[ib] == 1 || c.b_type[ibm1] == 1)) corner(SEL_CORNER_WP, ib);
   }
-  VEBI_LAUNCH(x, k_set_np, 1, 1, c, x.d.s);
+  const int per = mirror_block(c.npfb), nblk = (c.npfb + per - 1) / per;
+  // the emitting grid: a thread per mirror of a domain's usual number, more by striding
+  const int emit = nblk < 4 * x.nsm ? (nblk < 8 ? 8 : nblk) : 4 * x.nsm;
+  if (per == TPB) VEBI_LAUNCH(x, k_mirror_select<1>, nblk, TPB, c, x.d, pl);
+  else VEBI_LAUNCH(x, k_mirror_select<4>, nblk, TPB, c, x.d, pl);
+  VEBI_LAUNCH(x, k_mirror_scan, 1, 1024, x.d, pl.ns * nblk, made * nblk, c.mcap);
+  if (per == TPB) VEBI_LAUNCH(x, k_mirror_emit<1>, emit, TPB, c, x.d, pl, nblk);
+  else VEBI_LAUNCH(x, k_mirror_emit<4>, emit, TPB, c, x.d, pl, nblk);
+  VEBI_LAUNCH(x, k_mirror_corners, 1, 1024, c, x.d, pl);
 }
 
 // ------------------------------------------------------------------------------- mirror fields

@@ -404,7 +404,7 @@ __device__ __forceinline__ void calc_eigens(const M2& A, double& L1, double& L2,
     R = M2{1.0, 0.0, 0.0, 1.0};
   }
 }
-// the relaxation factor exp(-(alpha_R dt / Wi)); alpha_R = 1 is the step's own (k_set_np)
+// the relaxation factor exp(-(alpha_R dt / Wi)); alpha_R = 1 is the step's own (k_mirror_corners)
 static __device__ __noinline__ double relaxation(double alpha_R, double dt, double Wi) {
   return exp(-(alpha_R * 1.0 * dt / Wi));
 }
