@@ -154,13 +154,17 @@ VF_FN bool exact_residual(double a) { return exponent(hi(a)) > 110; }
 VF_FN double quotient_near(double a, double b, double y, double q) {
   return settle(q, fma(-b, q, a), y, 0) && exact_residual(a) ? q : divided(a, b);
 }
+VF_FN double magnitude(double x) { return pack(hi(x) & 0x7fffffff, lo(x)); }
 // a / b for any b, from y = 1 / |b| to some 45 bits
 VF_FN double quotient(double a, double b, double y) {
   if (is_zero(a)) return divided(a, b);
   const double ys = pack((int)((uint32_t)hi(y) | ((uint32_t)hi(b) & 0x80000000u)), lo(y));
   return quotient_near(a, b, ys, a * ys);
 }
-VF_FN double magnitude(double x) { return pack(hi(x) & 0x7fffffff, lo(x)); }
+// a / b; where 1 / b is not a normal number (as of 0, NaN or an infinity), as divided
+VF_FN double quotient(double a, double b) {
+  return (uint32_t)(exponent(hi(b)) - 1) < 2044u ? quotient(a, b, reciprocal(magnitude(b))) : divided(a, b);
+}
 // sqrt(x); y = reciprocal_root(x)
 VF_FN double root(double x, double& y) {
   y = reciprocal_root(x);

@@ -4,8 +4,8 @@
 // memory (raw allocations are forbidden or invisible to its accounting), or a real-time time
 // loop that must not allocate once it runs.  For them vebi_ppe_solve_noalloc runs the same
 // BiCGSTAB as the time step on an ELL matrix and right-hand side the caller already holds in
-// device memory, and keeps its Krylov vectors, block partial sums and barrier state in the
-// file-scope array below instead of in allocated buffers.
+// device memory, and keeps its Krylov vectors, block partial sums and barrier state in registers
+// and in the file-scope array below instead of in allocated buffers.
 //
 // Limits and rules of the shared array:
 //  * at most VEBI_NOALLOC_MAX_ROWS rows (65536); larger systems are rejected with VEBI_ERR_ARG;
@@ -23,7 +23,8 @@
 #include <mutex>
 #include <string>
 
-#include "vebi_ctx.cuh"
+#include "vebi_fp64.cuh"
+#include "vebi_resident.cuh"
 
 namespace vebi {
 
@@ -146,6 +147,10 @@ __device__ __forceinline__ double na_spmv(const NaArgs& a, const double* xv, int
   }
   return bb;
 }
+
+constexpr int NA_T_MAX = 512;  // rows of a block, one thread a row
+constexpr int NA_AHEAD = 16;   // a row's operands loaded at a time
+constexpr int NA_KEEP = 64;    // slots of a row held in shared memory, if it takes as many
 
 // SPARSE_PBICGSTAB_nonull / SPARSE_PBICGSTAB (linear_solver.F90:275-425 / 82-227) with x0 = 0
 template <bool NONULL>
@@ -278,11 +283,155 @@ __global__ void __launch_bounds__(TPB) k_na_bicgstab(NaArgs a) {
   }
 }
 
+// The same solve for up to NA_T_MAX rows per SM: the rows dealt in groups of 32 to one block per SM
+// (vebi_resident.cuh), a row a thread.  The row's vectors stay in registers and its first slots in
+// shared memory for the whole solve, so a product waits for L2 once per NA_AHEAD operands, all of
+// them in flight, and not twice per slot; only p_inv, s_inv and the partial sums pass through L2.
+// A row's product is one chain in slot order and every sum keeps k_na_bicgstab's order, so the
+// solution is that kernel's bit for bit.
+// What bounds it: up to two warps a scheduler, the chain of an iteration (seven barriers, five
+// sums, two products of 45 dependent FMAs), ~24 us; above that the FP64 pipe, at ~150 operations a row.
+// Measured against k_na_bicgstab, ms per solve: 576 rows x 24 iterations 0.57 / 1.45, 16k x 98
+// 2.70 / 6.29, 36k x 142 4.90 / 9.61, 65k x 196 8.4 / 15.7.
+template <bool NONULL>
+__global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, int nvb, int keep) {
+  extern __shared__ double na_mat[];  // the first `keep` slots of the block's rows: values, then columns
+  __shared__ ResSh sh;
+  NaCtrl* ctl = reinterpret_cast<NaCtrl*>(a.scratch);
+  const GridBar bar{&ctl->bar_count, &ctl->error};
+  const int n = a.n, t = threadIdx.x, R = blockDim.x;
+  const int i = blockIdx.x * R + t;
+  const bool mine = i < n;
+  double* const pinv_all = a.scratch + NA_CTRL;
+  double* const sinv_all = pinv_all + VEBI_NOALLOC_MAX_ROWS;
+  double* const part0 = sinv_all + VEBI_NOALLOC_MAX_ROWS;
+  double* const part1 = part0 + 2 * (size_t)nvb * RES_VB;  // used in turn: a slow block may still read one
+  const double small = NONULL ? 1.0e-6 : 4.0, dn = (double)n;
+  double* const vals = na_mat + t;
+  int* const cols = reinterpret_cast<int*>(na_mat + (size_t)keep * R) + t;
+  const int cnt = mine ? a.cnt[i] : 0;
+  for (int k = 0; k < keep && k < cnt; ++k) {
+    vals[k * R] = a.val[(size_t)k * a.stride + i];
+    cols[k * R] = a.col[(size_t)k * a.stride + i];
+  }
+  if (t == 0) {
+    sh.alpha = sh.omega = sh.n2r0 = sh.n2s0 = 1.0;
+    sh.beta = sh.n2 = 0.0;
+  }
+  const double di = mine ? a.diag[i] : 0.0;
+  const double den = NONULL ? (1.0 + 1.0e-15) : (di + 1.0e-15), rden = fp::reciprocal(fp::magnitude(den));
+  const double rdn = fp::reciprocal(dn);
+  // A's row times xv, slot after slot; NA_AHEAD operands are loaded at a time, before the chain
+  // that adds those before them.  The chain is left by a branch for the whole warp: predicated off,
+  // an FMA still takes its 64 cycles.
+  const int shared_slots = min(cnt, keep), warp_slots = __reduce_max_sync(0xffffffffu, shared_slots);
+  auto product = [&](const double* xv) {
+    double u[2][NA_AHEAD];
+    auto fetch = [&](int k0, double* o) {
+#pragma unroll
+      for (int e = 0; e < NA_AHEAD; ++e) o[e] = k0 + e < shared_slots ? __ldca(xv + cols[(k0 + e) * R]) : 0.0;
+    };
+    auto chain = [&](int k0, const double* o, double& b) {
+#pragma unroll
+      for (int e = 0; e < NA_AHEAD; ++e) {
+        if (e % 2 == 0 && k0 + e >= warp_slots) return;
+        if (k0 + e < shared_slots) b = fma(vals[(k0 + e) * R], o[e], b);
+      }
+    };
+    fetch(0, u[0]);
+    double b = mine ? di * __ldca(xv + i) : 0.0;
+#pragma unroll 1
+    for (int k = 0; k < warp_slots; k += 2 * NA_AHEAD) {
+      fetch(k + NA_AHEAD, u[1]);
+      chain(k, u[0], b);
+      fetch(k + 2 * NA_AHEAD, u[0]);
+      chain(k + NA_AHEAD, u[1], b);
+    }
+    for (int k = keep; k < cnt; ++k) {
+      const size_t e = (size_t)k * a.stride + i;
+      b = fma(a.val[e], __ldcg(xv + a.col[e]), b);
+    }
+    return b;
+  };
+  double r = mine ? a.rhs[i] : 0.0, rb = r, v = 0.0, p = 0.0, x = 0.0;
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  auto failed = [&]() {
+    if (mine) a.x[i] = nan;
+  };
+  if (!res_reduce<1>(bar, mine ? plus_zero(r * r) : 0.0, 0.0, part1, gpb, nvb, sh, [&]() { sh.rho = sh.v[0]; }))
+    return failed();
+  int iter = 1, warn = 0;
+  bool done = false, at_s = false;
+  while (iter <= a.itermax) {
+    if (is_zero(sh.rho)) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
+    p = iter == 1 ? r : r + sh.beta * (p - sh.omega * v);
+    if (NONULL) {
+      if (!res_reduce<1>(bar, mine ? plus_zero(p) : 0.0, 0.0, part0, gpb, nvb, sh, [&]() { sh.mean = fp::quotient(sh.v[0], dn, rdn); }))
+        return failed();
+      p = p - sh.mean;
+    }
+    const double pinv = fp::quotient(p, den, rden);
+    if (mine) pinv_all[i] = pinv;
+    if (!res_sync(bar)) return failed();
+    v = product(pinv_all);
+    if (!res_reduce<1>(bar, mine ? plus_zero(rb * v) : 0.0, 0.0, part1, gpb, nvb, sh,
+                       [&]() { sh.alpha = fp::quotient(sh.rho, sh.v[0] + 1.0e-15); }))
+      return failed();
+    const double alpha = sh.alpha;
+    double s = r - alpha * v;
+    if (!res_reduce<2>(bar, mine ? plus_zero(s * s) : 0.0, mine ? plus_zero(s) : 0.0, part0, gpb, nvb, sh, [&]() {
+          sh.n2 = sh.v[0];
+          if (iter == 1) sh.n2s0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
+          sh.flag = sh.v[0] <= a.tol * a.tol * sh.n2s0;
+          if (NONULL) sh.mean = fp::quotient(sh.v[1], dn, rdn);
+        }))
+      return failed();
+    if (sh.flag) {
+      x = x + alpha * pinv;
+      done = at_s = true;
+      break;
+    }
+    if (NONULL) s = s - sh.mean;
+    const double sinv = fp::quotient(s, den, rden);
+    if (mine) sinv_all[i] = sinv;
+    if (!res_sync(bar)) return failed();
+    const double tv = product(sinv_all);
+    if (!res_reduce<2>(bar, mine ? plus_zero(tv * s) : 0.0, mine ? plus_zero(tv * tv) : 0.0, part1, gpb, nvb, sh,
+                       [&]() { sh.omega = fp::quotient(sh.v[0], sh.v[1] + 1.0e-15); }))
+      return failed();
+    const double omega = sh.omega;
+    x = x + alpha * pinv + omega * sinv;
+    r = s - omega * tv;
+    if (!res_reduce<2>(bar, mine ? plus_zero(r * r) : 0.0, mine ? plus_zero(rb * r) : 0.0, part0, gpb, nvb, sh, [&]() {
+          sh.n2 = sh.v[0];
+          if (iter == 1) sh.n2r0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
+          sh.flag = sh.v[0] <= a.tol * a.tol * sh.n2r0;
+          sh.beta = fp::quotient(fp::quotient(sh.v[1], sh.rho + 1.0e-15) * alpha, omega + 1.0e-15);
+          sh.rho = sh.v[1];
+        }))
+      return failed();
+    if (sh.flag) { done = true; break; }
+    iter = iter + 1;
+  }
+  if (!done) warn |= VEBI_WARN_MAXITER;
+  if (mine) a.x[i] = x;
+  if (blockIdx.x == 0 && t == 0) {
+    ctl->iters = iter;
+    ctl->residual = sqrt(sh.n2 / (at_s ? sh.n2s0 : sh.n2r0));
+    ctl->warnings = warn;
+  }
+}
+
 // per-device set-up: the scratch's device address, looked up with that device current
 constexpr int NA_MAX_DEVICES = 64;
 std::mutex g_mu;
-double* g_dev_addr[NA_MAX_DEVICES] = {};
-int g_blocks[NA_MAX_DEVICES] = {};
+struct NaDevice {
+  double* addr;
+  int blocks;  // co-resident blocks of k_na_bicgstab
+  int nsm;
+  int shared;  // bytes of dynamic shared memory a block of k_na_resident may have
+};
+NaDevice g_dev[NA_MAX_DEVICES] = {};
 
 }  // namespace
 }  // namespace vebi
@@ -315,29 +464,36 @@ extern "C" int vebi_ppe_solve_noalloc(const int32_t* ij_count, const int32_t* pp
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= NA_MAX_DEVICES)
     return na_fail(VEBI_ERR_NO_DEVICE, "vebi_ppe_solve_noalloc: no current CUDA device");
-  double* addr = nullptr;
-  int blocks = 0;
+  NaDevice g;
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (!g_dev_addr[dev]) {
+    NaDevice& q = g_dev[dev];
+    if (!q.addr) {
       void* p = nullptr;
       cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
       if (e != cudaSuccess || !p)
         return na_fail(VEBI_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
-      int nsm = 0, per = 0, per2 = 0;
+      int nsm = 0, per = 0, per2 = 0, shared = 0;
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_na_bicgstab<true>, TPB, 0);
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_na_bicgstab<false>, TPB, 0);
       per = per < per2 ? per : per2;
-      long long b = (long long)(per < 1 ? 1 : per) * (nsm < 1 ? 1 : nsm);
-      g_blocks[dev] = (int)(b > NA_MAX_BLOCKS ? NA_MAX_BLOCKS : b);
-      g_dev_addr[dev] = static_cast<double*>(p);
+      q.nsm = nsm < 1 ? 1 : nsm;
+      const long long b = (long long)(per < 1 ? 1 : per) * q.nsm;
+      q.blocks = (int)(b > NA_MAX_BLOCKS ? NA_MAX_BLOCKS : b);
+      cudaDeviceGetAttribute(&shared, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+      shared -= (int)sizeof(ResSh) + 1024;
+      if (shared > 0 &&
+          cudaFuncSetAttribute(k_na_resident<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared) == cudaSuccess &&
+          cudaFuncSetAttribute(k_na_resident<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared) == cudaSuccess)
+        q.shared = shared;
+      else
+        cudaGetLastError();  // k_na_bicgstab then
+      q.addr = static_cast<double*>(p);
     }
-    addr = g_dev_addr[dev];
-    blocks = g_blocks[dev];
+    g = q;
   }
-  long long need = ((long long)n + TPB - 1) / TPB;
-  if (need < blocks) blocks = (int)need;
+  double* const addr = g.addr;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (iters_out || residual_out) {
     // the read-back waits for the stream, which a stream being captured cannot do
@@ -353,16 +509,31 @@ extern "C" int vebi_ppe_solve_noalloc(const int32_t* ij_count, const int32_t* pp
   if (e != cudaSuccess) return na_fail(VEBI_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
   NaArgs a{ij_count, ppe_col, ppe_val, ppe_diag, rhs, x, (long long)ell_stride, n, closed_domain ? 1 : 0,
            itermax, tol, addr};
+  // k_na_resident wherever its rows fit, as it is the faster one up to the 65,536 rows of the array;
+  // k_na_bicgstab is for a GPU (or a slice of one) of fewer than n / NA_T_MAX SMs
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(TPB);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = closed_domain ? cudaLaunchKernelEx(&cfg, k_na_bicgstab<true>, a) : cudaLaunchKernelEx(&cfg, k_na_bicgstab<false>, a);
+  const int nvb = (n + TPB - 1) / TPB, groups = nvb * RES_VB;
+  int gpb = (groups + g.nsm - 1) / g.nsm;
+  if (gpb < 2) gpb = 2;  // two warps: one for each of two sums
+  const int rows = gpb * RES_GROUP;
+  const int fit = rows <= NA_T_MAX ? g.shared / (12 * rows) : 0, keep = fit < NA_KEEP ? fit : NA_KEEP;
+  if (keep > 0) {
+    cfg.gridDim = dim3((groups + gpb - 1) / gpb);
+    cfg.blockDim = dim3(rows);
+    cfg.dynamicSmemBytes = (size_t)12 * rows * keep;
+    e = closed_domain ? cudaLaunchKernelEx(&cfg, k_na_resident<true>, a, gpb, nvb, keep)
+                      : cudaLaunchKernelEx(&cfg, k_na_resident<false>, a, gpb, nvb, keep);
+  } else {
+    cfg.gridDim = dim3(nvb < g.blocks ? nvb : g.blocks);
+    cfg.blockDim = dim3(TPB);
+    e = closed_domain ? cudaLaunchKernelEx(&cfg, k_na_bicgstab<true>, a) : cudaLaunchKernelEx(&cfg, k_na_bicgstab<false>, a);
+  }
   if (e != cudaSuccess) return na_fail(VEBI_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
   if (iters_out || residual_out) {
     NaCtrl ctl;

@@ -24,89 +24,13 @@
 // Measured, ms per solve, k_bicgstab / this kernel: 1.7k rows x 60 iterations 2.39 / 1.21, 2.9k x
 // 75 2.48 / 1.36, 10k x 139 5.37 / 3.40, 20k x 363 14.9 / 12.1, 29k x 247 10.2 /
 // 9.8.
-#include "vebi_solver.cuh"
+#include "vebi_resident.cuh"
 
 namespace vebi {
 
 namespace {
 
-constexpr int RES_GROUP = 32;       // rows of a group (a warp's rows in the vector passes)
-constexpr int RES_VB = 8;           // groups of a virtual block (256 rows)
 constexpr int RES_MAX_ROWS = 256;   // rows of a block: four lanes a row fill it
-constexpr int RES_MAX_VB = 256;     // virtual blocks the shared table holds
-
-struct ResSh {
-  double vec[RES_MAX_ROWS];  // a product's results, by row of the block
-  double vb[2 * RES_MAX_VB]; // virtual-block sums
-  double v[2];
-  double rho, alpha, omega, beta, n2r0, n2s0, n2, mean;
-  int flag;
-};
-
-// the grid-wide sums of a and (NV = 2) b over all rows, a barrier among them: for thread 0 the
-// totals are in sh.v when this returns true
-template <int NV>
-__device__ __noinline__ bool res_sums(Scal* s, double a, double b, double* part, int gpb, int nvb, ResSh& sh) {
-  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
-  const int G = nvb * RES_VB, g0 = blockIdx.x * gpb;
-  if (w < gpb) {
-    double z;
-    if (NV == 1) {
-      z = a;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) z += __shfl_down_sync(0xffffffffu, z, o);
-    } else {  // both trees at once: lanes 0..15 carry a's, lanes 16..31 b's
-      const bool lo = lane < 16;
-      z = (lo ? a : b) + __shfl_xor_sync(0xffffffffu, lo ? b : a, 16);
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) z += __shfl_down_sync(0xffffffffu, z, o, 16);
-    }
-    if ((lane == 0 || (NV > 1 && lane == 16)) && g0 + w < G) part[(size_t)(lane >> 4) * G + g0 + w] = z;
-  }
-  __syncthreads();
-  int bad = 0;
-  if (t == 0) bad = barrier_arrive_wait(&s->bar_count, &s->error, SPIN_LIMIT) ? 0 : 1;
-  if (__syncthreads_or(bad)) return false;
-  auto vb_sum = [&](int q, int vb) {  // a virtual block's eight group sums in sequence
-    const double2* p = reinterpret_cast<const double2*>(part + (size_t)q * G + (size_t)vb * RES_VB);
-    double2 u[RES_VB / 2];
-#pragma unroll
-    for (int k = 0; k < RES_VB / 2; ++k) u[k] = __ldcg(p + k);
-    double z = plus_zero(u[0].x) + u[0].y;
-#pragma unroll
-    for (int k = 1; k < RES_VB / 2; ++k) {
-      z += u[k].x;
-      z += u[k].y;
-    }
-    return z;
-  };
-  const bool spread = nvb > 32;  // over all threads, else each summing lane does its own
-  if (spread) {
-    for (int e = t; e < NV * nvb; e += blockDim.x) sh.vb[e] = vb_sum(e / nvb, e % nvb);
-    __syncthreads();
-  }
-  if (w < NV) {  // warp q: lane l adds virtual blocks l, l+32, ... in order, then the lanes' tree
-    double z = 0.0;
-    if (lane < nvb) z = plus_zero(spread ? sh.vb[w * nvb + lane] : vb_sum(w, lane));
-#pragma unroll 1
-    for (int e = lane + 32; e < nvb; e += 32) z += sh.vb[w * nvb + e];
-    for (int o = 16; o > 0; o >>= 1)
-      if (o < nvb) z += __shfl_down_sync(0xffffffffu, z, o);
-    if (lane == 0) sh.v[w] = z;
-  }
-  if (NV > 1) __syncthreads();
-  return true;
-}
-
-// grid_reduce over the resident layout: post() runs on thread 0 with the sums in sh.v
-template <int NV, class Post>
-__device__ __forceinline__ bool res_reduce(Scal* s, double a, double b, double* part, int gpb, int nvb, ResSh& sh,
-                                           Post post) {
-  if (!res_sums<NV>(s, a, b, part, gpb, nvb, sh)) return false;
-  if (threadIdx.x == 0) post();
-  __syncthreads();
-  return true;
-}
 
 // One of a row's four lanes: lane q has spmv_row's accumulator q, which takes slots q, q+4, ... of
 // the whole quads of slots; lane 0 also takes the diagonal before them and the up to three slots
@@ -143,10 +67,12 @@ struct LaneRow {
 template <bool NONULL, int T_MAX, int KEEP>
 __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gpb, int nvb) {
   __shared__ ResSh sh;
+  __shared__ double vec[RES_MAX_ROWS];  // a product's results, by row of the block
   const int n = a.n, t = threadIdx.x;
   const int R = gpb * RES_GROUP, row0 = blockIdx.x * R;
   Scal* s = a.sc;
   if (state_failed(s)) return;
+  const GridBar bar{&s->bar_count, &s->error};
   const double rinv1 = 1.0 / (1.0 + 1.0e-15);
   const double small = NONULL ? 1.0e-6 : 4.0;  // open solver: the integer expression 10-6
   const double dn = (double)n;
@@ -197,9 +123,9 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
     }
     b += __shfl_xor_sync(0xffffffffu, b, 1);  // (b0 + b1) + (b2 + b3)
     b += __shfl_xor_sync(0xffffffffu, b, 2);
-    if (L.q == 0 && L.row >= 0) sh.vec[l] = b;
+    if (L.q == 0 && L.row >= 0) vec[l] = b;
     __syncthreads();
-    return mine ? sh.vec[t] : 0.0;
+    return mine ? vec[t] : 0.0;
   };
   double r = 0.0, rb = 0.0, v = 0.0, p = 0.0, x = 0.0, rinvM = rinv1;
   if (a.warm) {  // x0 = P of the previous step: r0 = B - A x0
@@ -216,14 +142,14 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
   }
   rb = r;
   if (!NONULL && mine) rinvM = 1.0 / (__ldg(a.diag + i) + 1.0e-15);
-  if (!res_reduce<1>(s, mine ? fma(r, r, 0.0) : 0.0, 0.0, part1, gpb, nvb, sh, [&]() { sh.rho = sh.v[0]; })) return;
+  if (!res_reduce<1>(bar, mine ? fma(r, r, 0.0) : 0.0, 0.0, part1, gpb, nvb, sh, [&]() { sh.rho = sh.v[0]; })) return;
   int iter = 1, warn = 0;
   bool done = false, at_s = false;
   while (iter <= a.itermax) {
     if (is_zero(sh.rho)) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
     if (mine) p = iter == 1 ? r : fma(sh.beta, fma(-sh.omega, v, p), r);
     if (NONULL) {
-      if (!res_reduce<1>(s, mine ? plus_zero(p) : 0.0, 0.0, part0, gpb, nvb, sh, [&]() { sh.mean = sh.v[0] / dn; }))
+      if (!res_reduce<1>(bar, mine ? plus_zero(p) : 0.0, 0.0, part0, gpb, nvb, sh, [&]() { sh.mean = sh.v[0] / dn; }))
         return;
       p = p - sh.mean;
     }
@@ -231,12 +157,12 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
     if (mine) a.pinv[i] = pinv;
     if (!grid_sync(s)) return;
     v = product(a.pinv);
-    if (!res_reduce<1>(s, mine ? fma(rb, v, 0.0) : 0.0, 0.0, part1, gpb, nvb, sh,
+    if (!res_reduce<1>(bar, mine ? fma(rb, v, 0.0) : 0.0, 0.0, part1, gpb, nvb, sh,
                        [&]() { sh.alpha = sh.rho / (sh.v[0] + 1.0e-15); }))
       return;
     const double alpha = sh.alpha;
     double sv = mine ? fma(-alpha, v, r) : 0.0;
-    if (!res_reduce<2>(s, mine ? fma(sv, sv, 0.0) : 0.0, mine ? plus_zero(sv) : 0.0, part0, gpb, nvb, sh, [&]() {
+    if (!res_reduce<2>(bar, mine ? fma(sv, sv, 0.0) : 0.0, mine ? plus_zero(sv) : 0.0, part0, gpb, nvb, sh, [&]() {
           sh.n2 = sh.v[0];
           if (iter == 1) sh.n2s0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
           sh.flag = sh.v[0] <= a.tol * a.tol * sh.n2s0;
@@ -253,13 +179,13 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
     if (mine) a.sinv[i] = sinv;
     if (!grid_sync(s)) return;
     const double tv = product(a.sinv);
-    if (!res_reduce<2>(s, mine ? fma(tv, sv, 0.0) : 0.0, mine ? fma(tv, tv, 0.0) : 0.0, part1, gpb, nvb, sh,
+    if (!res_reduce<2>(bar, mine ? fma(tv, sv, 0.0) : 0.0, mine ? fma(tv, tv, 0.0) : 0.0, part1, gpb, nvb, sh,
                        [&]() { sh.omega = sh.v[0] / (sh.v[1] + 1.0e-15); }))
       return;
     const double omega = sh.omega;
     x = fma(omega, sinv, fma(alpha, pinv, x));
     r = fma(-omega, tv, sv);
-    if (!res_reduce<2>(s, mine ? fma(r, r, 0.0) : 0.0, mine ? fma(rb, r, 0.0) : 0.0, part0, gpb, nvb, sh, [&]() {
+    if (!res_reduce<2>(bar, mine ? fma(r, r, 0.0) : 0.0, mine ? fma(rb, r, 0.0) : 0.0, part0, gpb, nvb, sh, [&]() {
           sh.n2 = sh.v[0];
           if (iter == 1) sh.n2r0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
           sh.flag = sh.v[0] <= a.tol * a.tol * sh.n2r0;
