@@ -227,6 +227,7 @@ static int allocate_all(Ctx& x) {
   A_(d.n_surf, cap); A_(d.inbin, cap);
   A_(d.irel, cap); A_(d.vrel, cap); A_(d.dP_mp, cap);
   A_(d.cellpart, cap); A_(d.cell_fill, cap); A_(d.ip, cap);
+  d.mirror_rows = d.cell_fill;
   A_(d.cell_cnt, (size_t)c.nct); A_(d.cell_start, (size_t)c.nct + 1);
   A_(d.scan_part, (size_t)c.nct / 1024 + 2);
   const size_t stages = (size_t)c.nb + 2;  // mirror stages: circles, patches, candidates

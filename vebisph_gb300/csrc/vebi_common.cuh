@@ -74,6 +74,7 @@ struct Scal {
   int warnings;
   int error;
   int n_cand;                        // particles in cand
+  int n_mirror_rows;                 // rows listed for k_ppe_mirror_rows
   int n_end, n_node;                 // mirrors and particles listed for the corners (mir_list)
   unsigned int bar_count;            // grid barrier of the PPE solvers (vebi_solver.cuh)
   int refine_iters;
@@ -131,6 +132,7 @@ struct Dev {
   int *scan_part;
   // ordered select scratch
   int* sel_blk;
+  int* mirror_rows;                          // cell_fill's storage, free once the cells are filled
   unsigned* sel_bits;                        // [plane][particle / 32]
   int* mir_list;                             // corners: mirrors past a wall's end, particles by a node
   int* cand;                                 // with circles: particles near a boundary or circle, ascending

@@ -55,13 +55,17 @@ __global__ void k_ppe_mean(Consts c, Dev d, int nblk) {
   double s = 0.0;
   for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += d.partials[b];
   s = block_sum<TPB>(s, sh);
-  if (threadIdx.x == 0) d.s->rhs_mean = (c.open_domain == 0) ? s / (double)c.npfb : 0.0;
+  if (threadIdx.x == 0) {
+    d.s->rhs_mean = (c.open_domain == 0) ? s / (double)c.npfb : 0.0;
+    d.s->n_mirror_rows = 0;
+  }
 }
 
 // ---------------------------------------------------------------------- assembly
 // Rows without a mirror neighbour (all but a thin layer along the boundaries) hold distinct
 // columns, so one pass writes each slot once with the same value (0 + temp) the general path
-// accumulates; the first mirror neighbour sends the row to the general path, which starts over.
+// accumulates; the first mirror neighbour puts the row on the list of k_ppe_mirror_rows, which
+// starts it over.
 // The mixed step (wL32 given) also writes the FP32 off-diagonal values and the FP64 row sums
 // diag + sum_k A_ik, in slot order, that its difference-form SpMV reads.  Its solvers read no
 // FP64 off-diagonal value, so a mixed row without mirrors, smoothing or a free-surface
@@ -97,7 +101,7 @@ __global__ void k_ppe_assemble(Consts c, Dev d, const float* __restrict__ wL32, 
         if (k0 + u >= cnt) break;
         const int j = j4[u];
         const float w = w4[u];
-        any_mirror |= j >= c.npfb;  // such a row starts over in the general path below
+        any_mirror |= j >= c.npfb;  // such a row is k_ppe_mirror_rows's
         const float t = hs + w, bp = t - hs;
         hc += (hs - (t - bp)) + (w - bp);
         hs = t;
@@ -125,7 +129,7 @@ __global__ void k_ppe_assemble(Consts c, Dev d, const float* __restrict__ wL32, 
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (k0 + u >= cnt) break;
-        any_mirror |= j4[u] >= c.npfb;  // such a row starts over in the general path below
+        any_mirror |= j4[u] >= c.npfb;  // such a row is k_ppe_mirror_rows's
         Adiag = Adiag - t4[u];
         d.ppe_col[ELL(k0 + u, i)] = j4[u];
         d.ppe_val[ELL(k0 + u, i)] = plus_zero(t4[u]);
@@ -133,33 +137,8 @@ __global__ void k_ppe_assemble(Consts c, Dev d, const float* __restrict__ wL32, 
     }
   }
   if (any_mirror) {
-    for (int k = 0; k < cnt; ++k) {
-      int j = d.ij_link[ELL(k, i)];
-      d.ppe_col[ELL(k, i)] = j >= c.npfb ? d.irel[j] : j;
-      d.ppe_val[ELL(k, i)] = 0.0;
-    }
-    Adiag = 0.0;
-    for (int k = 0; k < cnt; ++k) {
-      int j = d.ij_link[ELL(k, i)];
-      // the mixed step assembles in FP64 from its FP32 Morris weights
-      double temp = wL32 ? -(double)wL32[ELL(k, i)] : -d.wL[ELL(k, i)];
-      Adiag = Adiag - temp;
-      int colk = j;
-      bool self = false;
-      if (j >= c.npfb) {
-        colk = d.irel[j];
-        if (colk == i) self = true;
-        B = B - d.dP_mp[j] * temp;
-      }
-      if (self) {
-        Adiag = Adiag + temp;
-      } else {
-        int nt = k;  // last slot holding this column
-        for (int kk = cnt - 1; kk >= 0; --kk)
-          if (d.ppe_col[ELL(kk, i)] == colk) { nt = kk; break; }
-        d.ppe_val[ELL(nt, i)] = d.ppe_val[ELL(nt, i)] + temp;
-      }
-    }
+    d.mirror_rows[atomicAdd(&d.s->n_mirror_rows, 1)] = i;
+    return;
   }
   if (d.n_surf[i] != 0) Adiag = 1.0e30;
   const double diag = 0.0 + Adiag;
@@ -179,6 +158,102 @@ __global__ void k_ppe_assemble(Consts c, Dev d, const float* __restrict__ wL32, 
     }
     d.rowsum[i] = rs;
     if (c.open_domain == 1) d.bM[i] = 1.0 / (diag + 1.0e-15);
+  }
+}
+
+// Rows with mirror neighbours, a warp per row and MR_ROWS rows per block.  A mirror's term goes to its
+// parent's column (the last slot that holds it, in slot order) or, if the row is the parent, out
+// of the diagonal again, and its dP_mp to the right-hand side.  Each lane finds the slots that
+// share its slot's column by integer compares in shared memory and adds their terms; the row's
+// three chains (diagonal, right-hand side, row sum) run a thread per row, as the FP64 pipe takes
+// as long for one lane as for all.
+// What bounds it: latency, ~3 dependent loads and ~100 dependent FP64 adds.  By one thread per row
+// in k_ppe_assemble, searching the columns in memory, these few rows were most of the assembly: the
+// stage took 0.21 / 0.22 / 0.43 / 1.73 ms at 1.7k / 20k / 250k / 4M particles, 0.08 / 0.05 / 0.15 /
+// 1.38 with this kernel (of it 23 us at 20k, 0.28 ms at 4M).
+constexpr int MR_ROWS = TPB / 32, MR_SLOTS = 96;  // vebi_create accepts nplink <= 96
+__global__ void __launch_bounds__(TPB) k_ppe_mirror_rows(Consts c, Dev d, const float* __restrict__ wL32) {
+  __shared__ int col[MR_ROWS][MR_SLOTS];            // bit 31: the term leaves the diagonal (own mirror)
+  __shared__ double term[MR_ROWS][MR_SLOTS], val[MR_ROWS][MR_SLOTS], dp[MR_ROWS][MR_SLOTS];
+  __shared__ unsigned mir[MR_ROWS][MR_SLOTS / 32];  // slots with a mirror
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = d.s->n_mirror_rows;
+  const double mean = c.open_domain == 0 ? d.s->rhs_mean : 0.0;
+  for (int base = blockIdx.x * MR_ROWS; base < n; base += gridDim.x * MR_ROWS) {
+    if (base + w < n) {
+      const int i = d.mirror_rows[base + w], cnt = d.ij_count[i];
+      const bool smooth = c.open_domain == 1 && d.n_surf[i] != 1 && d.ppe_smooth[i] != 1.0;
+#pragma unroll
+      for (int q = 0; q < MR_SLOTS / 32; ++q) {
+        const int k = q * 32 + lane;
+        bool mirror = false;
+        if (k < cnt) {
+          const int j = d.ij_link[ELL(k, i)];
+          // the mixed step assembles in FP64 from its FP32 Morris weights
+          const double t = wL32 ? -(double)wL32[ELL(k, i)] : -d.wL[ELL(k, i)];
+          mirror = j >= c.npfb;
+          const int ck = mirror ? d.irel[j] : j;
+          col[w][k] = mirror && ck == i ? (int)(0x80000000u | (unsigned)ck) : ck;
+          term[w][k] = t;
+          dp[w][k] = mirror ? d.dP_mp[j] * t : 0.0;
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, mirror);
+        if (lane == 0) mir[w][q] = b;
+      }
+      __syncwarp();
+      const double ps = smooth ? d.ppe_smooth[i] : 1.0;
+      for (int k = lane; k < cnt; k += 32) {
+        const int ck = col[w][k];
+        unsigned m[MR_SLOTS / 32];
+        int last = 0;
+#pragma unroll
+        for (int q = 0; q < MR_SLOTS / 32; ++q) {
+          m[q] = 0;
+          for (int u = 0; u < 32 && q * 32 + u < cnt; ++u) m[q] |= (col[w][q * 32 + u] == ck ? 1u : 0u) << u;
+          if (m[q]) last = q * 32 + 31 - __clz(m[q]);
+        }
+        double v = 0.0;
+        if (last == k && ck >= 0) {
+#pragma unroll
+          for (int q = 0; q < MR_SLOTS / 32; ++q)
+            for (unsigned b = m[q]; b; b &= b - 1) v += term[w][q * 32 + __ffs(b) - 1];
+        }
+        if (smooth) v *= ps;
+        val[w][k] = v;
+        d.ppe_col[ELL(k, i)] = ck & 0x7fffffff;
+        d.ppe_val[ELL(k, i)] = v;
+        if (wL32) d.ppe_val32[ELL(k, i)] = (float)v;
+      }
+    }
+    __syncthreads();
+    if (w < 2 && lane < MR_ROWS && base + lane < n) {
+      const int i = d.mirror_rows[base + lane], cnt = d.ij_count[i];
+      if (w == 0) {
+        double Adiag = 0.0;
+        for (int k = 0; k < cnt; ++k) {
+          const double t = term[lane][k];
+          Adiag = Adiag - t;
+          if (col[lane][k] < 0) Adiag = Adiag + t;
+        }
+        if (d.n_surf[i] != 0) Adiag = 1.0e30;
+        const double diag = 0.0 + Adiag;
+        d.ppe_diag[i] = diag;
+        if (wL32) {
+          double rs = diag;
+          for (int k = 0; k < cnt; ++k) rs += val[lane][k];
+          d.rowsum[i] = rs;
+          if (c.open_domain == 1) d.bM[i] = 1.0 / (diag + 1.0e-15);
+        }
+      } else {
+        double B = d.ppe_B[i];
+        if (c.open_domain == 0) B = B - mean;
+        for (int q = 0; q < MR_SLOTS / 32; ++q)
+          for (unsigned b = mir[lane][q]; b; b &= b - 1) B = B - dp[lane][q * 32 + __ffs(b) - 1];
+        if (c.open_domain == 1 && d.n_surf[i] != 1 && d.ppe_smooth[i] != 1.0) B = B * d.ppe_smooth[i];
+        d.ppe_B[i] = B;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -399,6 +474,10 @@ void launch_ppe(Ctx& x) {
   VEBI_LAUNCH(x, k_ppe_mean, 1, TPB, c, x.d, g);
   VEBI_LAUNCH(x, k_ppe_assemble, g, TPB, c, x.d, mixed ? (const float*)x.d.wL32 : (const float*)nullptr,
               x.rep_p != nullptr ? 1 : 0);
+  // the list's length is on the device: enough blocks for a small domain's, striding over a large one's
+  const int mr = (c.npfb + MR_ROWS - 1) / MR_ROWS;
+  VEBI_LAUNCH(x, k_ppe_mirror_rows, mr < 6 * x.nsm ? mr : 6 * x.nsm, TPB, c, x.d,
+              mixed ? (const float*)x.d.wL32 : (const float*)nullptr);
   stage_mark(x, 10);
   if (x.rep_p) {  // a recorded step recomputed by the adjoint: its solution is known
     cudaMemcpyAsync(x.d.p, x.rep_p, sizeof(double) * (size_t)c.npfb, cudaMemcpyDeviceToDevice, x.st);
