@@ -175,6 +175,117 @@ __global__ void k_mg_level1(Consts c, Dev d, MgLevel L, const int* __restrict__ 
   if (!ok) d.s->mg_fail = 1;
 }
 
+// A coarse row by a warp.  Lane m keeps the m-th column in order of first appearance and its sum,
+// the last lane the row's own column (the diagonal).  The entries come in their order, up to one a
+// lane: every lane marks its column's, a column without a lane takes the next one, then the lanes
+// add theirs, so each sum runs in the order of the entries, as a thread's searched table adds them.
+// What bounds it: ~10 instructions per entry.  A thread per row waits for each entry's loads and
+// table search in turn, ~130 us for a level-1 row however few rows there are (mg_setup has both).
+struct WarpRow {
+  int key, m;
+  double sum;
+  bool ok;
+  __device__ __forceinline__ explicit WarpRow(int own)
+      : key((threadIdx.x & 31) == 31 ? own : -1), m(0), sum(0.0), ok(true) {}
+  __device__ __forceinline__ void add(bool in, int a, double v) {
+    const int lane = threadIdx.x & 31;
+    unsigned mine = 0;
+    for (unsigned todo = __ballot_sync(0xffffffffu, in); todo; todo &= todo - 1) {
+      const int u = __ffs(todo) - 1, au = __shfl_sync(0xffffffffu, a, u);
+      if (!__ballot_sync(0xffffffffu, key == au)) {
+        if (m == MG_SLOTS) { ok = false; continue; }
+        if (lane == m) key = au;
+        ++m;
+      }
+      if (key == au) mine |= 1u << u;
+    }
+    while (__any_sync(0xffffffffu, mine != 0)) {
+      const double w = __shfl_sync(0xffffffffu, v, mine ? __ffs(mine) - 1 : lane);
+      if (mine) sum += w;
+      mine &= mine - 1;
+    }
+  }
+  __device__ __forceinline__ void store(const MgLevel& L, int row) const {
+    const int lane = threadIdx.x & 31;
+    if (lane < m) {
+      L.col[(size_t)lane * L.n + row] = key;
+      L.val[(size_t)lane * L.n + row] = sum;
+    }
+    if (lane == 0) L.cnt[row] = m;
+    if (lane == 31) {
+      L.diag[row] = sum;
+      L.dinv[row] = sum != 0.0 ? 1.0 / sum : 0.0;
+    }
+  }
+};
+static_assert(MG_SLOTS < 32 && MG_ROW_SLOTS == 16, "a lane per column; two particles' pairs at a time");
+
+__global__ void __launch_bounds__(TPB) k_mg_level1_warp(Consts c, Dev d, MgLevel L, const int* __restrict__ ragg,
+                                                        const double* __restrict__ rval,
+                                                        const int* __restrict__ rcnt) {
+  const int cc = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (cc >= L.n) return;
+  WarpRow R(cc);
+  const int s0 = d.cell_start[cc], ne = d.cell_cnt[cc];
+  for (int q0 = 0; q0 < ne; q0 += 32) {
+    int id = -1, pairs = 0;  // of particle q0 + lane; mirrors follow the particles in a sorted cell list
+    if (q0 + lane < ne) {
+      id = d.ip[s0 + q0 + lane];
+      if (id < c.npfb) pairs = rcnt[id];
+    }
+    const int np = __popc(__ballot_sync(0xffffffffu, q0 + lane < ne && id < c.npfb));
+    const int t = lane & 15;
+    auto fetch = [&](int q, int& a, double& v) {  // pair t of particles q and q + 1
+      const int from = q + (lane >> 4);
+      const int i = __shfl_sync(0xffffffffu, id, from & 31), n = __shfl_sync(0xffffffffu, pairs, from & 31);
+      const bool in = from < np && t < n;
+      a = in ? ragg[(size_t)t * c.npfb + i] : -1;
+      v = in ? rval[(size_t)t * c.npfb + i] : 0.0;
+      return in;
+    };
+    int a, a_next;
+    double v, v_next;
+    bool in = fetch(0, a, v);
+    for (int q = 0; q < np; q += 2) {
+      const bool in_next = fetch(q + 2, a_next, v_next);
+      R.add(in, a, v);
+      in = in_next;
+      a = a_next;
+      v = v_next;
+    }
+    if (np < 32) break;
+  }
+  R.store(L, cc);
+  if (!R.ok && lane == 0) d.s->mg_fail = 1;
+}
+
+__global__ void __launch_bounds__(TPB) k_mg_coarsen_warp(MgLevel F, MgLevel G, Scal* s) {
+  const int C = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (C >= G.n) return;
+  const int X = C % G.gx, Y = C / G.gx;
+  WarpRow R(C);
+  int a[4];
+  double v[4];
+  bool in[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {  // a child's diagonal, then its slots
+    const int fx = 2 * X + (q & 1), fy = 2 * Y + (q >> 1), f = fx + fy * F.gx;
+    in[q] = fx < F.gx && fy < F.gy && lane <= F.cnt[f];
+    a[q] = -1;
+    v[q] = 0.0;
+    if (in[q]) {
+      const size_t e = (size_t)(lane - 1) * F.n + f;
+      const int cf = lane ? F.col[e] : f;
+      a[q] = (cf % F.gx) / 2 + ((cf / F.gx) / 2) * G.gx;
+      v[q] = lane ? F.val[e] : F.diag[f];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) R.add(in[q], a[q], v[q]);
+  R.store(G, C);
+  if (!R.ok && lane == 0) s->mg_fail = 1;
+}
+
 // level l+1 from level l: one thread per coarse row sums its (up to) 2x2 child rows
 __global__ void k_mg_coarsen(MgLevel F, MgLevel G, Scal* s) {
   const int C = blockIdx.x * blockDim.x + threadIdx.x;
@@ -204,71 +315,78 @@ __global__ void k_mg_coarsen(MgLevel F, MgLevel G, Scal* s) {
 }
 
 // The coarsest level's dense inverse, for a direct coarse solve in the V-cycle: Gauss-Jordan
-// with partial pivoting in one 32 x 32 block, thread (ty, tx) owning row ty and columns tx and
-// tx + 32 of [M | I] (at most MG_COARSEST = 32 rows).  A closed domain's coarse matrix is
-// singular (its rows sum to zero: the constant is in its null space), so it is inverted as
-// M + alpha 1 1^T with alpha = mean |diag| / n, which moves that eigenvalue to mean |diag| and
-// leaves the mean-free solution of M x = b unchanged.  *ok = 0 (a zero pivot, or a level too
-// large) makes the V-cycle fall back to Jacobi sweeps.
+// with partial pivoting in one 32 x 32 block, a warp per row of [M | I] (at most MG_COARSEST = 32
+// rows).  A step changes n of the 2n columns: those of M right of the pivot, and those of I that
+// belong to the pivots so far (the pivot row's other entries of I are still zero); a lane takes one.
+// (At 27 to 32 rows 32 us; all 2n columns, five block barriers a step and FP64 compares took 83.)
+// A closed domain's coarse matrix is singular (its rows sum to zero: the constant is in its null
+// space), so it is inverted as M + alpha 1 1^T with alpha = mean |diag| / n, which moves that
+// eigenvalue to mean |diag| and leaves the mean-free solution of M x = b unchanged.  *ok = 0 (a zero
+// pivot, or a level too large) makes the V-cycle fall back to Jacobi sweeps.
 __global__ void __launch_bounds__(1024) k_mg_coarse_inverse(MgLevel K, double* inv, int* ok, int closed) {
   __shared__ double M[MG_COARSEST][2 * MG_COARSEST + 1];
-  __shared__ double fcol[MG_COARSEST];
-  __shared__ int piv_row;
+  __shared__ int orig[MG_COARSEST];  // the row of M that now is row r
+  __shared__ int good;
   __shared__ double alpha_s;
-  const int n = K.n, tx = threadIdx.x, ty = threadIdx.y;
+  const int n = K.n, tx = threadIdx.x, r = threadIdx.y;
   if (n > MG_COARSEST || n < 1) {
-    if (tx == 0 && ty == 0) *ok = 0;
+    if (tx == 0 && r == 0) *ok = 0;
     return;
   }
-  if (ty == 0) {  // alpha from the warp of row-owners
+  if (r == 0) {  // alpha from the warp of row-owners
     double ad = tx < n ? fabs(K.diag[tx]) : 0.0;
     for (int o = 16; o > 0; o >>= 1) ad += __shfl_xor_sync(0xffffffffu, ad, o);
     if (tx == 0) alpha_s = closed ? ad / ((double)n * (double)n) : 0.0;
+    orig[tx] = tx;
+    if (tx == 0) good = 1;
   }
   __syncthreads();
-  const int r = ty;
-  if (r < n)
+  if (r < n) {
     for (int c = tx; c < 2 * n; c += 32) M[r][c] = c < n ? alpha_s : (c - n == r ? 1.0 : 0.0);
-  __syncthreads();
-  if (r < n && tx == 0) {
-    M[r][r] += K.diag[r];
-    const int m = K.cnt[r];
-    for (int t = 0; t < m; ++t) M[r][K.col[(size_t)t * K.n + r]] += K.val[(size_t)t * K.n + r];
+    __syncwarp();
+    const int m = K.cnt[r];  // distinct columns, none of them r
+    if (tx == 31) M[r][r] += K.diag[r];
+    if (tx < m) M[r][K.col[(size_t)tx * K.n + r]] += K.val[(size_t)tx * K.n + r];
   }
   __syncthreads();
-  bool good = true;
   for (int k = 0; k < n; ++k) {
-    if (ty == 0) {  // argmax of |M[i][k]| over i >= k, ties to the lower row
-      double v = (tx >= k && tx < n) ? fabs(M[tx][k]) : -1.0;
+    auto column = [&]() { return tx < n - 1 - k ? k + 1 + tx : n + orig[tx - (n - 1 - k)]; };
+    if (r == 0) {
+      // argmax of |M[i][k]| over i >= k, ties to the lower row; ordered as the bits are
+      long long v = -1;
+      if (tx >= k && tx < n) {
+        const double x = fabs(M[tx][k]);
+        v = x == x ? __double_as_longlong(x) : 0;
+      }
       int p = tx;
+#pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
-        const double v2 = __shfl_xor_sync(0xffffffffu, v, o);
+        const long long v2 = __shfl_xor_sync(0xffffffffu, v, o);
         const int p2 = __shfl_xor_sync(0xffffffffu, p, o);
         if (v2 > v || (v2 == v && p2 < p)) { v = v2; p = p2; }
       }
-      if (tx == 0) piv_row = v > 0.0 ? p : -1;
+      if (v <= 0) {
+        if (tx == 0) good = 0;
+      } else {
+        if (p != k) {
+          for (int c = tx; c < 2 * n; c += 32) { const double t = M[k][c]; M[k][c] = M[p][c]; M[p][c] = t; }
+          if (tx == 0) { const int t = orig[k]; orig[k] = orig[p]; orig[p] = t; }
+        }
+        __syncwarp();
+        if (tx < n) M[k][column()] /= M[k][k];
+      }
     }
     __syncthreads();
-    const int p = piv_row;
-    if (p < 0) { good = false; break; }
-    if (ty == 0 && p != k)
-      for (int c = tx; c < 2 * n; c += 32) { const double t = M[k][c]; M[k][c] = M[p][c]; M[p][c] = t; }
-    __syncthreads();
-    const double piv = M[k][k];
-    __syncthreads();
-    if (ty == 0)
-      for (int c = tx; c < 2 * n; c += 32) M[k][c] /= piv;
-    if (tx == 0 && r < n) fcol[r] = M[r][k];
-    __syncthreads();
-    if (r < n && r != k) {
-      const double f = fcol[r];
-      for (int c = tx; c < 2 * n; c += 32) M[r][c] = fma(-f, M[k][c], M[r][c]);
+    if (!good) break;
+    if (r < n && r != k && tx < n) {
+      const int c = column();
+      M[r][c] = fma(-M[r][k], M[k][c], M[r][c]);
     }
     __syncthreads();
   }
   if (good && r < n)
     for (int c = tx; c < n; c += 32) inv[(size_t)r * n + c] = M[r][n + c];
-  if (tx == 0 && ty == 0) *ok = good ? 1 : 0;
+  if (tx == 0 && r == 0) *ok = good;
 }
 
 // The row's A P g in direct form, vown g_own + sum_c (A P)_ic g_c, from its direction table:
@@ -1209,9 +1327,17 @@ static int mg_setup(Ctx& x) {
   const float* v32 = x.precision == VEBI_PREC_MIXED ? x.d.ppe_val32 : nullptr;
   VEBI_LAUNCH(x, k_mg_rows, grid_for(c.npfb), TPB, c, x.d, v32, x.mg_ragg, x.mg_rval, x.mg_rcnt, x.mg_rv9,
               x.mg_rx);
-  VEBI_LAUNCH(x, k_mg_level1, grid_for(x.mg[0].n), TPB, c, x.d, x.mg[0], x.mg_ragg, x.mg_rval, x.mg_rcnt);
-  for (int l = 0; l + 1 < nl; ++l)
-    VEBI_LAUNCH(x, k_mg_coarsen, grid_for(x.mg[l + 1].n), TPB, x.mg[l], x.mg[l + 1], x.d.s);
+  // A warp per row until the GPU is full of them.  Measured, a thread / a warp per row: level 1 of
+  // 1.8k / 22k / 90k / 360k rows 128 / 137 / 139 / 400 and 19 / 58 / 196 / 743 us; a coarser level of
+  // 500 / 22k / 90k rows 34 / 33 / 42 and 11 / 31 / 101 us.
+  const auto level1 = x.mg[0].n <= 65536 ? k_mg_level1_warp : k_mg_level1;
+  VEBI_LAUNCH(x, level1, grid_for(level1 == k_mg_level1_warp ? 32ll * x.mg[0].n : x.mg[0].n), TPB, c, x.d, x.mg[0],
+              x.mg_ragg, x.mg_rval, x.mg_rcnt);
+  for (int l = 0; l + 1 < nl; ++l) {
+    const auto coarsen = x.mg[l + 1].n <= 16384 ? k_mg_coarsen_warp : k_mg_coarsen;
+    VEBI_LAUNCH(x, coarsen, grid_for(coarsen == k_mg_coarsen_warp ? 32ll * x.mg[l + 1].n : x.mg[l + 1].n), TPB, x.mg[l],
+                x.mg[l + 1], x.d.s);
+  }
   VEBI_LAUNCH(x, k_mg_coarse_inverse, 1, dim3(32, 32), x.mg[nl - 1], x.mg_kinv, x.mg_kinv_ok,
               c.open_domain == 0 ? 1 : 0);
   int tail = nl - 1;
