@@ -66,3 +66,18 @@ def test_matrix_of_rows_with_mirrors(built, name):
         assert rep[nm][0] <= tol, (nm, rep[nm])
     gpu.close()
     ref.close()
+
+
+@pytest.mark.parametrize("const_mod", [1, 2])
+@pytest.mark.parametrize("name", ["cylinder", "two_circles"])
+def test_force_on_circles(built, name, const_mod):
+    """k_circle_terms, Newtonian and viscoelastic: within the pressure's tolerance of the oracle."""
+    from oracle.oracle import OracleSolver
+    from vebisph_gb300.solver import StepSolver
+    case = CASES[name]()
+    case.const_mod = const_mod
+    gpu, ref = StepSolver(case), OracleSolver(case)
+    fg, fo = np.array(gpu.step()["circle_force"]), np.array(ref.step()["circle_force"])
+    assert np.abs(fo).max() > 0 and np.abs(fg - fo).max() <= 1e-5 * np.abs(fo).max(), (fg, fo)
+    gpu.close()
+    ref.close()

@@ -234,6 +234,7 @@ static int allocate_all(Ctx& x) {
   A_(d.sel_blk, stages * (n > 200000 ? n / 1024 + 1 : n / 256 + 1) + 1);
   A_(d.sel_bits, (stages + c.ncirc) * ((n + 31) / 32)); A_(d.mir_list, 2 * MIR_LIST);
   A_(d.cand, n);
+  if (c.ncirc > 0) A_(d.circle_f, 2 * n);
   A_(d.pk, cap); A_(d.pko, cap);
   A_(d.ij_count, n); A_(d.ij_link, E);
   A_(d.wGx, E); A_(d.wGy, E); A_(d.wL, E);

@@ -132,6 +132,7 @@ struct Dev {
   int *scan_part;
   // ordered select scratch
   int* sel_blk;
+  double* circle_f;                          // force on the circles by candidate, x and y
   int* mirror_rows;                          // cell_fill's storage, free once the cells are filled
   unsigned* sel_bits;                        // [plane][particle / 32]
   int* mir_list;                             // corners: mirrors past a wall's end, particles by a node

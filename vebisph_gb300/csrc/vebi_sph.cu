@@ -655,49 +655,79 @@ __global__ void k_secondary_final(Consts c, Dev d, int nblk) {
 // A circle mirror lies at radius 2R - rad of a source at rad (inside the support band), so a
 // particle that has one as a neighbour (distance <= sup) is within sup of the circle: the
 // mirror stages' candidate list (every particle within sup plus a margin of a boundary, in
-// ascending index) holds all of them, and the kernel walks that list alone.
+// ascending index) holds all of them, and the kernels walk that list alone.
+// k_circle_terms: a warp per candidate, a lane per pair; then four lanes add the mirrors' terms in
+// slot order, one lane for each of the viscous and pressure sums.  k_circle_force adds the candidates.
+// Measured, both: 19 us at 20k particles; by one thread per candidate, pair after pair, 137.
 constexpr int CF_BLOCKS = 256;
 
 template <class W>
-__global__ void k_circle_force(Consts c, Dev d, const W* __restrict__ wgx, const W* __restrict__ wgy,
-                               const W* __restrict__ wl_, const W* __restrict__ k11, const W* __restrict__ k21,
-                               const W* __restrict__ k12, const W* __restrict__ k22) {
-  __shared__ double sh[TPB / 32 + 1];
+__global__ void __launch_bounds__(TPB) k_circle_terms(Consts c, Dev d, const W* __restrict__ wgx, const W* __restrict__ wgy,
+                                                      const W* __restrict__ wl_, const W* __restrict__ k11,
+                                                      const W* __restrict__ k21, const W* __restrict__ k12,
+                                                      const W* __restrict__ k22) {
+  __shared__ double first[TPB / 32][4][32], second[TPB / 32][4][32];  // terms of the sums s1, s2, a, b
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ncand = d.s->n_cand;
-  double fx = 0.0, fy = 0.0;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < ncand; q += gridDim.x * blockDim.x) {
+  const bool ve = c.const_mod != 1;
+  const double cs = c.coeff_solvent, cp = c.coeff_polymeric;
+  for (int q = blockIdx.x * (TPB / 32) + w; q < ncand; q += gridDim.x * (TPB / 32)) {
     const int i = d.cand[q];
-    if (i < c.nbS || i >= c.npfb || d.inbin[i]) continue;
-    const bool ve = c.const_mod != 1;
+    if (i < c.nbS || i >= c.npfb || d.inbin[i]) {
+      if (lane < 2) d.circle_f[2 * (size_t)q + lane] = 0.0;
+      continue;
+    }
     const double ui = d.u0x[i], vi = d.u0y[i], pi_ = d.p[i];
     const double K11 = (double)k11[i], K21 = (double)k21[i], K12 = (double)k12[i], K22 = (double)k22[i];
     double Ti11 = 0, Ti21 = 0, Ti12 = 0, Ti22 = 0;
     if (ve) { Ti11 = d.tau[0][i]; Ti21 = d.tau[1][i]; Ti12 = d.tau[2][i]; Ti22 = d.tau[3][i]; }
-    const double cs = c.coeff_solvent, cp = c.coeff_polymeric;
-    double s1 = 0, s2 = 0, a = 0, b = 0;
+    double sum = 0.0;  // of lanes 0..3
     const int cnt = d.ij_count[i];
-    for (int k = 0; k < cnt; ++k) {
-      int j = d.ij_link[ELL(k, i)];
-      if (j < c.npfb || d.vrel[j] <= 999) continue;
-      double w1 = (double)wgx[ELL(k, i)], w2 = (double)wgy[ELL(k, i)], wl = (double)wl_[ELL(k, i)];
-      double u1 = ui - d.ux[j], u2 = vi - d.uy[j];
-      if (ve) {
-        double T11 = d.tau[0][j] - Ti11, T21 = d.tau[1][j] - Ti21;
-        double T12 = d.tau[2][j] - Ti12, T22 = d.tau[3][j] - Ti22;
-        double kw1 = K11 * w1 + K12 * w2, kw2 = K21 * w1 + K22 * w2;
-        s1 = s1 + cp * (T11 * kw1 + T12 * kw2) + cs * u1 * wl;
-        s2 = s2 + cp * (T21 * kw1 + T22 * kw2) + cs * u2 * wl;
-      } else {
-        s1 = s1 + cs * u1 * wl;
-        s2 = s2 + cs * u2 * wl;
+    for (int k0 = 0; k0 < cnt; k0 += 32) {
+      const int k = k0 + lane, j = k < cnt ? d.ij_link[ELL(k, i)] : -1;
+      const bool hit = j >= c.npfb && d.vrel[j] > 999;
+      unsigned hits = __ballot_sync(0xffffffffu, hit);
+      if (!hits) continue;
+      if (hit) {
+        const double w1 = (double)wgx[ELL(k, i)], w2 = (double)wgy[ELL(k, i)], wl = (double)wl_[ELL(k, i)];
+        const double u1 = ui - d.ux[j], u2 = vi - d.uy[j], temp = d.p[j] - pi_;
+        if (ve) {
+          const double T11 = d.tau[0][j] - Ti11, T21 = d.tau[1][j] - Ti21;
+          const double T12 = d.tau[2][j] - Ti12, T22 = d.tau[3][j] - Ti22;
+          const double kw1 = K11 * w1 + K12 * w2, kw2 = K21 * w1 + K22 * w2;
+          first[w][0][lane] = cp * (T11 * kw1 + T12 * kw2);
+          first[w][1][lane] = cp * (T21 * kw1 + T22 * kw2);
+        }
+        second[w][0][lane] = cs * u1 * wl;
+        second[w][1][lane] = cs * u2 * wl;
+        second[w][2][lane] = temp * w1;
+        second[w][3][lane] = temp * w2;
       }
-      double temp = d.p[j] - pi_;
-      a = a + temp * w1;
-      b = b + temp * w2;
+      __syncwarp();
+      if (lane < 4)
+        for (; hits; hits &= hits - 1) {
+          const int u = __ffs(hits) - 1;
+          if (ve && lane < 2) sum = sum + first[w][lane][u];
+          sum = sum + second[w][lane][u];
+        }
+      __syncwarp();
     }
-    const double gx = K11 * a + K12 * b, gy = K21 * a + K22 * b;
-    fx += c.dv * (gx - s1);
-    fy += c.dv * (gy - s2);
+    const double s = __shfl_sync(0xffffffffu, sum, lane & 1);
+    const double a = __shfl_sync(0xffffffffu, sum, 2), b = __shfl_sync(0xffffffffu, sum, 3);
+    if (lane < 2) {
+      const double g = lane == 0 ? K11 * a + K12 * b : K21 * a + K22 * b;
+      d.circle_f[2 * (size_t)q + lane] = c.dv * (g - s);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(TPB) k_circle_force(Dev d) {
+  __shared__ double sh[TPB / 32 + 1];
+  const int ncand = d.s->n_cand;
+  double fx = 0.0, fy = 0.0;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < ncand; q += gridDim.x * blockDim.x) {
+    fx += d.circle_f[2 * (size_t)q];
+    fy += d.circle_f[2 * (size_t)q + 1];
   }
   double bx = block_sum<TPB>(fx, sh);
   double by = block_sum<TPB>(fy, sh);
@@ -804,12 +834,14 @@ void launch_final(Ctx& x, int secondary) {
     VEBI_LAUNCH(x, k_advect_final, g, TPB, c, x.d);
   }
   if (c.ncirc > 0) {
+    const int cb = 6 * x.nsm < (c.npfb + 7) / 8 ? 6 * x.nsm : (c.npfb + 7) / 8;
     if (mixed)
-      VEBI_LAUNCH(x, k_circle_force<float>, CF_BLOCKS, TPB, c, x.d, x.d.wGx32, x.d.wGy32, x.d.wL32, x.d.kgcm32[0],
+      VEBI_LAUNCH(x, k_circle_terms<float>, cb, TPB, c, x.d, x.d.wGx32, x.d.wGy32, x.d.wL32, x.d.kgcm32[0],
                   x.d.kgcm32[1], x.d.kgcm32[2], x.d.kgcm32[3]);
     else
-      VEBI_LAUNCH(x, k_circle_force<double>, CF_BLOCKS, TPB, c, x.d, x.d.wGx, x.d.wGy, x.d.wL, x.d.kgcm[0], x.d.kgcm[1],
+      VEBI_LAUNCH(x, k_circle_terms<double>, cb, TPB, c, x.d, x.d.wGx, x.d.wGy, x.d.wL, x.d.kgcm[0], x.d.kgcm[1],
                   x.d.kgcm[2], x.d.kgcm[3]);
+    VEBI_LAUNCH(x, k_circle_force, CF_BLOCKS, TPB, x.d);
     VEBI_LAUNCH(x, k_circle_force_final, 1, TPB, x.d, CF_BLOCKS);
   }
   if (secondary) {
