@@ -279,8 +279,6 @@ static int allocate_all(Ctx& x) {
       A_(L.diag, ln); A_(L.dinv, ln); A_(L.x, ln); A_(L.b, ln); A_(L.r, ln);
       x.mg.push_back(L);
     }
-    A_(x.d_mg, x.mg.size());
-    cudaMemcpy(x.d_mg, x.mg.data(), sizeof(MgLevel) * x.mg.size(), cudaMemcpyHostToDevice);
     A_(x.mg_z, n); A_(x.mg_fr, n); A_(x.mg_dinv0, n); A_(x.mg_rsum, n); A_(x.mg_w, n);
     A_(x.mg_ragg, n * MG_ROW_SLOTS); A_(x.mg_rval, n * MG_ROW_SLOTS); A_(x.mg_rcnt, n);
     A_(x.mg_rv9, n * 8); A_(x.mg_rx, n); A_(x.mg_g32, (size_t)x.mg[0].n); A_(x.mg_q32, n);

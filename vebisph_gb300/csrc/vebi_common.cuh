@@ -88,11 +88,9 @@ struct Scal {
 
 // multigrid preconditioner (opt-in): coarse-row capacity, coarsest size, level cap, levels run
 // by one block, coarsest sweeps, Jacobi damping, coarse-correction scaling.  MG_BLOCK_ROWS is
-// measured: the 20k / 250k / 4M mixed solves take 1.99 / 4.11 / 26.7 ms at 512 (within 1% from
-// 256 to 1024) and 2.36 / 4.50 / 27.5 ms at 2048.
-// items of each of the corners' two lists
-constexpr int MIR_LIST = 4096;
-
+// measured: the 20k / 250k / 4M mixed solves take 1.44 / 3.69 / 25.9 ms at 512 and 1.48 / 3.65 /
+// 25.9 at 256; before the coarsest level's sweeps were one warp's, 1.99 / 4.11 / 26.7 at 512 (within
+// 1% from 256 to 1024) and 2.36 / 4.50 / 27.5 at 2048.
 constexpr int MG_SLOTS = 24;
 constexpr int MG_ROW_SLOTS = 16;
 constexpr int MG_COARSEST = 32;
@@ -112,6 +110,9 @@ struct MgLevel {
   double *val, *diag, *dinv;
   double *x, *b, *r;
 };
+
+// items of each of the two lists for the mirrors' corners
+constexpr int MIR_LIST = 4096;
 
 // Device arrays of one context.  Particle fields have capacity cap = npfb + mcap and are
 // indexed 0..np-1 with mirrors at npfb..np-1.  Pair arrays are ELL [k][i], stride npfb.

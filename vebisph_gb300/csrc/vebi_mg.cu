@@ -423,7 +423,7 @@ __device__ __forceinline__ double ap_stencil(const double* __restrict__ rv9, con
 // ---------------------------------------------------------------- V-cycle
 // the coarse levels, as the FP64 and the mixed V-cycle share them
 struct MgCoarse {
-  const MgLevel* lv;   // finest first
+  MgLevel lv[MG_MAX_LEVELS];  // finest first; a kernel parameter, so a phase does not wait for it
   int nl;              // number of coarse levels (>= 1)
   int tail;            // first level handled by block 0 alone
   const double* kinv;  // the coarsest level's dense inverse, if *kinv_ok
@@ -577,9 +577,78 @@ __device__ __forceinline__ void lv_prolong_smooth(const MgLevel& F, const double
   }
 }
 
+// MG_SWEEPS damped Jacobi sweeps of a level of at most 32 rows by one warp, a row a lane, with x, b
+// and the row's first slots in registers: lv_smooth's sums without its loads and block barriers
+// (where aggregates outside the domain leave the coarsest level without an inverse, its sweeps were
+// about half of the one-block levels' 22 us a V-cycle; with the levels in the kernel's parameters and
+// cell_sum, the 20k / 250k / 4M mixed solves went from 1.61 / 3.96 / 26.2 to 1.44 / 3.69 / 25.9 ms.
+// All the one-block levels in registers and shared memory were slower: 1.57 / 4.03 / 28.4, as the
+// call or the code around it costs the particle level's loops more registers).
+constexpr int SWEEP_SLOTS = 8;
+__device__ __forceinline__ void lv_sweeps(const MgLevel& L) {
+  const int c = threadIdx.x & 31;
+  const bool in = c < L.n;
+  const int m = in ? __ldg(L.cnt + c) : 0;
+  int k[SWEEP_SLOTS];
+  double v[SWEEP_SLOTS];
+#pragma unroll
+  for (int u = 0; u < SWEEP_SLOTS; ++u) {
+    k[u] = u < m ? __ldg(L.col + u * L.n + c) : c;
+    v[u] = u < m ? __ldg(L.val + u * L.n + c) : 0.0;
+  }
+  double x = 0.0, b = 0.0, dg = 0.0, od = 0.0;
+  if (in) {
+    x = L.x[c];
+    b = L.b[c];
+    dg = __ldg(L.diag + c);
+    od = MG_OMEGA * __ldg(L.dinv + c);
+  }
+  const int most = __reduce_max_sync(0xffffffffu, m);
+#pragma unroll 1
+  for (int sw = 0; sw < MG_SWEEPS; ++sw) {
+    double o[SWEEP_SLOTS], y = dg * x;
+#pragma unroll
+    for (int u = 0; u < SWEEP_SLOTS; ++u) o[u] = __shfl_sync(0xffffffffu, x, k[u]);
+#pragma unroll
+    for (int u = 0; u < SWEEP_SLOTS; ++u) {
+      if (u >= most) break;
+      if (u < m) y = fma(v[u], o[u], y);
+    }
+#pragma unroll 1
+    for (int u = SWEEP_SLOTS; u < most; ++u) {
+      const double xo = __shfl_sync(0xffffffffu, x, u < m ? __ldg(L.col + u * L.n + c) : c);
+      if (u < m) y = fma(__ldg(L.val + u * L.n + c), xo, y);
+    }
+    x = fma(od, b - y, x);
+  }
+  if (in) L.x[c] = x;
+}
+
 // the solution of level l after the upward pass: post-smoothed into r, or x on the coarsest
 __device__ __forceinline__ const double* lv_sol(const MgCoarse& a, int l) {
   return l == a.nl - 1 ? a.lv[l].x : a.lv[l].r;
+}
+
+// sum of a cell's entries of r in cell-list order (mirrors, n and up, follow the particles); the
+// loads of eight are in flight together
+template <class T>
+__device__ __forceinline__ T cell_sum(const int* __restrict__ ip, int ne, int n, const T* r) {
+  T b = 0;
+#pragma unroll 1
+  for (int k0 = 0; k0 < ne; k0 += 8) {
+    int i[8];
+    T v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) i[u] = k0 + u < ne ? __ldg(ip + k0 + u) : n;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = i[u] < n ? r[i[u]] : T(0);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (i[u] >= n) return b;
+      b += v[u];
+    }
+  }
+  return b;
 }
 
 // levels tail..nl-1 by block 0 alone
@@ -599,6 +668,9 @@ __device__ __forceinline__ void mg_block_levels(const MgCoarse& a) {
       for (int c = 0; c < K.n; ++c) v = fma(__ldg(a.kinv + (size_t)r * K.n + c), K.b[c], v);
       K.x[r] = v;
     }
+    __syncthreads();
+  } else if (K.n <= 32) {
+    if (i0 < 32) lv_sweeps(K);
     __syncthreads();
   } else {
     for (int sw = 0; sw < MG_SWEEPS; ++sw) {
@@ -644,12 +716,7 @@ __device__ bool mg_vcycle(const MgArgs& a, double* q, double qshift, double* out
     const MgLevel L1 = a.co.lv[0];
     for (int cc = tid; cc < L1.n; cc += stride) {
       const int s0 = __ldg(a.cstart + cc), ne = __ldg(a.ccnt + cc);
-      double b = 0.0;
-      for (int k = 0; k < ne; ++k) {
-        const int i = __ldg(a.ip + s0 + k);
-        if (i >= n) break;
-        b += a.fr[i];
-      }
+      const double b = cell_sum(a.ip + s0, ne, n, a.fr);
       L1.b[cc] = b;
       L1.x[cc] = MG_OMEGA * __ldg(L1.dinv + cc) * b;
     }
@@ -709,7 +776,7 @@ __device__ bool mg_vcycle(const MgArgs& a, double* q, double qshift, double* out
 
 // ---------------------------------------------------------------- preconditioned BiCGSTAB
 template <bool NONULL>
-__global__ void __launch_bounds__(TPB, 4) k_bicgstab_mg(MgArgs m) {
+__global__ void __launch_bounds__(TPB, 4) k_bicgstab_mg(const __grid_constant__ MgArgs m) {
   __shared__ SolverSh sh;
   const BiArgs& a = m.b;
   const int n = a.n;
@@ -1014,13 +1081,7 @@ __device__ bool mg_vcycle_mixed(const MgMxArgs& a, double* q, double qshift, dou
     const MgLevel L1 = a.co.lv[0];
     for (int cc = tid; cc < L1.n; cc += stride) {
       const int s0 = __ldg(a.cstart + cc), ne = __ldg(a.ccnt + cc);
-      float b32 = 0.f;  // the cell's residuals summed in FP32, in cell-list order
-      for (int k = 0; k < ne; ++k) {
-        const int i = __ldg(a.ip + s0 + k);
-        if (i >= n) break;
-        b32 += a.fr[i];
-      }
-      const double b = widen(b32);
+      const double b = widen(cell_sum(a.ip + s0, ne, n, a.fr));  // in FP32, as fr is
       L1.b[cc] = b;
       L1.x[cc] = MG_OMEGA * __ldg(L1.dinv + cc) * b;
     }
@@ -1086,7 +1147,7 @@ __device__ bool mg_vcycle_mixed(const MgMxArgs& a, double* q, double qshift, dou
 #endif
 
 template <bool NONULL>
-__global__ void __launch_bounds__(TPB, VEBI_MIXED_MG_BLOCKS_PER_SM) k_bicgstab_mixed_mg(MgMxArgs m) {
+__global__ void __launch_bounds__(TPB, VEBI_MIXED_MG_BLOCKS_PER_SM) k_bicgstab_mixed_mg(const __grid_constant__ MgMxArgs m) {
   __shared__ SolverSh sh;
   const MxArgs& a = m.b;
   const int n = a.n;
@@ -1346,6 +1407,17 @@ static int mg_setup(Ctx& x) {
   return tail;
 }
 
+static MgCoarse coarse_args(const Ctx& x, int tail, float* g32) {
+  MgCoarse co{};
+  co.nl = (int)x.mg.size();
+  for (int l = 0; l < co.nl; ++l) co.lv[l] = x.mg[l];
+  co.tail = tail;
+  co.kinv = x.mg_kinv;
+  co.kinv_ok = x.mg_kinv_ok;
+  co.g32 = g32;
+  return co;
+}
+
 void launch_ppe_mg_mixed(Ctx& x) {
   const Consts& c = x.c;
   const Dev& d = x.d;
@@ -1366,8 +1438,8 @@ void launch_ppe_mg_mixed(Ctx& x) {
   MgMxArgs m{MxArgs{d.bx, d.br, d.brb, d.bv, d.bp, d.bs, d.bt, d.bM, d.partials, d.p, d.pi2, d.si2, d.ppe_B,
                     d.rowsum, d.ppe_val32, d.ppe_col, d.ij_count, d.s, (long long)c.npfb, c.npfb, c.itermax, c.tol,
                     c.warm_start},
-             MgCoarse{x.d_mg, (int)x.mg.size(), tail, x.mg_kinv, x.mg_kinv_ok, x.mg_g32}, d.cellpart, d.cell_start, d.cell_cnt, d.ip, (float*)x.mg_z,
-             (float*)x.mg_fr, (float*)x.mg_dinv0, x.mg_ragg, x.mg_rx, x.mg_rval, (const float*)x.mg_rv9, c.ncx,
+             coarse_args(x, tail, x.mg_g32), d.cellpart, d.cell_start, d.cell_cnt, d.ip, (float*)x.mg_z, (float*)x.mg_fr,
+             (float*)x.mg_dinv0, x.mg_ragg, x.mg_rx, x.mg_rval, (const float*)x.mg_rv9, c.ncx,
              (float*)x.mg_w, (float*)x.mg_rsum, x.mg_q32, d.ppe_diag};
   if (c.open_domain == 0) cudaLaunchKernelEx(&cfg, k_bicgstab_mixed_mg<true>, m);
   else cudaLaunchKernelEx(&cfg, k_bicgstab_mixed_mg<false>, m);
@@ -1377,7 +1449,6 @@ void launch_ppe_mg_mixed(Ctx& x) {
 void launch_ppe_mg(Ctx& x) {
   const Consts& c = x.c;
   const Dev& d = x.d;
-  const int nl = (int)x.mg.size();
   const int tail = mg_setup(x);
   int nblk = x.mg_blocks;
   const long long rows_per_block = (long long)TPB * (x.solver_rows_per_thread > 0 ? x.solver_rows_per_thread : 1);
@@ -1395,8 +1466,8 @@ void launch_ppe_mg(Ctx& x) {
   MgArgs m{BiArgs{d.bx, d.br, d.brb, d.bv, d.bp, d.bpi, d.bs, d.bsi, d.bt, d.bM, d.partials, d.p, d.ppe_B,
                   d.ppe_diag, d.ppe_val, d.ppe_col, d.ij_count, d.s, (long long)c.npfb, c.npfb, c.itermax, c.tol,
                   c.warm_start},
-           MgCoarse{x.d_mg, nl, tail, x.mg_kinv, x.mg_kinv_ok, nullptr}, d.cellpart, d.cell_start, d.cell_cnt, d.ip, x.mg_z, x.mg_fr, x.mg_dinv0, x.mg_rsum,
-           x.mg_ragg, x.mg_rx, x.mg_rval, x.mg_rv9, c.ncx, x.mg_w};
+           coarse_args(x, tail, nullptr), d.cellpart, d.cell_start, d.cell_cnt, d.ip, x.mg_z, x.mg_fr, x.mg_dinv0,
+           x.mg_rsum, x.mg_ragg, x.mg_rx, x.mg_rval, x.mg_rv9, c.ncx, x.mg_w};
   if (c.open_domain == 0) cudaLaunchKernelEx(&cfg, k_bicgstab_mg<true>, m);
   else cudaLaunchKernelEx(&cfg, k_bicgstab_mg<false>, m);
   x.launches++;
