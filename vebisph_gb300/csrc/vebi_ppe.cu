@@ -19,6 +19,7 @@
 //   p-update+sum(p) | p-=mean, p_inv | v=A p_inv, (r_bar,v) | s, |s|^2, sum(s) |
 //   s-=mean, s_inv | t=A s_inv, (t,s), |t|^2 | x,r update, |r|^2, (r_bar,r)
 // The barrier spins are bounded: on timeout the kernel records VEBI_ERR_TIMEOUT and returns.
+#include "vebi_lanes.cuh"
 #include "vebi_solver.cuh"
 
 namespace vebi {
@@ -26,27 +27,44 @@ namespace vebi {
 #define ELL(k, i) ((size_t)(k) * c.npfb + (i))
 
 // ---------------------------------------------------------------------- right-hand side
-__global__ void k_ppe_rhs(Consts c, Dev d) {
+template <int P>
+__global__ void __launch_bounds__(P == 1 ? TPB : LANES_TPB) k_ppe_rhs(Consts c, Dev d) {
   using fp::mul_int;  // the products beside the FP64 pipe, as in k_gradients
   __shared__ double sh[TPB / 32 + 1];
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double b = 0.0;
-  if (i < c.npfb) {
-    const double ui = d.ux2[i], vi = d.uy2[i];  // u* (predictor output, mirrors included)
-    const double K11 = d.kgcm[0][i], K21 = d.kgcm[1][i], K12 = d.kgcm[2][i], K22 = d.kgcm[3][i];
-    double fb = 0.0;
-    const int cnt = d.ij_count[i];
-    for (int k = 0; k < cnt; ++k) {
-      int j = d.ij_link[ELL(k, i)];
-      double u1 = ui - d.ux2[j], u2 = vi - d.uy2[j];
-      double w1 = d.wGx[ELL(k, i)], w2 = d.wGy[ELL(k, i)];
-      double kw1 = mul_int(K11, w1) + mul_int(K12, w2), kw2 = mul_int(K21, w1) + mul_int(K22, w2);
-      fb = fb - (mul_int(u1, kw1) + mul_int(u2, kw2));
-    }
-    b = fb / d.s->dt;
-    d.ppe_B[i] = b;
+  bool in;
+  const int i = lane_row<P>(c.npfb, in);
+  const double ui = d.ux2[i], vi = d.uy2[i];  // u* (predictor output, mirrors included)
+  const double K11 = d.kgcm[0][i], K21 = d.kgcm[1][i], K12 = d.kgcm[2][i], K22 = d.kgcm[3][i];
+  double fb = 0.0;
+  const int cnt = in ? d.ij_count[i] : 0;
+  auto pair = [&](int k) {
+    const int j = d.ij_link[ELL(k, i)];
+    const double u1 = ui - d.ux2[j], u2 = vi - d.uy2[j];
+    const double w1 = d.wGx[ELL(k, i)], w2 = d.wGy[ELL(k, i)];
+    const double kw1 = mul_int(K11, w1) + mul_int(K12, w2), kw2 = mul_int(K21, w1) + mul_int(K22, w2);
+    return mul_int(u1, kw1) + mul_int(u2, kw2);
+  };
+  if constexpr (P == 1) {
+    for (int k = 0; k < cnt; ++k) fb = fb - pair(k);
+  } else {
+    double s[1];
+    pair_sums64<1, 1>(cnt, [&](int k, double* t) { t[0] = -pair(k); }, s);
+    fb = s[0];
   }
-  double bs = block_sum<TPB>(b, sh);
+  double b = 0.0;
+  if (in) b = fb / d.s->dt;
+  if (in && (P == 1 || (threadIdx.x & (P - 1)) == 0)) d.ppe_B[i] = b;
+  if constexpr (P == 1) {  // else k_ppe_row_sums
+    const double bs = block_sum<TPB>(b, sh);
+    if (threadIdx.x == 0) d.partials[blockIdx.x] = bs;
+  }
+}
+
+// the right-hand side's sum by blocks of TPB rows
+__global__ void k_ppe_row_sums(Consts c, Dev d) {
+  __shared__ double sh[TPB / 32 + 1];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const double bs = block_sum<TPB>(i < c.npfb ? d.ppe_B[i] : 0.0, sh);
   if (threadIdx.x == 0) d.partials[blockIdx.x] = bs;
 }
 
@@ -470,7 +488,8 @@ void launch_ppe(Ctx& x) {
   stage_mark(x, 9);
   const bool mixed = x.precision == VEBI_PREC_MIXED;
   if (mixed) launch_ppe_rhs32(x);
-  else VEBI_LAUNCH(x, k_ppe_rhs, g, TPB, c, x.d);
+  else LAUNCH_ROWS(x, k_ppe_rhs, LANE_ROWS);
+  if (c.npfb <= LANE_ROWS) VEBI_LAUNCH(x, k_ppe_row_sums, g, TPB, c, x.d);
   VEBI_LAUNCH(x, k_ppe_mean, 1, TPB, c, x.d, g);
   VEBI_LAUNCH(x, k_ppe_assemble, g, TPB, c, x.d, mixed ? (const float*)x.d.wL32 : (const float*)nullptr,
               x.rep_p != nullptr ? 1 : 0);

@@ -15,6 +15,7 @@
 // One thread per particle walks that particle's ELL row k = 0..ij_count-1 in the reference's
 // order with the reference's association, so every per-particle sum is the reference's sum.
 #include "vebi_ctx.cuh"
+#include "vebi_lanes.cuh"
 
 namespace vebi {
 
@@ -339,23 +340,42 @@ __global__ void k_copy_normals(Consts c, Dev d) {
 // these kernels on large domains; on small ones they cost nothing either.  4M particles, without /
 // with: gradients 5.28 / 3.24 ms, predictor 10.97 / 5.81 ms (7.31 with two blocks per SM: 82
 // registers leave too few warps to cover the gathers), right-hand side 3.9 / 1.9 ms.
-__global__ void __launch_bounds__(TPB, 4) k_gradients(Consts c, Dev d) {
+template <int P>
+__global__ void __launch_bounds__(P == 1 ? TPB : LANES_TPB, P == 1 ? 4 : 1) k_gradients(Consts c, Dev d) {
   using fp::mul_int;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.npfb) return;
+  bool in;
+  const int i = lane_row<P>(c.npfb, in);
+  if (P == 1 && !in) return;
   const double ui = d.ux[i], vi = d.uy[i], ti = d.th[i];
   double a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0;
-  const int cnt = d.ij_count[i];
-  for (int k = 0; k < cnt; ++k) {
-    int j = d.ij_link[ELL(k, i)];
-    double w1 = d.wGx[ELL(k, i)], w2 = d.wGy[ELL(k, i)];
-    double du = d.ux[j] - ui, dvv = d.uy[j] - vi, dth = d.th[j] - ti;
-    a0 = a0 + mul_int(du, w1);
-    a1 = a1 + mul_int(du, w2);
-    a2 = a2 + mul_int(dvv, w1);
-    a3 = a3 + mul_int(dvv, w2);
-    a4 = a4 + mul_int(dth, w1);
-    a5 = a5 + mul_int(dth, w2);
+  const int cnt = in ? d.ij_count[i] : 0;
+  auto pair = [&](int k, auto put) {
+    const int j = d.ij_link[ELL(k, i)];
+    const double w1 = d.wGx[ELL(k, i)], w2 = d.wGy[ELL(k, i)];
+    const double du = d.ux[j] - ui, dvv = d.uy[j] - vi, dth = d.th[j] - ti;
+    put(0, mul_int(du, w1));
+    put(1, mul_int(du, w2));
+    put(2, mul_int(dvv, w1));
+    put(3, mul_int(dvv, w2));
+    put(4, mul_int(dth, w1));
+    put(5, mul_int(dth, w2));
+  };
+  if constexpr (P == 1) {
+    for (int k = 0; k < cnt; ++k)
+      pair(k, [&](int e, double v) {
+        if (e == 0) a0 = a0 + v;
+        if (e == 1) a1 = a1 + v;
+        if (e == 2) a2 = a2 + v;
+        if (e == 3) a3 = a3 + v;
+        if (e == 4) a4 = a4 + v;
+        if (e == 5) a5 = a5 + v;
+      });
+  } else {
+    double a[6];
+    pair_sums64<6, 1>(
+        cnt, [&](int k, double* t) { pair(k, [&](int e, double v) { t[e] = v; }); }, a);
+    if (!in || (threadIdx.x & (P - 1))) return;
+    a0 = a[0], a1 = a[1], a2 = a[2], a3 = a[3], a4 = a[4], a5 = a[5];
   }
   const double K11 = d.kgcm[0][i], K21 = d.kgcm[1][i], K12 = d.kgcm[2][i], K22 = d.kgcm[3][i];
   d.grad[0][i] = K11 * a0 + K12 * a1;
@@ -472,10 +492,12 @@ __global__ void k_logconf(Consts c, Dev d) {
 
 // ---------------------------------------------------------------------- predictor
 // rhs pair loop + buoyancy; u*, theta* written to the second buffers (walls copied)
-__global__ void __launch_bounds__(TPB, 4) k_predictor(Consts c, Dev d) {
+template <int P>
+__global__ void __launch_bounds__(P == 1 ? TPB : LANES_TPB, P == 1 ? 4 : 1) k_predictor(Consts c, Dev d) {
   using fp::mul_int;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.npfb) return;
+  bool in;
+  const int i = lane_row<P>(c.npfb, in);
+  if (P == 1 && !in) return;
   const double ui = d.ux[i], vi = d.uy[i], ti = d.th[i];
   const double K11 = d.kgcm[0][i], K21 = d.kgcm[1][i], K12 = d.kgcm[2][i], K22 = d.kgcm[3][i];
   double Ti11 = 0, Ti21 = 0, Ti12 = 0, Ti22 = 0;
@@ -483,25 +505,46 @@ __global__ void __launch_bounds__(TPB, 4) k_predictor(Consts c, Dev d) {
   if (ve) { Ti11 = d.tau[0][i]; Ti21 = d.tau[1][i]; Ti12 = d.tau[2][i]; Ti22 = d.tau[3][i]; }
   const double cs = c.coeff_solvent, cp = c.coeff_polymeric, ct = c.coeff_theta;
   double s1 = 0, s2 = 0, st = 0;
-  const int cnt = d.ij_count[i];
-  for (int k = 0; k < cnt; ++k) {
-    int j = d.ij_link[ELL(k, i)];
-    double u1 = ui - d.ux[j], u2 = vi - d.uy[j];
-    double wl = d.wL[ELL(k, i)];
+  const int cnt = in ? d.ij_count[i] : 0;
+  // terms 0 and 1 of u, the polymeric and the solvent one, 2 and 3 of v, 5 of theta
+  auto pair = [&](int k, auto put) {
+    const int j = d.ij_link[ELL(k, i)];
+    const double u1 = ui - d.ux[j], u2 = vi - d.uy[j];
+    const double wl = d.wL[ELL(k, i)];
     if (ve) {
-      double w1 = d.wGx[ELL(k, i)], w2 = d.wGy[ELL(k, i)];
-      double T11 = d.tau[0][j] - Ti11, T21 = d.tau[1][j] - Ti21;
-      double T12 = d.tau[2][j] - Ti12, T22 = d.tau[3][j] - Ti22;
-      double kw1 = mul_int(K11, w1) + mul_int(K12, w2), kw2 = mul_int(K21, w1) + mul_int(K22, w2);
-      double tw1 = mul_int(T11, kw1) + mul_int(T12, kw2), tw2 = mul_int(T21, kw1) + mul_int(T22, kw2);
-      s1 = s1 + mul_int(cp, tw1) + mul_int(mul_int(cs, u1), wl);
-      s2 = s2 + mul_int(cp, tw2) + mul_int(mul_int(cs, u2), wl);
+      const double w1 = d.wGx[ELL(k, i)], w2 = d.wGy[ELL(k, i)];
+      const double T11 = d.tau[0][j] - Ti11, T21 = d.tau[1][j] - Ti21;
+      const double T12 = d.tau[2][j] - Ti12, T22 = d.tau[3][j] - Ti22;
+      const double kw1 = mul_int(K11, w1) + mul_int(K12, w2), kw2 = mul_int(K21, w1) + mul_int(K22, w2);
+      const double tw1 = mul_int(T11, kw1) + mul_int(T12, kw2), tw2 = mul_int(T21, kw1) + mul_int(T22, kw2);
+      put(0, mul_int(cp, tw1));
+      put(1, mul_int(mul_int(cs, u1), wl));
+      put(2, mul_int(cp, tw2));
+      put(3, mul_int(mul_int(cs, u2), wl));
     } else {
-      s1 = s1 + mul_int(mul_int(cs, u1), wl);
-      s2 = s2 + mul_int(mul_int(cs, u2), wl);
+      put(1, mul_int(mul_int(cs, u1), wl));
+      put(3, mul_int(mul_int(cs, u2), wl));
     }
-    double thij = ti - d.th[j];
-    st = st + mul_int(mul_int(ct, thij), wl);
+    put(5, mul_int(mul_int(ct, ti - d.th[j]), wl));
+  };
+  if constexpr (P == 1) {
+    for (int k = 0; k < cnt; ++k)
+      pair(k, [&](int e, double v) {
+        if (e < 2) s1 = s1 + v;
+        else if (e < 4) s2 = s2 + v;
+        else st = st + v;
+      });
+  } else {
+    double s[3];
+    pair_sums64<3, 2>(
+        cnt,
+        [&](int k, double* t) {
+          t[0] = t[2] = t[4] = 0.0;
+          pair(k, [&](int e, double v) { t[e] = v; });
+        },
+        s);
+    if (!in || (threadIdx.x & (P - 1))) return;
+    s1 = s[0], s2 = s[1], st = s[2];
   }
   s2 = s2 + ti;  // buoyancy (predictor_mod.F90:111-119)
   const double dt = d.s->dt;
@@ -516,17 +559,9 @@ __global__ void __launch_bounds__(TPB, 4) k_predictor(Consts c, Dev d) {
   }
 }
 
-__device__ __forceinline__ void pgrad_one(const Consts& c, const Dev& d, int i, double& mu, double& mv,
-                                          double& mp) {
+__device__ __forceinline__ void pgrad_one(const Consts& c, const Dev& d, int i, int cnt, double a, double b, double& mu,
+                                          double& mv, double& mp) {
   const double pi_ = d.p[i];
-  double a = 0, b = 0;
-  const int cnt = d.ij_count[i];
-  for (int k = 0; k < cnt; ++k) {
-    int j = d.ij_link[ELL(k, i)];
-    double temp = d.p[j] - pi_;
-    a = a + temp * d.wGx[ELL(k, i)];
-    b = b + temp * d.wGy[ELL(k, i)];
-  }
   const double K11 = d.kgcm[0][i], K21 = d.kgcm[1][i], K12 = d.kgcm[2][i], K22 = d.kgcm[3][i];
   double gx = K11 * a + K12 * b, gy = K21 * a + K22 * b;
   d.gpx[i] = gx;
@@ -557,12 +592,35 @@ __device__ __forceinline__ void pgrad_one(const Consts& c, const Dev& d, int i, 
 // ---------------------------------------------------------------------- pressure gradient
 // grad P, velocity update (div_free.F90:96-101), final advection (:111-117): reads u* (ux2)
 // and writes u^{n+1} and r^{n+1} in place (no kernel of this launch reads neighbours' u or r).
-__global__ void k_pgrad_final(Consts c, Dev d) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+template <int P>
+__global__ void __launch_bounds__(P == 1 ? TPB : LANES_TPB) k_pgrad_final(Consts c, Dev d) {
+  bool in;
+  const int i = lane_row<P>(c.npfb, in);
   double mu = -1.0, mv = -1.0, mp = -1.0;
-  if (i < c.npfb) pgrad_one(c, d, i, mu, mv, mp);
+  const int cnt = in ? d.ij_count[i] : 0;
+  const double pi_ = d.p[i];
+  double a = 0, b = 0;
+  auto pair = [&](int k, double* t) {
+    const double temp = d.p[d.ij_link[ELL(k, i)]] - pi_;
+    t[0] = temp * d.wGx[ELL(k, i)];
+    t[1] = temp * d.wGy[ELL(k, i)];
+  };
+  if constexpr (P == 1) {
+    for (int k = 0; k < cnt; ++k) {
+      double t[2];
+      pair(k, t);
+      a = a + t[0];
+      b = b + t[1];
+    }
+  } else {
+    double s[2];
+    pair_sums64<2, 1>(cnt, pair, s);
+    a = s[0], b = s[1];
+    if (threadIdx.x & (P - 1)) in = false;  // the row's first lane has the rest
+  }
+  if (in) pgrad_one(c, d, i, cnt, a, b, mu, mv, mp);
   // divergence guard (opt-in) on the new velocity (false for NaN too)
-  if (c.u_limit > 0.0 && i < c.npfb && !(mu <= c.u_limit && mv <= c.u_limit)) set_error(d.s, VEBI_ERR_DIVERGED);
+  if (c.u_limit > 0.0 && in && !(mu <= c.u_limit && mv <= c.u_limit)) set_error(d.s, VEBI_ERR_DIVERGED);
   warp_max_pos(&d.s->absu_bits, mu);
   warp_max_pos(&d.s->absv_bits, mv);
   warp_max_pos(&d.s->absp_bits, mp);
@@ -803,7 +861,7 @@ void launch_predictor(Ctx& x) {
   const bool mixed = x.precision == VEBI_PREC_MIXED;
   stage_mark(x, 6);
   if (mixed) launch_gradients32(x);
-  else VEBI_LAUNCH(x, k_gradients, g, TPB, c, x.d);
+  else LAUNCH_ROWS(x, k_gradients, LANE_ROWS);
   launch_grad_mirrors(x);
   stage_mark(x, 7);
   if (c.const_mod != 1) {
@@ -812,7 +870,7 @@ void launch_predictor(Ctx& x) {
   }
   stage_mark(x, 8);
   if (mixed) launch_predictor32(x);
-  else VEBI_LAUNCH(x, k_predictor, g, TPB, c, x.d);
+  else LAUNCH_ROWS(x, k_predictor, LANE_ROWS);
   launch_mirror_velocities(x);
   // theta* replaces theta for walls and fluid; u* stays in ux2/uy2 for the PPE and the update
   cudaMemcpyAsync(x.d.th, x.d.th2, sizeof(double) * (size_t)c.npfb, cudaMemcpyDeviceToDevice, x.st);
@@ -828,7 +886,7 @@ void launch_final(Ctx& x, int secondary) {
   cudaMemcpyAsync(x.d.ry2, x.d.ry, sizeof(double) * (size_t)c.cap, cudaMemcpyDeviceToDevice, x.st);
   const bool mixed = x.precision == VEBI_PREC_MIXED;
   if (mixed) launch_pgrad_final32(x);
-  else VEBI_LAUNCH(x, k_pgrad_final, g, TPB, c, x.d);
+  else LAUNCH_ROWS(x, k_pgrad_final, LANE_ROWS_PGRAD);
   if (c.correct_velocity) {
     VEBI_LAUNCH(x, k_correct_velocity, g, TPB, c, x.d);
     VEBI_LAUNCH(x, k_advect_final, g, TPB, c, x.d);
