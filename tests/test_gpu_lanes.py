@@ -50,3 +50,23 @@ def test_fp32_sums_close_to_fp64(built, name):
         assert np.abs(x - y).max() <= 44 * 2.0**-24 * 10 * scale, (nm, np.abs(x - y).max() / scale)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("name", ["dam:4", "dam:33", "dam:118", "dam:119", "surface:75"])
+def test_free_surface_sums_equal_the_oracle(built, name):
+    from oracle.oracle import OracleSolver
+    from vebisph_gb300.solver import StepSolver
+    kind, n = name.split(":")
+    case = (cases.dam_break if kind == "dam" else cases.free_surface_periodic)(int(n), seed=int(n))
+    case.itermax = 2
+    gpu, ref = StepSolver(case), OracleSolver(case)
+    gpu.step(), ref.step()
+    assert np.array_equal(gpu.get("n_surf")[: case.npfb], ref.get("n_surf")[: case.npfb])
+    for nm in ("conc", "div_r"):
+        a, b = gpu.get(nm), ref.get(nm)
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max(), nm
+    rep = compare_step(gpu, ref, case)
+    for nm in ("ushift_x", "ushift_y", *SUMS):
+        assert rep[nm][0] <= rep[nm][1], (nm, rep[nm])
+    gpu.close()
+    ref.close()
