@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(TPB) k_na_bicgstab(NaArgs a) {
 // What bounds it: up to two warps a scheduler, the chain of an iteration (seven barriers, five
 // sums, two products of 45 dependent FMAs), ~24 us; above that the FP64 pipe, at ~150 operations a row.
 // Measured against k_na_bicgstab, ms per solve: 576 rows x 24 iterations 0.57 / 1.45, 16k x 98
-// 2.70 / 6.29, 36k x 142 4.90 / 9.61, 65k x 196 8.4 / 15.7.
+// 2.70 / 6.29 (open, x 164, 3.84 / 9.57), 36k x 142 4.90 / 9.61, 65k x 196 8.4 / 15.7.
 template <bool NONULL>
 __global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, int nvb, int keep) {
   extern __shared__ double na_mat[];  // the first `keep` slots of the block's rows: values, then columns
@@ -378,7 +378,11 @@ __global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, 
                        [&]() { sh.alpha = fp::quotient(sh.rho, sh.v[0] + 1.0e-15); }))
       return failed();
     const double alpha = sh.alpha;
-    double s = r - alpha * v;
+    double s = r - alpha * v, sinv = 0.0;
+    if (!NONULL) {  // before the reduction, whose barrier the product needs anyway
+      sinv = fp::quotient(s, den, rden);
+      if (mine) sinv_all[i] = sinv;
+    }
     if (!res_reduce<2>(bar, mine ? plus_zero(s * s) : 0.0, mine ? plus_zero(s) : 0.0, part0, gpb, nvb, sh, [&]() {
           sh.n2 = sh.v[0];
           if (iter == 1) sh.n2s0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
@@ -391,10 +395,12 @@ __global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, 
       done = at_s = true;
       break;
     }
-    if (NONULL) s = s - sh.mean;
-    const double sinv = fp::quotient(s, den, rden);
-    if (mine) sinv_all[i] = sinv;
-    if (!res_sync(bar)) return failed();
+    if (NONULL) {
+      s = s - sh.mean;
+      sinv = fp::quotient(s, den, rden);
+      if (mine) sinv_all[i] = sinv;
+      if (!res_sync(bar)) return failed();
+    }
     const double tv = product(sinv_all);
     if (!res_reduce<2>(bar, mine ? plus_zero(tv * s) : 0.0, mine ? plus_zero(tv * tv) : 0.0, part1, gpb, nvb, sh,
                        [&]() { sh.omega = fp::quotient(sh.v[0], sh.v[1] + 1.0e-15); }))

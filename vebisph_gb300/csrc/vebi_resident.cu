@@ -19,11 +19,10 @@
 //
 // What bounds it.  FP64 issues one warp instruction per 64-76 cycles and scheduler on this GPU:
 // ~107 operations a row and iteration are 64 cycles per row of an SM (2 us at 66 rows).  The
-// dependent chain of an iteration is the rest: seven barriers of ~1.1 us, five sums of some 20
-// dependent adds (0.6-1 us with their load), six divisions of 0.27 us, two products' gathers.
-// Measured, ms per solve, k_bicgstab / this kernel: 1.7k rows x 60 iterations 2.39 / 1.21, 2.9k x
-// 75 2.48 / 1.36, 10k x 139 5.37 / 3.40, 20k x 363 14.9 / 12.1, 29k x 247 10.2 /
-// 9.8.
+// dependent chain of an iteration is the rest: five to seven barriers of ~1.1 us, five sums of some 20
+// dependent adds (0.6-1 us with their load), six quotients of ~0.2 us, two products' gathers.
+// Measured, ms per solve, k_bicgstab / this kernel: 1.7k rows x 60 iterations 2.39 / 1.16, 2.9k x
+// 75 (open) 2.48 / 1.25, 10k x 139 5.37 / 3.36, 20k x 363 14.9 / 12.0, 29k x 247 10.2 / 9.7.
 #include "vebi_resident.cuh"
 
 namespace vebi {
@@ -45,8 +44,8 @@ struct LaneRow {
     }
   }
   // N slots k(u), u = 0.. N-1, of which those with in(u): columns and values, then operands, then FMAs
-  template <int N, class Slot, class In>
-  __device__ __forceinline__ void slots(const BiArgs& a, const double* xv, double& b, Slot k, In in) const {
+  template <int N, class Slot, class In, class Value>
+  __device__ __forceinline__ void slots(const BiArgs& a, const double* xv, double& b, Slot k, In in, Value value) const {
     int c[N];
     double v[N], x[N];
 #pragma unroll
@@ -59,15 +58,20 @@ struct LaneRow {
     for (int u = 0; u < N; ++u) x[u] = in(u) ? __ldca(xv + c[u]) : 0.0;
 #pragma unroll
     for (int u = 0; u < N; ++u)
-      if (in(u)) b = fma(v[u], x[u], b);
+      if (in(u)) b = fma(v[u], value(x[u]), b);
   }
 };
 
-// KEEP: this many quads of a row stay in registers for the whole solve (0: all come from L2)
-template <bool NONULL, int T_MAX, int KEEP>
+// KEEP: this many quads of a row stay in registers for the whole solve (0: all come from L2).
+// RAW (closed domains): the products gather p and s and take off the mean and scale as they do, twice the
+// FP64 operations a slot for two barriers less.
+template <bool NONULL, int T_MAX, int KEEP, bool RAW = false>
 __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gpb, int nvb) {
   __shared__ ResSh sh;
   __shared__ double vec[RES_MAX_ROWS];  // a product's results, by row of the block
+  // the vector a product gathers goes out before the reduction that precedes the product, whose barrier
+  // then is the only one: s_inv of an open domain as it is; with RAW, p and s before their mean is known
+  constexpr bool EARLY = RAW || !NONULL;
   const int n = a.n, t = threadIdx.x;
   const int R = gpb * RES_GROUP, row0 = blockIdx.x * R;
   Scal* s = a.sc;
@@ -75,7 +79,7 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
   const GridBar bar{&s->bar_count, &s->error};
   const double rinv1 = 1.0 / (1.0 + 1.0e-15);
   const double small = NONULL ? 1.0e-6 : 4.0;  // open solver: the integer expression 10-6
-  const double dn = (double)n;
+  const double dn = (double)n, rdn = fp::reciprocal(dn), tol2 = a.tol * a.tol;
   double* const part0 = a.part;
   double* const part1 = a.part + 2 * (size_t)nvb * RES_VB;  // used in turn: a slow block may still read one
   if (t == 0) {
@@ -100,26 +104,27 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
     }
   }
   // y = A x for the block's rows, to their threads (x complete and visible in every block)
-  auto product = [&](const double* xv) {
+  auto product = [&](const double* xv, double shift) {
+    auto value = [&](double x) { return RAW ? fp::mul_int(x - shift, rinv1) : x; };
     double b = 0.0;
     if (L.row >= 0) {
       if (KEEP) {
         double x[KEEP ? KEEP : 1];
 #pragma unroll
         for (int e = 0; e < KEEP; ++e) x[e] = e < L.nq ? __ldca(xv + ck[e]) : 0.0;
-        if (L.q == 0) b = dk * __ldca(xv + L.row);
+        if (L.q == 0) b = dk * value(__ldca(xv + L.row));
 #pragma unroll
         for (int e = 0; e < KEEP; ++e)
-          if (e < L.nq) b = fma(vk[e], x[e], b);
+          if (e < L.nq) b = fma(vk[e], value(x[e]), b);
       } else if (L.q == 0) {
-        b = dk * __ldca(xv + L.row);
+        b = dk * value(__ldca(xv + L.row));
       }
       constexpr int Q = KEEP ? 4 : 6;
 #pragma unroll 1
       for (int m = KEEP; m < L.nq; m += Q)
-        L.slots<Q>(a, xv, b, [&](int u) { return 4 * (m + u) + L.q; }, [&](int u) { return m + u < L.nq; });
+        L.slots<Q>(a, xv, b, [&](int u) { return 4 * (m + u) + L.q; }, [&](int u) { return m + u < L.nq; }, value);
       if (L.q == 0)
-        L.slots<3>(a, xv, b, [&](int u) { return 4 * L.nq + u; }, [&](int u) { return 4 * L.nq + u < L.cnt; });
+        L.slots<3>(a, xv, b, [&](int u) { return 4 * L.nq + u; }, [&](int u) { return 4 * L.nq + u < L.cnt; }, value);
     }
     b += __shfl_xor_sync(0xffffffffu, b, 1);  // (b0 + b1) + (b2 + b3)
     b += __shfl_xor_sync(0xffffffffu, b, 2);
@@ -134,7 +139,7 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
       a.pinv[i] = x;
     }
     if (!grid_sync(s)) return;
-    const double y = product(a.pinv);
+    const double y = product(a.pinv, 0.0);
     if (mine) r = a.B[i] - y;
     if (!grid_sync(s)) return;  // every product has read x0 before p_inv is written
   } else if (mine) {
@@ -148,25 +153,29 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
   while (iter <= a.itermax) {
     if (is_zero(sh.rho)) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
     if (mine) p = iter == 1 ? r : fma(sh.beta, fma(-sh.omega, v, p), r);
+    if (RAW && mine) a.pinv[i] = p;
     if (NONULL) {
-      if (!res_reduce<1>(bar, mine ? plus_zero(p) : 0.0, 0.0, part0, gpb, nvb, sh, [&]() { sh.mean = sh.v[0] / dn; }))
+      if (!res_reduce<1>(bar, mine ? plus_zero(p) : 0.0, 0.0, part0, gpb, nvb, sh, [&]() { sh.mean = fp::quotient(sh.v[0], dn, rdn); }))
         return;
       p = p - sh.mean;
     }
     const double pinv = p * rinvM;
-    if (mine) a.pinv[i] = pinv;
-    if (!grid_sync(s)) return;
-    v = product(a.pinv);
+    if (!RAW) {
+      if (mine) a.pinv[i] = pinv;
+      if (!grid_sync(s)) return;
+    }
+    v = product(a.pinv, sh.mean);
     if (!res_reduce<1>(bar, mine ? fma(rb, v, 0.0) : 0.0, 0.0, part1, gpb, nvb, sh,
-                       [&]() { sh.alpha = sh.rho / (sh.v[0] + 1.0e-15); }))
+                       [&]() { sh.alpha = fp::quotient(sh.rho, sh.v[0] + 1.0e-15); }))
       return;
     const double alpha = sh.alpha;
     double sv = mine ? fma(-alpha, v, r) : 0.0;
+    if (EARLY && mine) a.sinv[i] = NONULL ? sv : sv * rinvM;
     if (!res_reduce<2>(bar, mine ? fma(sv, sv, 0.0) : 0.0, mine ? plus_zero(sv) : 0.0, part0, gpb, nvb, sh, [&]() {
           sh.n2 = sh.v[0];
           if (iter == 1) sh.n2s0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
-          sh.flag = sh.v[0] <= a.tol * a.tol * sh.n2s0;
-          if (NONULL) sh.mean = sh.v[1] / dn;
+          sh.flag = sh.v[0] <= tol2 * sh.n2s0;
+          if (NONULL) sh.mean = fp::quotient(sh.v[1], dn, rdn);
         }))
       return;
     if (sh.flag) {
@@ -176,11 +185,13 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
     }
     if (NONULL) sv = sv - sh.mean;
     const double sinv = sv * rinvM;
-    if (mine) a.sinv[i] = sinv;
-    if (!grid_sync(s)) return;
-    const double tv = product(a.sinv);
+    if (!EARLY) {
+      if (mine) a.sinv[i] = sinv;
+      if (!grid_sync(s)) return;
+    }
+    const double tv = product(a.sinv, sh.mean);
     if (!res_reduce<2>(bar, mine ? fma(tv, sv, 0.0) : 0.0, mine ? fma(tv, tv, 0.0) : 0.0, part1, gpb, nvb, sh,
-                       [&]() { sh.omega = sh.v[0] / (sh.v[1] + 1.0e-15); }))
+                       [&]() { sh.omega = fp::quotient(sh.v[0], sh.v[1] + 1.0e-15); }))
       return;
     const double omega = sh.omega;
     x = fma(omega, sinv, fma(alpha, pinv, x));
@@ -188,8 +199,8 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
     if (!res_reduce<2>(bar, mine ? fma(r, r, 0.0) : 0.0, mine ? fma(rb, r, 0.0) : 0.0, part0, gpb, nvb, sh, [&]() {
           sh.n2 = sh.v[0];
           if (iter == 1) sh.n2r0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
-          sh.flag = sh.v[0] <= a.tol * a.tol * sh.n2r0;
-          sh.beta = sh.v[1] / (sh.rho + 1.0e-15) * alpha / (omega + 1.0e-15);
+          sh.flag = sh.v[0] <= tol2 * sh.n2r0;
+          sh.beta = fp::quotient(fp::quotient(sh.v[1], sh.rho + 1.0e-15) * alpha, omega + 1.0e-15);
           sh.rho = sh.v[1];
         }))
       return;
@@ -230,8 +241,12 @@ bool launch_bicgstab_resident(Ctx& x, const BiArgs& a, bool nonull) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   auto go = [&](auto closed, auto open) { return cudaLaunchKernelEx(&cfg, nonull ? closed : open, a, gpb, nvb); };
-  const cudaError_t e = cfg.blockDim.x <= 512 ? go(k_bicgstab_resident<true, 512, 14>, k_bicgstab_resident<false, 512, 14>)
-                                              : go(k_bicgstab_resident<true, 1024, 0>, k_bicgstab_resident<false, 1024, 0>);
+  // RAW while an SM has one group of rows: 40^2 / 60^2 / 80^2 particles (one, one, two groups) without and
+  // with it 1.21 / 2.79 / 2.60 and 1.16 / 2.72 / 2.65 ms
+  const cudaError_t e =
+      nonull && !a.warm && gpb == 1 ? cudaLaunchKernelEx(&cfg, k_bicgstab_resident<true, 512, 14, true>, a, gpb, nvb)
+      : cfg.blockDim.x <= 512       ? go(k_bicgstab_resident<true, 512, 14>, k_bicgstab_resident<false, 512, 14>)
+                                    : go(k_bicgstab_resident<true, 1024, 0>, k_bicgstab_resident<false, 1024, 0>);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return false;
