@@ -64,6 +64,11 @@ constexpr int MCO = 20;       // per-mirror coefficients: cu, ctheta, cv, (pad),
 constexpr int ATB = 1024;     // scan block
 
 // ------------------------------------------------------------------------- device helpers
+// The pair loops' products run beside the FP64 pipe that bounds them (vebi_fp64.cuh); the same bits.
+// A reversed step of 1M particles, on the FP64 pipe / now, ms: predictor rows 1.61 / 0.87 and gather 2.19 /
+// 1.33, right-hand side 0.77 / 0.42 and 0.92 / 0.58, gradients 0.78 / 0.42 and 0.74 / 0.48.
+using fp::mul_int;
+
 struct Tape {
   int nm = 0, kmax = 0;
   double dt = 0.0;
@@ -536,8 +541,8 @@ __global__ void k_adj_rhs_rows(Consts c, Tape t, AdjVec a) {
   for (int k = 0; k < cnt; ++k) {
     const size_t e = (size_t)k * c.npfb + i;
     const double w1 = t.wgx[e], w2 = t.wgy[e];
-    s1 += K11 * w1 + K12 * w2;
-    s2 += K21 * w1 + K22 * w2;
+    s1 += mul_int(K11, w1) + mul_int(K12, w2);
+    s2 += mul_int(K21, w1) + mul_int(K22, w2);
   }
   a.aus[i] += q * s1;  // d b_i / d u*_i = -(1/dt) sum kw
   a.avs[i] += q * s2;
@@ -552,8 +557,8 @@ __global__ void k_adj_gather_us(Consts c, Tape t, Trans T, AdjVec a, int np) {
     const size_t e = (size_t)k * c.npfb + i;
     const double w1 = t.wgx[e], w2 = t.wgy[e];
     const double qi = a.q[i];
-    gu -= qi * (t.kg[0][i] * w1 + t.kg[2][i] * w2);
-    gv -= qi * (t.kg[1][i] * w1 + t.kg[3][i] * w2);
+    gu -= mul_int(qi, mul_int(t.kg[0][i], w1) + mul_int(t.kg[2][i], w2));
+    gv -= mul_int(qi, mul_int(t.kg[1][i], w1) + mul_int(t.kg[3][i], w2));
   }
   if (cc < c.npfb) {
     a.aus[cc] += gu;
@@ -591,11 +596,12 @@ __global__ void k_adj_pred_rows(Consts c, Tape t, AdjVec a, int ve) {
       swl += t.wl[e];
       if (ve) {
         const double w1 = t.wgx[e], w2 = t.wgy[e];
-        const double kw1 = K11 * w1 + K12 * w2, kw2 = K21 * w1 + K22 * w2;
-        o0 -= cp * kw1 * s1;
-        o2 -= cp * kw2 * s1;
-        o1 -= cp * kw1 * s2;
-        o3 -= cp * kw2 * s2;
+        const double kw1 = mul_int(K11, w1) + mul_int(K12, w2), kw2 = mul_int(K21, w1) + mul_int(K22, w2);
+        const double ck1 = mul_int(cp, kw1), ck2 = mul_int(cp, kw2);
+        o0 -= mul_int(ck1, s1);
+        o2 -= mul_int(ck2, s1);
+        o1 -= mul_int(ck1, s2);
+        o3 -= mul_int(ck2, s2);
       }
     }
     a.Nu[i] += cs * s1 * swl;
@@ -617,16 +623,19 @@ __global__ void k_adj_gather_pred(Consts c, Tape t, Trans T, AdjVec a, int np, i
     const int i = en >> SLOT_BITS, k = en & ((1 << SLOT_BITS) - 1);
     const size_t e = (size_t)k * c.npfb + i;
     const double wl = t.wl[e], s1 = a.s1[i], s2 = a.s2[i];
-    gu -= cs * wl * s1;
-    gv -= cs * wl * s2;
-    gth -= ct * wl * a.st[i];
+    const double cw = mul_int(cs, wl);
+    gu -= mul_int(cw, s1);
+    gv -= mul_int(cw, s2);
+    gth -= mul_int(mul_int(ct, wl), a.st[i]);
     if (ve) {
       const double w1 = t.wgx[e], w2 = t.wgy[e];
-      const double kw1 = t.kg[0][i] * w1 + t.kg[2][i] * w2, kw2 = t.kg[1][i] * w1 + t.kg[3][i] * w2;
-      g0 += cp * kw1 * s1;
-      g2 += cp * kw2 * s1;
-      g1 += cp * kw1 * s2;
-      g3 += cp * kw2 * s2;
+      const double kw1 = mul_int(t.kg[0][i], w1) + mul_int(t.kg[2][i], w2);
+      const double kw2 = mul_int(t.kg[1][i], w1) + mul_int(t.kg[3][i], w2);
+      const double ck1 = mul_int(cp, kw1), ck2 = mul_int(cp, kw2);
+      g0 += mul_int(ck1, s1);
+      g2 += mul_int(ck2, s1);
+      g1 += mul_int(ck1, s2);
+      g3 += mul_int(ck2, s2);
     }
   }
   if (cc < c.npfb) {
@@ -716,8 +725,8 @@ __global__ void k_adj_grad_rows(Consts c, Tape t, AdjVec a) {
   for (int k = 0; k < cnt; ++k) {
     const size_t e = (size_t)k * c.npfb + i;
     const double w1 = t.wgx[e], w2 = t.wgy[e];
-    su += a0 * w1 + a1 * w2;
-    sv += a2 * w1 + a3 * w2;
+    su += mul_int(a0, w1) + mul_int(a1, w2);
+    sv += mul_int(a2, w1) + mul_int(a3, w2);
   }
   a.Nu[i] -= su;
   a.Nv[i] -= sv;
@@ -731,8 +740,8 @@ __global__ void k_adj_gather_grad(Consts c, Tape t, Trans T, AdjVec a, int np) {
     const int i = en >> SLOT_BITS, k = en & ((1 << SLOT_BITS) - 1);
     const size_t e = (size_t)k * c.npfb + i;
     const double w1 = t.wgx[e], w2 = t.wgy[e];
-    gu += a.s1[i] * w1 + a.s2[i] * w2;
-    gv += a.st[i] * w1 + a.q[i] * w2;
+    gu += mul_int(a.s1[i], w1) + mul_int(a.s2[i], w2);
+    gv += mul_int(a.st[i], w1) + mul_int(a.q[i], w2);
   }
   if (cc < c.npfb) {
     a.Nu[cc] += gu;
