@@ -11,8 +11,8 @@ time block 0 spent working before it (the phase) and waiting in it (the slowest 
 lateness plus the barrier's own latency).  It also records every block's arrival at 64
 consecutive barriers, with the SM each block runs on.
 
-With L grid-wide coarse levels an iteration (closed domain) has 4L + 15 barriers, 31 at 4M
-(L = 4).  The phases, in order:
+With L grid-wide coarse levels an iteration (closed domain) has 4L + 15 barriers, 35 at 4M
+(L = 5).  The phases, in order:
   0 p update and its mean; 1 .. 2L+5 the V-cycle on p (1 mean removal + first sweep, 2 fine
   residual, 3 restriction to the cells, then per grid-wide level one fused residual+restriction
   phase, the one-block levels and the coarsest solve, per level one fused prolongation+smoothing
