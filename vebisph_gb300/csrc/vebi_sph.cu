@@ -122,7 +122,7 @@ __device__ __forceinline__ double negated(double x) {
 // of the partner's row for the slot waits in the shadow of the arithmetic.  A pair that one
 // particle alone lists (d.s->one_sided) is computed by that one.  Each lane first lists the slots
 // it computes, so that all lanes of a warp compute in every round.  P lanes share a row when the
-// // rows alone would not fill the GPU.
+// rows alone would not fill the GPU.
 // What bounds it: the issue of ~1000 integer and FP32 instructions a pair, with the FP64 pipe at 40%.
 // Measured with k_weight_sums at 4M / 250k / 20k / 1.7k particles: 12.6 / 1.08 / 0.15 / 0.08 ms, where
 // a kernel each for the weights and the shifting, all pairs from both sides in FP64 instructions,
