@@ -304,8 +304,7 @@ __global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, 
   const bool mine = i < n;
   double* const pinv_all = a.scratch + NA_CTRL;
   double* const sinv_all = pinv_all + VEBI_NOALLOC_MAX_ROWS;
-  double* const part0 = sinv_all + VEBI_NOALLOC_MAX_ROWS;
-  double* const part1 = part0 + 2 * (size_t)nvb * RES_VB;  // used in turn: a slow block may still read one
+  double* const parts = sinv_all + VEBI_NOALLOC_MAX_ROWS;
   const double small = NONULL ? 1.0e-6 : 4.0, dn = (double)n;
   double* const vals = na_mat + t;
   int* const cols = reinterpret_cast<int*>(na_mat + (size_t)keep * R) + t;
@@ -314,10 +313,7 @@ __global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, 
     vals[k * R] = a.val[(size_t)k * a.stride + i];
     cols[k * R] = a.col[(size_t)k * a.stride + i];
   }
-  if (t == 0) {
-    sh.alpha = sh.omega = sh.n2r0 = sh.n2s0 = 1.0;
-    sh.beta = sh.n2 = 0.0;
-  }
+  res_begin(sh);
   const double di = mine ? a.diag[i] : 0.0;
   const double den = NONULL ? (1.0 + 1.0e-15) : (di + 1.0e-15), rden = fp::reciprocal(fp::magnitude(den));
   const double rdn = fp::reciprocal(dn);
@@ -358,7 +354,7 @@ __global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, 
   auto failed = [&]() {
     if (mine) a.x[i] = nan;
   };
-  if (!res_reduce<1>(bar, mine ? plus_zero(r * r) : 0.0, 0.0, part1, gpb, nvb, sh, [&]() { sh.rho = sh.v[0]; }))
+  if (!res_reduce<1>(bar, mine ? plus_zero(r * r) : 0.0, 0.0, parts, gpb, nvb, sh, [&]() { sh.rho = sh.v[0]; }))
     return failed();
   int iter = 1, warn = 0;
   bool done = false, at_s = false;
@@ -366,7 +362,7 @@ __global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, 
     if (is_zero(sh.rho)) { warn |= VEBI_WARN_BICGSTAB_BREAKDOWN; done = true; break; }
     p = iter == 1 ? r : r + sh.beta * (p - sh.omega * v);
     if (NONULL) {
-      if (!res_reduce<1>(bar, mine ? plus_zero(p) : 0.0, 0.0, part0, gpb, nvb, sh, [&]() { sh.mean = fp::quotient(sh.v[0], dn, rdn); }))
+      if (!res_reduce<1>(bar, mine ? plus_zero(p) : 0.0, 0.0, parts, gpb, nvb, sh, [&]() { sh.mean = fp::quotient(sh.v[0], dn, rdn); }))
         return failed();
       p = p - sh.mean;
     }
@@ -374,7 +370,7 @@ __global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, 
     if (mine) pinv_all[i] = pinv;
     if (!res_sync(bar)) return failed();
     v = product(pinv_all);
-    if (!res_reduce<1>(bar, mine ? plus_zero(rb * v) : 0.0, 0.0, part1, gpb, nvb, sh,
+    if (!res_reduce<1>(bar, mine ? plus_zero(rb * v) : 0.0, 0.0, parts, gpb, nvb, sh,
                        [&]() { sh.alpha = fp::quotient(sh.rho, sh.v[0] + 1.0e-15); }))
       return failed();
     const double alpha = sh.alpha;
@@ -383,7 +379,7 @@ __global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, 
       sinv = fp::quotient(s, den, rden);
       if (mine) sinv_all[i] = sinv;
     }
-    if (!res_reduce<2>(bar, mine ? plus_zero(s * s) : 0.0, mine ? plus_zero(s) : 0.0, part0, gpb, nvb, sh, [&]() {
+    if (!res_reduce<2>(bar, mine ? plus_zero(s * s) : 0.0, mine ? plus_zero(s) : 0.0, parts, gpb, nvb, sh, [&]() {
           sh.n2 = sh.v[0];
           if (iter == 1) sh.n2s0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
           sh.flag = sh.v[0] <= a.tol * a.tol * sh.n2s0;
@@ -402,13 +398,13 @@ __global__ void __launch_bounds__(NA_T_MAX, 1) k_na_resident(NaArgs a, int gpb, 
       if (!res_sync(bar)) return failed();
     }
     const double tv = product(sinv_all);
-    if (!res_reduce<2>(bar, mine ? plus_zero(tv * s) : 0.0, mine ? plus_zero(tv * tv) : 0.0, part1, gpb, nvb, sh,
+    if (!res_reduce<2>(bar, mine ? plus_zero(tv * s) : 0.0, mine ? plus_zero(tv * tv) : 0.0, parts, gpb, nvb, sh,
                        [&]() { sh.omega = fp::quotient(sh.v[0], sh.v[1] + 1.0e-15); }))
       return failed();
     const double omega = sh.omega;
     x = x + alpha * pinv + omega * sinv;
     r = s - omega * tv;
-    if (!res_reduce<2>(bar, mine ? plus_zero(r * r) : 0.0, mine ? plus_zero(rb * r) : 0.0, part0, gpb, nvb, sh, [&]() {
+    if (!res_reduce<2>(bar, mine ? plus_zero(r * r) : 0.0, mine ? plus_zero(rb * r) : 0.0, parts, gpb, nvb, sh, [&]() {
           sh.n2 = sh.v[0];
           if (iter == 1) sh.n2r0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
           sh.flag = sh.v[0] <= a.tol * a.tol * sh.n2r0;

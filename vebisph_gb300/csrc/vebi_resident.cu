@@ -80,12 +80,7 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
   const double rinv1 = 1.0 / (1.0 + 1.0e-15);
   const double small = NONULL ? 1.0e-6 : 4.0;  // open solver: the integer expression 10-6
   const double dn = (double)n, rdn = fp::reciprocal(dn), tol2 = a.tol * a.tol;
-  double* const part0 = a.part;
-  double* const part1 = a.part + 2 * (size_t)nvb * RES_VB;  // used in turn: a slow block may still read one
-  if (t == 0) {
-    sh.alpha = sh.omega = sh.n2r0 = sh.n2s0 = 1.0;
-    sh.beta = sh.n2 = 0.0;
-  }
+  res_begin(sh);
   // this thread's row in the vector passes
   const int i = row0 + t;
   const bool mine = t < R && i < n;
@@ -147,7 +142,7 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
   }
   rb = r;
   if (!NONULL && mine) rinvM = 1.0 / (__ldg(a.diag + i) + 1.0e-15);
-  if (!res_reduce<1>(bar, mine ? fma(r, r, 0.0) : 0.0, 0.0, part1, gpb, nvb, sh, [&]() { sh.rho = sh.v[0]; })) return;
+  if (!res_reduce<1>(bar, mine ? fma(r, r, 0.0) : 0.0, 0.0, a.part, gpb, nvb, sh, [&]() { sh.rho = sh.v[0]; })) return;
   int iter = 1, warn = 0;
   bool done = false, at_s = false;
   while (iter <= a.itermax) {
@@ -155,7 +150,7 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
     if (mine) p = iter == 1 ? r : fma(sh.beta, fma(-sh.omega, v, p), r);
     if (RAW && mine) a.pinv[i] = p;
     if (NONULL) {
-      if (!res_reduce<1>(bar, mine ? plus_zero(p) : 0.0, 0.0, part0, gpb, nvb, sh, [&]() { sh.mean = fp::quotient(sh.v[0], dn, rdn); }))
+      if (!res_reduce<1>(bar, mine ? plus_zero(p) : 0.0, 0.0, a.part, gpb, nvb, sh, [&]() { sh.mean = fp::quotient(sh.v[0], dn, rdn); }))
         return;
       p = p - sh.mean;
     }
@@ -165,13 +160,13 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
       if (!grid_sync(s)) return;
     }
     v = product(a.pinv, sh.mean);
-    if (!res_reduce<1>(bar, mine ? fma(rb, v, 0.0) : 0.0, 0.0, part1, gpb, nvb, sh,
+    if (!res_reduce<1>(bar, mine ? fma(rb, v, 0.0) : 0.0, 0.0, a.part, gpb, nvb, sh,
                        [&]() { sh.alpha = fp::quotient(sh.rho, sh.v[0] + 1.0e-15); }))
       return;
     const double alpha = sh.alpha;
     double sv = mine ? fma(-alpha, v, r) : 0.0;
     if (EARLY && mine) a.sinv[i] = NONULL ? sv : sv * rinvM;
-    if (!res_reduce<2>(bar, mine ? fma(sv, sv, 0.0) : 0.0, mine ? plus_zero(sv) : 0.0, part0, gpb, nvb, sh, [&]() {
+    if (!res_reduce<2>(bar, mine ? fma(sv, sv, 0.0) : 0.0, mine ? plus_zero(sv) : 0.0, a.part, gpb, nvb, sh, [&]() {
           sh.n2 = sh.v[0];
           if (iter == 1) sh.n2s0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
           sh.flag = sh.v[0] <= tol2 * sh.n2s0;
@@ -190,13 +185,13 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
       if (!grid_sync(s)) return;
     }
     const double tv = product(a.sinv, sh.mean);
-    if (!res_reduce<2>(bar, mine ? fma(tv, sv, 0.0) : 0.0, mine ? fma(tv, tv, 0.0) : 0.0, part1, gpb, nvb, sh,
+    if (!res_reduce<2>(bar, mine ? fma(tv, sv, 0.0) : 0.0, mine ? fma(tv, tv, 0.0) : 0.0, a.part, gpb, nvb, sh,
                        [&]() { sh.omega = fp::quotient(sh.v[0], sh.v[1] + 1.0e-15); }))
       return;
     const double omega = sh.omega;
     x = fma(omega, sinv, fma(alpha, pinv, x));
     r = fma(-omega, tv, sv);
-    if (!res_reduce<2>(bar, mine ? fma(r, r, 0.0) : 0.0, mine ? fma(rb, r, 0.0) : 0.0, part0, gpb, nvb, sh, [&]() {
+    if (!res_reduce<2>(bar, mine ? fma(r, r, 0.0) : 0.0, mine ? fma(rb, r, 0.0) : 0.0, a.part, gpb, nvb, sh, [&]() {
           sh.n2 = sh.v[0];
           if (iter == 1) sh.n2r0 = (sh.v[0] <= small) ? 1.0 : sh.v[0];
           sh.flag = sh.v[0] <= tol2 * sh.n2r0;
@@ -219,7 +214,7 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
 
 }  // namespace
 
-// doubles of partial sums the resident solver needs for n rows
+// doubles of partial sums the resident solver needs for n rows: two areas of two sums a group
 size_t resident_partials(int n) { return 4 * (size_t)RES_VB * ((n + 255) / 256); }
 
 // Runs the solve when it fits: at most 256 rows (eight groups, four lanes a row) per SM, and a

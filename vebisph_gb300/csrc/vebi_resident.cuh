@@ -18,15 +18,34 @@ struct ResSh {
   double vb[2 * RES_MAX_VB]; // virtual-block sums
   double v[2];
   double rho, alpha, omega, beta, n2r0, n2s0, n2, mean;
-  int flag;
+  int flag, turn;
 };
 
+// every resident solver's first statement
+__device__ __forceinline__ void res_begin(ResSh& sh) {
+  if (threadIdx.x == 0) {
+    sh.alpha = sh.omega = sh.n2r0 = sh.n2s0 = 1.0;
+    sh.beta = sh.n2 = 0.0;
+    sh.turn = 0;
+  }
+  __syncthreads();
+}
+
 // the grid-wide sums of a and (NV = 2) b over all rows, a barrier among them: for thread 0 the
-// totals are in sh.v when this returns true
+// totals are in sh.v when this returns true.
+// The partial sums go to one of two areas of `parts`, each reduction to the one that the last did not
+// take.  A reduction writes its area before its barrier and reads it after, and a block that has read
+// goes on to the next reduction's writes while a slower one still reads: those two must not share an
+// area.  Two are enough, as a block writes an area again only past the barrier of the reduction between,
+// at which every block arrives after its reads.  The turn is kept here and not written into the solvers:
+// a closed domain's iteration has five reductions, so areas fixed per reduction would give its last and
+// the next iteration's first the same one.
 template <int NV>
-static __device__ __noinline__ bool res_sums(GridBar bar, double a, double b, double* part, int gpb, int nvb, ResSh& sh) {
+static __device__ __noinline__ bool res_sums(GridBar bar, double a, double b, double* parts, int gpb, int nvb, ResSh& sh) {
   const int t = threadIdx.x, w = t >> 5, lane = t & 31;
   const int G = nvb * RES_VB, g0 = blockIdx.x * gpb;
+  const int turn = sh.turn;
+  double* const part = parts + turn * 2 * G;
   if (w < gpb) {
     double z;
     if (NV == 1) {
@@ -43,7 +62,10 @@ static __device__ __noinline__ bool res_sums(GridBar bar, double a, double b, do
   }
   __syncthreads();
   int bad = 0;
-  if (t == 0) bad = barrier_arrive_wait(bar.count, bar.error, SPIN_LIMIT) ? 0 : 1;
+  if (t == 0) {
+    sh.turn = turn ^ 1;
+    bad = barrier_arrive_wait(bar.count, bar.error, SPIN_LIMIT) ? 0 : 1;
+  }
   if (__syncthreads_or(bad)) return false;
   auto vb_sum = [&](int q, int vb) {  // a virtual block's eight group sums in sequence
     const double2* p = reinterpret_cast<const double2*>(part + (size_t)q * G + (size_t)vb * RES_VB);
@@ -85,9 +107,9 @@ __device__ __forceinline__ bool res_sync(GridBar bar) {
 
 // grid_reduce over the resident layout: post() runs on thread 0 with the sums in sh.v
 template <int NV, class Post>
-__device__ __forceinline__ bool res_reduce(GridBar bar, double a, double b, double* part, int gpb, int nvb, ResSh& sh,
+__device__ __forceinline__ bool res_reduce(GridBar bar, double a, double b, double* parts, int gpb, int nvb, ResSh& sh,
                                            Post post) {
-  if (!res_sums<NV>(bar, a, b, part, gpb, nvb, sh)) return false;
+  if (!res_sums<NV>(bar, a, b, parts, gpb, nvb, sh)) return false;
   if (threadIdx.x == 0) post();
   __syncthreads();
   return true;

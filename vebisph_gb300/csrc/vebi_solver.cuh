@@ -56,6 +56,7 @@ __device__ __forceinline__ void bar_mark(unsigned long long ts_arrive) {
 #endif
 
 // ---- words that blocks of the grid signal each other through (gpu scope)
+#ifdef __CUDACC__
 __device__ __forceinline__ unsigned int atom_add_release(unsigned int* a, unsigned int v) {
   unsigned int old;
   asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(a), "r"(v) : "memory");
@@ -66,6 +67,10 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* a) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
   return v;
 }
+#else  // the emulation's that runs these kernels on the CPU
+unsigned int atom_add_release(unsigned int* a, unsigned int v);
+unsigned int ld_acquire(const unsigned int* a);
+#endif
 
 // Poll *word until done(value); false when more than `limit` polls go by (VEBI_ERR_TIMEOUT is
 // recorded) or another block has recorded an error, looked at every 64th poll.  A poll is one
