@@ -262,11 +262,12 @@ class BatchSolver:
         for inst in self.instances:
             inst.set_coarse_block_rows(rows)
 
-    def autotune(self, candidates=(1, 2, 4, 8), coarse_candidates=(2048,)) -> dict:
+    def autotune(self, candidates=(1, 2, 4, 8), coarse_candidates=(512,)) -> dict:
         """Pick the batch's solver tiles by measurement: the rows each solver thread owns (so
         the rows per block and the blocks per instance) and, with the multigrid preconditioner,
         the size up to which coarse levels run in one block.  Every pair of candidates costs one
-        step to capture the graphs and one timed step (real steps of the simulations).  The rows
+        step to capture the graphs and one timed step (real steps of the simulations).  Unless
+        others are given, the coarse-level size stays the library's default (MG_BLOCK_ROWS).  The rows
         per thread set the solver's block count and so the order of its block-partial sums
         (results move by rounding); the coarse-level size leaves results unchanged."""
         times = {}
