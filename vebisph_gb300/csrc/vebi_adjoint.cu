@@ -1252,11 +1252,13 @@ int vebi_adjoint_create(vebi_ctx* ctx, int32_t max_steps, int32_t checkpoint_eve
 
 int vebi_adjoint_record(vebi_adjoint* a, int32_t nsteps, vebi_step_stats* last) {
   if (!a) return vebi::afail(VEBI_ERR_ARG, "adjoint: null handle");
+  const vebi::Stepping call(a->a->x->device);
   return vebi::adjoint_record(*a->a, nsteps, last);
 }
 
 int vebi_adjoint_replay(vebi_adjoint* a, int32_t nsteps, vebi_step_stats* last) {
   if (!a) return vebi::afail(VEBI_ERR_ARG, "adjoint: null handle");
+  const vebi::Stepping call(a->a->x->device);
   return vebi::adjoint_replay(*a->a, nsteps, last);
 }
 
@@ -1269,6 +1271,7 @@ int vebi_adjoint_reverse(vebi_adjoint* a, const double* seed_u, const double* se
                          int32_t ld, double* grad_u, double* grad_theta, double* grad_tau, double* grad_wi,
                          int32_t* ls_iters) {
   if (!a) return vebi::afail(VEBI_ERR_ARG, "adjoint: null handle");
+  const vebi::Stepping call(a->a->x->device);
   return vebi::adjoint_reverse(*a->a, seed_u, seed_theta, seed_tau, ld, grad_u, grad_theta, grad_tau, grad_wi,
                                ls_iters);
 }

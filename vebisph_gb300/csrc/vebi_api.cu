@@ -458,12 +458,13 @@ static void enqueue_step(Ctx& x, int secondary) {
   launch_final(x, secondary);
 }
 
-// Capture one step (without the dump-time diagnostic) into a CUDA graph, once per context and
-// timing mode; later steps replay it with one launch.  Every kernel argument of a step is the
+// Capture one step (without the dump-time diagnostic) into a CUDA graph, once per context, timing
+// mode and, where its solver depends on it, with and without company on the GPU; later steps replay it with one launch.  Every kernel argument of a step is the
 // same from step to step (counts live in device memory), so one capture serves all steps.
 // If capture is not possible the step is launched kernel by kernel instead.
+static int graph_index(const Ctx& x) { return (x.timing ? 1 : 0) + (!x.alone && resident_by_company(x) ? 2 : 0); }
 static bool graph_ready(Ctx& x) {
-  const int m = x.timing ? 1 : 0;
+  const int m = graph_index(x);
   if (x.graph[m]) return true;
   if (x.graph_failed[m]) return false;
   cudaGraph_t g = nullptr;
@@ -495,8 +496,9 @@ static bool graph_ready(Ctx& x) {
 
 // enqueue one step: the captured graph when possible, else kernel by kernel
 static void launch_step(Ctx& x, int secondary) {
+  x.alone = stepping_alone(x.device);
   if (!secondary && graph_ready(x)) {
-    const int m = x.timing ? 1 : 0;
+    const int m = graph_index(x);
     cudaGraphLaunch(x.graph[m], x.st);
     x.launches += x.graph_launches[m];
     for (int q = 0; q < VEBI_NSTAGES; ++q) x.ev_used[q] = x.graph_used[m][q];
@@ -513,6 +515,7 @@ int vebi_step(vebi_ctx* h, double x_mint, double y_mint, double x_maxt, double y
   if (!x.have_state) return fail(VEBI_ERR_ARG, "no state uploaded");
   if (x_mint != x.c.x_mint || x_maxt != x.c.x_maxt || y_mint != x.c.y_mint || y_maxt != x.c.y_maxt)
     return fail(VEBI_ERR_ARG, "domain box differs from the one the context was created with");
+  const Stepping call(x.device);
   x.launches = 0;
   launch_step(x, secondary);
   return finish_step(x, stats, true);
@@ -525,6 +528,7 @@ int vebi_run_steps(vebi_ctx* h, double x_mint, double y_mint, double x_maxt, dou
   if (!x.have_state) return fail(VEBI_ERR_ARG, "no state uploaded");
   if (x_mint != x.c.x_mint || x_maxt != x.c.x_maxt || y_mint != x.c.y_mint || y_maxt != x.c.y_maxt)
     return fail(VEBI_ERR_ARG, "domain box differs from the one the context was created with");
+  const Stepping call(x.device);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -644,7 +648,7 @@ int vebi_set_solver_grid(vebi_ctx* h, int32_t rows_per_thread) {
   cudaStreamSynchronize(x.st);
   x.solver_rows_per_thread = rows_per_thread;
   ++x.grid_gen;
-  for (int m = 0; m < 2; ++m) {  // the captured steps hold the old grid
+  for (int m = 0; m < 4; ++m) {  // the captured steps hold the old grid
     if (x.graph[m]) cudaGraphExecDestroy(x.graph[m]);
     x.graph[m] = nullptr;
     x.graph_failed[m] = false;
@@ -659,7 +663,7 @@ int vebi_set_coarse_block_rows(vebi_ctx* h, int32_t rows) {
   cudaStreamSynchronize(x.st);
   x.mg_block_rows = rows;
   ++x.grid_gen;
-  for (int m = 0; m < 2; ++m) {  // the captured steps hold the old launch arguments
+  for (int m = 0; m < 4; ++m) {  // the captured steps hold the old launch arguments
     if (x.graph[m]) cudaGraphExecDestroy(x.graph[m]);
     x.graph[m] = nullptr;
     x.graph_failed[m] = false;
@@ -677,7 +681,7 @@ int vebi_set_weissenberg(vebi_ctx* h, double wi) {
   x.c.Wi = P.El * std::sqrt(P.Ra / P.Pr);
   x.c.coeff_polymeric = (1.0 - P.beta) * P.Pr / (P.Ra * P.El);
   ++x.grid_gen;
-  for (int m = 0; m < 2; ++m) {  // the captured steps hold the old constants
+  for (int m = 0; m < 4; ++m) {  // the captured steps hold the old constants
     if (x.graph[m]) cudaGraphExecDestroy(x.graph[m]);
     x.graph[m] = nullptr;
     x.graph_failed[m] = false;
@@ -692,7 +696,7 @@ int vebi_set_velocity_limit(vebi_ctx* h, double u_limit) {
   cudaStreamSynchronize(x.st);
   x.c.u_limit = u_limit;
   ++x.grid_gen;
-  for (int m = 0; m < 2; ++m) {  // the captured steps hold the old constants
+  for (int m = 0; m < 4; ++m) {  // the captured steps hold the old constants
     if (x.graph[m]) cudaGraphExecDestroy(x.graph[m]);
     x.graph[m] = nullptr;
     x.graph_failed[m] = false;
@@ -827,6 +831,7 @@ int vebi_batch_step(vebi_batch* b, int32_t nsteps, double* ms, vebi_step_stats* 
     Ctx& x = b->ctx[i]->x;
     if (!x.have_state) return fail(VEBI_ERR_ARG, "batch instance without state");
   }
+  const Stepping call(b->ctx[0]->x.device);
   const bool graph = batch_graph_ready(b);
   cudaStream_t s0 = b->ctx[0]->x.st;
   // every instance's pending work (uploads) is ordered before the batch; the whole batch
@@ -1003,6 +1008,7 @@ int vebi_debug_get(vebi_ctx* h, const char* name, void* out, int64_t bytes) {
 
 namespace vebi {
 int run_one_step(Ctx& x, vebi_step_stats* stats) {
+  x.alone = stepping_alone(x.device);
   x.launches = 0;
   enqueue_step(x, 0);
   if (x.timing) cudaEventRecord(x.ev[VEBI_NSTAGES], x.st);

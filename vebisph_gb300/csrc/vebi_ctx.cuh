@@ -25,13 +25,15 @@ struct Ctx {
   cudaEvent_t* ev_run = nullptr;   // per-step stage events of vebi_run_steps (timing on)
   int ev_run_step = -1;            // step whose events stage_mark records, -1 = use ev[]
   bool capturing = false;          // enqueue_step is being captured into a CUDA graph
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one step: [0] plain, [1] with stage events
-  bool graph_failed[2] = {false, false};
-  int graph_launches[2] = {0, 0};
-  bool graph_used[2][VEBI_NSTAGES] = {};
+  // one step: [0] plain, [1] with stage events; [2], [3] the same in company (resident_by_company)
+  cudaGraphExec_t graph[4] = {};
+  bool graph_failed[4] = {};
+  int graph_launches[4] = {};
+  bool graph_used[4][VEBI_NSTAGES] = {};
   int coop_blocks = 0;       // persistent PPE grid (co-resident blocks)
   int coop_blocks_mixed = 0; // same for the mixed-precision solver
   bool in_batch = false;     // one of a batch's instances: its solver leaves room on the SMs for the others'
+  bool alone = true;         // no other host call was stepping a context on this GPU when the step was launched
   int solver_rows_per_thread = 1;  // batch tuning: rows per solver thread
   int mg_block_rows = MG_BLOCK_ROWS;  // batch tuning: coarse levels of at most this many rows run in one block
   int grid_gen = 0;                // bumped when a launch shape changes (captured graphs are stale)
@@ -75,6 +77,16 @@ Ctx* ctx_of(vebi_ctx* h);
 struct BiArgs;
 size_t resident_partials(int n);
 bool launch_bicgstab_resident(Ctx& x, const BiArgs& a, bool nonull);
+bool resident_by_company(const Ctx& x);
+
+// a host call that steps contexts on a GPU, from before its first launch until its work is done
+struct Stepping {
+  const int device;
+  explicit Stepping(int device);
+  ~Stepping();
+  Stepping(const Stepping&) = delete;
+};
+bool stepping_alone(int device);  // asked from within such a call
 
 // kernel launch with launch accounting and an immediate launch-error check
 #define VEBI_LAUNCH(x, kern, grid, block, ...)                         \

@@ -460,7 +460,7 @@ void launch_ppe_mg(Ctx& x);
 void launch_ppe_rhs32(Ctx& x);
 
 // The FP64 solve on its grid: the resident kernel where it fits (one row per thread, outside a
-// batch, whose instances' solves share the SMs), else the persistent kernel, as a cooperative
+// batch, whose instances' solves share the SMs, and not beside other contexts' steps), else the persistent kernel, as a cooperative
 // launch (all blocks co-resident, so the grid barrier is safe).
 static void launch_bicgstab(Ctx& x, const BiArgs& a, bool nonull, int rows_per_thread) {
   if (rows_per_thread == 1 && !x.in_batch && launch_bicgstab_resident(x, a, nonull)) return;
@@ -519,7 +519,10 @@ void launch_ppe(Ctx& x) {
 
 // The persistent FP64 BiCGSTAB on a caller's system (the adjoint's transposed PPE): the same
 // grid and kernels as the step's solve, other arrays.
-void launch_bicgstab_on(Ctx& x, const BiArgs& a, bool nonull) { launch_bicgstab(x, a, nonull, 1); }
+void launch_bicgstab_on(Ctx& x, const BiArgs& a, bool nonull) {
+  x.alone = stepping_alone(x.device);
+  launch_bicgstab(x, a, nonull, 1);
+}
 
 
 }  // namespace vebi

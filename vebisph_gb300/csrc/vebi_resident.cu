@@ -23,6 +23,8 @@
 // dependent adds (0.6-1 us with their load), six quotients of ~0.2 us, two products' gathers.
 // Measured, ms per solve, k_bicgstab / this kernel: 1.7k rows x 60 iterations 2.39 / 1.16, 2.9k x
 // 75 (open) 2.48 / 1.25, 10k x 139 5.37 / 3.36, 20k x 363 14.9 / 12.0, 29k x 247 10.2 / 9.7.
+#include <atomic>
+
 #include "vebi_resident.cuh"
 
 namespace vebi {
@@ -217,15 +219,47 @@ __global__ void __launch_bounds__(T_MAX, 1) k_bicgstab_resident(BiArgs a, int gp
 // doubles of partial sums the resident solver needs for n rows: two areas of two sums a group
 size_t resident_partials(int n) { return 4 * (size_t)RES_VB * ((n + 255) / 256); }
 
-// Runs the solve when it fits: at most 256 rows (eight groups, four lanes a row) per SM, and a
-// caller whose k_bicgstab grid has one row per thread (ceil(n / 256) blocks, whose summation order
-// this kernel keeps).  false: not launched.  Above 256 rows an SM the FP64 pipe is busy either way:
-// 60k / 100k rows with two rows or one lane a row took 33 / 47 ms against k_bicgstab's 32 / 48.
-bool launch_bicgstab_resident(Ctx& x, const BiArgs& a, bool nonull) {
-  const int nvb = (a.n + TPB - 1) / TPB;
-  if (nvb > x.coop_blocks || nvb > RES_MAX_VB) return false;
+namespace {
+
+// groups of rows per SM, or 0 when the solve does not fit: at most 256 rows (eight groups, four lanes a
+// row) per SM, and a caller whose k_bicgstab grid has one row per thread (ceil(n / 256) blocks, whose
+// summation order this kernel keeps).  Above 256 rows an SM the FP64 pipe is busy either way: 60k /
+// 100k rows with two rows or one lane a row took 33 / 47 ms against k_bicgstab's 32 / 48.
+int resident_groups(const Ctx& x, int n) {
+  const int nvb = (n + TPB - 1) / TPB;
+  if (nvb > x.coop_blocks || nvb > RES_MAX_VB) return 0;
   const int gpb = (nvb * RES_VB + x.nsm - 1) / x.nsm;
-  if (gpb * RES_GROUP > RES_MAX_ROWS) return false;
+  return gpb * RES_GROUP <= RES_MAX_ROWS ? gpb : 0;
+}
+
+// From two groups per SM on, one spread solve fills the register files, so those of several contexts
+// that host threads step at the same time follow one another; k_bicgstab takes few SMs and overlaps.
+// So a spread solve of that size is for a call that has the GPU to itself.  Steps per second of 1 / 2 /
+// 4 / 8 / 16 contexts with a thread each, spread / k_bicgstab: 10k rows 255 / 295 / 289 / 293 / 294 and
+// 193 / 381 / 653 / 1037 / 1363, 20k 149 / 156 / 156 / 156 / 155 and 135 / 243 / 371 / 475 / 503; one
+// group per SM, 1.7k rows, 718 / 1360 / 2459 / 4104 / 5108 and 465 / 893 / 1752 / 3377 / 6259.  The bits
+// are the same either way.
+bool by_company(int gpb) { return gpb > 1; }
+
+std::atomic<int> g_stepping[64];  // calls in progress by device
+std::atomic<int>& stepping(int device) { return g_stepping[device < 64 ? device : 63]; }
+
+}  // namespace
+
+Stepping::Stepping(int device_) : device(device_) { ++stepping(device); }
+Stepping::~Stepping() { --stepping(device); }
+bool stepping_alone(int device) { return stepping(device) <= 1; }
+
+// whether the kernel of x's solve depends on x.alone, and so the captured step does
+bool resident_by_company(const Ctx& x) {
+  return x.precision == VEBI_PREC_FP64 && x.c.precond == 0 && !x.in_batch && x.solver_rows_per_thread <= 1 &&
+         by_company(resident_groups(x, x.c.npfb));
+}
+
+// Runs the solve when it fits and the GPU is free for it.  false: not launched.
+bool launch_bicgstab_resident(Ctx& x, const BiArgs& a, bool nonull) {
+  const int gpb = resident_groups(x, a.n), nvb = (a.n + TPB - 1) / TPB;
+  if (!gpb || (by_company(gpb) && !x.alone)) return false;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((nvb * RES_VB + gpb - 1) / gpb);
   cfg.blockDim = dim3(4 * gpb * RES_GROUP);
