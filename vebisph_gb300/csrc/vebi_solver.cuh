@@ -6,7 +6,9 @@
 
 namespace vebi {
 
-constexpr unsigned long long SPIN_LIMIT = 1ull << 25;  // ~2-4 s of __nanosleep(64) polls
+// polls of a grid barrier before it gives up: 1.9 to 2.1 s with 64 to 2 blocks on an idle GPU (a poll takes
+// 0.22 to 0.25 us, measured), longer beside other traffic to L2
+constexpr unsigned long long SPIN_LIMIT = 1ull << 23;
 
 #ifdef VEBI_BARRIER_TIMESTAMPS
 // Diagnostic build only (vebisph_gb300/barrier_profile.py): block 0 records the global timer
@@ -74,7 +76,7 @@ unsigned int ld_acquire(const unsigned int* a);
 
 // Poll *word until done(value); false when more than `limit` polls go by (VEBI_ERR_TIMEOUT is
 // recorded) or another block has recorded an error, looked at every 64th poll.  A poll is one
-// round trip to L2 (~0.5 us on GB300), so sleeping between polls only adds to the wait.
+// round trip to L2 (0.22-0.25 us), so sleeping between polls only adds to the wait.
 template <class Done>
 __device__ __forceinline__ bool poll_bounded(const unsigned int* word, int* error, unsigned long long limit, Done done) {
   for (unsigned long long spins = 0;; ++spins) {
