@@ -245,6 +245,18 @@ template <class T> T __shfl_down_sync(unsigned, T v, int d, int w = 32) {
   const int l = emu::lane(), in = (l & (w - 1)) + d;
   return emu::shuffle(v, in < w ? l + d : l);
 }
+template <class T> T __shfl_up_sync(unsigned, T v, int d) {
+  const int l = emu::lane();
+  return emu::shuffle(v, l >= d ? l - d : l);
+}
+inline unsigned __ballot_sync(unsigned, bool p) {
+  unsigned b = p ? 1u << emu::lane() : 0u;
+  for (int o = 16; o > 0; o >>= 1) b |= emu::shuffle(b, emu::lane() ^ o);
+  return b;
+}
+inline bool __any_sync(unsigned m, bool p) { return __ballot_sync(m, p) != 0u; }
+inline int __popc(unsigned v) { return __builtin_popcount(v); }
+inline int __ffs(int v) { return __builtin_ffs(v); }
 inline int __reduce_max_sync(unsigned, int v) {
   int r = v;
   for (int o = 16; o > 0; o >>= 1) r = std::max(r, emu::shuffle(r, emu::lane() ^ o));
@@ -261,6 +273,7 @@ template <class T, class C, class V> T atomicCAS(T* a, C c, V v) { T o = *a; if 
 template <class T> T __ldg(const T* p) { return *p; }
 template <class T> T __ldca(const T* p) { return *p; }
 template <class T> T __ldcg(const T* p) { return *p; }
+using std::isnan;
 using std::max;
 using std::min;
 
