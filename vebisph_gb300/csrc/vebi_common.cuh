@@ -170,24 +170,8 @@ struct Dev {
 
 // ---------------------------------------------------------------------------------------------
 // small helpers
-__device__ __forceinline__ double pw4(double x) { double x2 = x * x; return x2 * x2; }
 __device__ __forceinline__ double pw5(double x) { double x2 = x * x; double x3 = x * x2; return x2 * x3; }
 
-// quintic spline derivative `fac` (sphtools.F90:11-44)
-__device__ __forceinline__ double fac(const Consts& c, double qq) {
-  int isel = (int)floor(qq);
-  if (isel == 0) {
-    double q3 = 3.0 - qq, q2 = 2.0 - qq, q1 = 1.0 - qq;
-    return c.ad_7h * (-5.0 * pw4(q3) + 30.0 * pw4(q2) - 75.0 * pw4(q1));
-  } else if (isel == 1) {
-    double q3 = 3.0 - qq, q2 = 2.0 - qq;
-    return c.ad_7h * (-5.0 * pw4(q3) + 30.0 * pw4(q2));
-  } else if (isel == 2) {
-    double q3 = 3.0 - qq;
-    return c.ad_7h * (-5.0 * pw4(q3));
-  }
-  return 0.0;
-}
 // quintic spline `Wab` (sphtools.F90:46-76)
 __device__ __forceinline__ double wab(const Consts& c, double qq) {
   int isel = (int)floor(qq);
