@@ -11,10 +11,14 @@ namespace vebi {
 
 constexpr int LANES = 8;       // lanes a row
 constexpr int LANES_TPB = 64;  // threads a block: small blocks spread a small domain over the SMs
-// Rows up to which eight lanes take a row.  Measured, us, a thread / eight lanes a row, with 1.7k, 20k and
-// 60k rows: FP64 predictor 154 / 33, 176 / 86, 207 / 227; FP64 gradients 76 / 25, 84 / 47, 108 / 98;
-// FP32 weights (20k, 60k) 48 / 16, 46 / 33; shifting 41 / 21, 41 / 43; predictor 72 / 37, 84 / 76;
-// the pressure gradient, whose pairs are cheap, FP64 34 / 18 at 1.7k, 31 / 29 at 10k, 53 / 63 at 20k.
+// Rows up to which eight lanes take a row: one line for all kernels, between 20k, where every
+// one gains, and 60k, where the heaviest (the FP64 predictor) loses.  Measured, us, a thread / eight lanes
+// a row, with 1.7k, 20k and 60k rows: FP64 predictor 154 / 33, 176 / 86, 207 / 227; FP64 gradients
+// 76 / 25, 84 / 47, 108 / 98; FP32 weights (20k, 60k) 48 / 16, 46 / 33; shifting 41 / 21, 41 / 43;
+// predictor 72 / 37, 84 / 76: lines of their own would win the FP64 gradients and the FP32 weights and
+// predictor some 10 us each about 60k rows.
+// The pressure gradient, whose pairs are cheap, has its own, measured on the FP64 kernel: 34 / 18 at 1.7k,
+// 31 / 29 at 10k, 53 / 63 at 20k.  The FP32 one takes the same line; it is not measured by eight lanes.
 constexpr int LANE_ROWS = 30000;
 constexpr int LANE_ROWS_PGRAD = 10000;
 

@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(TPB) k_na_bicgstab(NaArgs a) {
 // shared memory for the whole solve, so a product waits for L2 once per NA_AHEAD operands, all of
 // them in flight, and not twice per slot; only p_inv, s_inv and the partial sums pass through L2.
 // A row's product is one chain in slot order and every sum keeps k_na_bicgstab's order, so the
-// solution is that kernel's bit for bit.
+// solution is that kernel's bit for bit (compared on the CPU, where the number of SMs is a test's).
 // What bounds it: up to two warps a scheduler, the chain of an iteration (seven barriers, five
 // sums, two products of 45 dependent FMAs), ~24 us; above that the FP64 pipe, at ~150 operations a row.
 // Measured against k_na_bicgstab, ms per solve: 576 rows x 24 iterations 0.57 / 1.45, 16k x 98
